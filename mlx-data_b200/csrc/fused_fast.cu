@@ -911,7 +911,9 @@ __device__ void gather_rows(
     const int x_first = xa + 4 * q;
     const int npx = min(4, xb - x_first);
     const int gy = s.post_y + y0 + ry;
-    unsigned px[4][C];   // source bytes of the four pixels
+    // source bytes of the four pixels; 0 where a mirrored row's last quad has fewer than
+    // four, since they index the cast table whether they are stored or not
+    unsigned px[4][C] = {};
     if (s.mode == kModeAffine) {
 #pragma unroll
       for (int j = 0; j < 4; j++) {
