@@ -268,7 +268,6 @@ int mlxd_fused_batch_on_stream(
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   // validate + plan
   std::vector<DevSample> dev;
-  PassNeed need;
   mlxd_batch_desc b = *batch;
   Lane& ring = *ctx->lanes[ctx->n_user_lanes + 1];
   LutUse table_in_use(ctx);
@@ -278,16 +277,11 @@ int mlxd_fused_batch_on_stream(
     return rc;
   }
   p.status = ring.d_status;
-  rc = plan_samples(samples, n, &b, dev, need);
+  rc = plan_samples(samples, n, &b, dev, p.walk);
   if (rc != MLXD_OK) {
     return rc;
   }
-  p.src_tile_bytes = need.src_bytes;
-  p.mid_float4s = need.mid_float4s;
-  p.weight_floats = need.weight_floats;
-  p.u_cap = need.u_cap;
-  p.fast_smem_bytes = (int32_t)need.fast_smem_bytes;
-  choose_kernel(p, need, dev.data(), n);
+  choose_kernels(p, dev.data(), n);
   const size_t esize = p.out_f32 ? 4 : 1;
   const size_t slot_bytes = (size_t)b.slot_h * b.slot_w * p.c_out * esize;
   uint64_t algo_src = 0;

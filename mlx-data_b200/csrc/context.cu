@@ -142,76 +142,7 @@ static int check_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc*
   return MLXD_OK;
 }
 
-// Shared memory of the float32 kernel that grows with the pass (staged source,
-// planar buffer, two table sets, vertical weights), and the budget under which
-// three CTAs still fit on one SM next to the fixed part (cast table, headers).
-static long long pass_bytes(const PassNeed& n) {
-  return (long long)n.src_bytes + 16LL * n.mid_float4s + 16LL * n.weight_floats + 256LL * n.u_cap;
-}
-constexpr long long kPassBudgetBytes = 69 * 1024;
-
-static int plan_resize(DevSample& s, int C, int i, PassNeed& need, long long pass_budget) {
-  // First look for the largest pass within the three-CTA budget, not going
-  // below 4 x 16 outputs; failing that, take the largest pass that fits at all.
-  for (int budgeted = 1; budgeted >= 0; budgeted--) {
-    int sub_h = kTileH, sub_w = kTileW;
-    for (;;) {
-      const AxisPlan ay = plan_axis(s.pre_h, s.geom_h, sub_h);
-      const AxisPlan ax = plan_axis(s.pre_w, s.geom_w, sub_w);
-      bool fits = false;
-      PassNeed n = plan_pass(ay, ax, sub_h, sub_w, s.pre_h, s.pre_w, C, fits);
-      // source rows feeding one group of (at most) four adjacent output rows
-      n.u_cap = plan_axis(s.pre_h, s.geom_h, std::min(4, sub_h)).extent;
-      fits = fits && n.u_cap <= kMaxStagedRows;
-      if (budgeted) {
-        fits = fits && pass_bytes(n) <= pass_budget;
-      }
-      if (fits) {
-        s.sub_h = sub_h;
-        s.sub_w = sub_w;
-        s.cap_y = ay.cap;
-        s.cap_x = ax.cap;
-        need.src_bytes = std::max(need.src_bytes, n.src_bytes);
-        need.mid_float4s = std::max(need.mid_float4s, n.mid_float4s);
-        need.weight_floats = std::max(need.weight_floats, n.weight_floats);
-        need.u_cap = std::max(need.u_cap, n.u_cap);
-        // the float32 kernel lays a CTA out from its own sample's needs
-        s.need_src = n.src_bytes;
-        s.need_mid4 = n.mid_float4s;
-        s.need_wts_ucap = n.weight_floats | (n.u_cap << 16);
-        need.sum_bytes = std::max<int64_t>(need.sum_bytes, pass_bytes(n));
-        need.fast_smem_bytes = std::max<int64_t>(
-            need.fast_smem_bytes,
-            (int64_t)fused_fast_layout_bytes(C, n.u_cap, n.weight_floats, n.mid_float4s, n.src_bytes));
-        return MLXD_OK;
-      }
-      if (budgeted && sub_h <= 4 && sub_w <= 16) {
-        break;
-      }
-      if (sub_h > 4) {
-        sub_h /= 2;
-      } else if (sub_w > 8) {
-        sub_w /= 2;
-      } else if (sub_h > 1) {
-        sub_h /= 2;
-      } else if (sub_w > 1) {
-        sub_w /= 2;
-      } else {
-        break;
-      }
-    }
-  }
-  // No pass size holds the taps of even one output: the sample is filtered
-  // pixel by pixel from global memory instead.
-  (void)i;
-  s.mode = kModeResizeDirect;
-  s.cap_y = plan_axis(s.pre_h, s.geom_h, 1).cap;
-  s.cap_x = plan_axis(s.pre_w, s.geom_w, 1).cap;
-  return MLXD_OK;
-}
-
-int plan_one_sample(
-    const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, DevSample& out, PassNeed& need, long long pass_budget) {
+int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, DevSample& out) {
   {
     int rc = check_sample(d, i, b, b->slot_h, b->slot_w);
     if (rc != MLXD_OK) {
@@ -237,18 +168,13 @@ int plan_one_sample(
     s.slot_h = b->slot_h;
     s.slot_w = b->slot_w;
     std::memcpy(s.mx, d.mx, sizeof(s.mx));
-    s.sub_h = kTileH;
-    s.sub_w = kTileW;
-    s.cap_y = s.cap_x = 1;
+    s.cap_x = 1;
     if (d.geom == MLXD_GEOM_RESIZE) {
       if (d.pre_w == d.geom_w && d.pre_h == d.geom_h) {
         s.mode = kModeCopy;  // identity on both axes
       } else {
-        s.mode = kModeResize;
-        rc = plan_resize(s, b->channels, i, need, pass_budget);
-        if (rc != MLXD_OK) {
-          return rc;
-        }
+        s.mode = walk_fits(s, b->channels) ? kModeResize : kModeResizeDirect;
+        s.cap_x = plan_axis(s.pre_w, s.geom_w, 1).cap;
       }
     } else if (d.geom == MLXD_GEOM_AFFINE) {
       s.mode = kModeAffine;
@@ -266,34 +192,22 @@ int plan_one_sample(
   return MLXD_OK;
 }
 
-int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, DevSample* out, PassNeed& need) {
-  // A launch allocates the largest need of every kind over its samples, which
-  // may come from different samples.  If the combination misses the three-CTA
-  // budget, one try with smaller passes; if that is not enough either, the
-  // full-size passes at two CTAs per SM are the better deal.
-  const long long budgets[3] = {kPassBudgetBytes, kPassBudgetBytes - 8 * 1024, kPassBudgetBytes};
-  for (int k = 0; k < 3; k++) {
-    need = PassNeed{0, 0, 0, 0, 0, 0};
-    for (int i = 0; i < n; i++) {
-      const int rc = plan_one_sample(samples[i], i, b, out[i], need, budgets[k]);
-      if (rc != MLXD_OK) {
-        return rc;
-      }
-    }
-    // the float32 kernel needs the largest per-sample sum, the generic one the sum of the largest parts
-    const bool fast = true;
-    if ((fast ? (long long)need.sum_bytes : pass_bytes(need)) <= kPassBudgetBytes) {
-      break;
+int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, DevSample* out, WalkPlan& walk) {
+  for (int i = 0; i < n; i++) {
+    const int rc = plan_one_sample(samples[i], i, b, out[i]);
+    if (rc != MLXD_OK) {
+      return rc;
     }
   }
+  plan_walk(out, n, b->channels, walk);
   return MLXD_OK;
 }
 
 int plan_samples(
     const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b,
-    std::vector<DevSample>& out, PassNeed& need) {
+    std::vector<DevSample>& out, WalkPlan& walk) {
   out.resize(n);
-  return plan_into(samples, n, b, out.data(), need);
+  return plan_into(samples, n, b, out.data(), walk);
 }
 
 // Source samples of an n_src -> n_dst axis that outputs [o_lo, o_hi) can read,
@@ -477,18 +391,12 @@ int enqueue_on_lane(
     return rc;
   }
   std::vector<DevSample> dev;
-  PassNeed need;
   p.status = lane.d_status;
-  rc = plan_samples(samples, n, batch, dev, need);
+  rc = plan_samples(samples, n, batch, dev, p.walk);
   if (rc != MLXD_OK) {
     return rc;
   }
-  p.src_tile_bytes = need.src_bytes;
-  p.mid_float4s = need.mid_float4s;
-  p.weight_floats = need.weight_floats;
-  p.u_cap = need.u_cap;
-  p.fast_smem_bytes = (int32_t)need.fast_smem_bytes;
-  choose_kernel(p, need, dev.data(), n);
+  choose_kernels(p, dev.data(), n);
   const size_t esize = p.out_f32 ? 4 : 1;
   const size_t slot_bytes = (size_t)batch->slot_h * batch->slot_w * p.c_out * esize;
   const size_t out_bytes = slot_bytes * n;

@@ -8,21 +8,21 @@
 
 namespace mlxd {
 
-constexpr int kTileH = 16;    // output rows per CTA
-constexpr int kTileW = 64;    // output pixels per row per CTA
+constexpr int kTileH = 16;    // copy and affine bands: output rows per CTA
+constexpr int kTileW = 64;    // and output pixels per tile
 constexpr int kThreads = 256;
 
-// Upper bounds on the shared memory one resize pass may ask for.  The planner
-// shrinks the pass (sub_h x sub_w outputs) until its footprint fits; a launch
-// then allocates only the largest need among its samples.
-constexpr int kSrcTileBytes = 48 * 1024;   // staged source footprint, uint8
-constexpr int kMidFloats = 12 * 1024;      // vertically filtered values, float32
-constexpr int kWeightFloats = 2 * 1024;    // tap weights of both axes
-constexpr int kMaxStagedRows = 192;        // source rows per pass
+// Resize kernel (resize_walk.cu).
+constexpr int kWalkThreads = 128;
+constexpr int kWalkRow = 832;       // floats per row in shared memory: source bytes of a chunk, alignment included
+constexpr int kWalkMaxRows = 32;    // output rows per CTA
+constexpr int kWalkMaxSteps = 1024; // source rows walked per CTA
+constexpr int kWalkPadPx = 256;     // columns per strip of padding
 
-// kModeResizeDirect: a resize whose tap footprint does not fit the on-chip
-// passes at any pass size (shrink ratios of about 60 and more); every output
-// pixel is then filtered straight from global memory by resize_direct_kernel.
+// kModeResizeDirect: a resize whose taps do not fit one chunk of the resize
+// kernel (shrink ratios of about 100 and more along a row, 300 down the rows);
+// every output pixel is then filtered straight from global memory by
+// resize_direct_kernel.
 enum Mode : int32_t { kModeCopy = 0, kModeResize = 1, kModeAffine = 2, kModeResizeDirect = 3 };
 
 // One sample's program.  Coordinates name four nested images:
@@ -39,15 +39,21 @@ struct __align__(16) DevSample {
   int32_t slot_h, slot_w;
   int32_t mode;
   int32_t pre_flip, post_flip;
-  int32_t sub_h, sub_w;   // resize: geometric-output rows / columns filtered per pass
-  int32_t cap_y, cap_x;   // resize: tap-count bound per axis
+  int32_t cap_x;          // resize: bound on the horizontal tap count
+  int32_t walk_px;        // resize kernel: most output columns of a chunk,
+  int32_t walk_chunks;    // chunks that share the post window's columns,
+  int32_t walk_rows;      // output rows per CTA
   float mx[6];
   int32_t r0_staged;      // host use: first source row held by the staged copy
-  // resize, float32 kernel: this sample's own shared-memory needs.  A CTA lays
-  // its shared memory out from these, so a launch is sized by the largest sum
-  // over its samples, not by the sum of the largest parts.
-  int32_t need_src, need_mid4;
-  int32_t need_wts_ucap;  // weight floats in the low 16 bits, u_cap above
+};
+
+// What the resize kernel of one launch is sized by: the largest needs of its samples.
+struct WalkPlan {
+  int32_t px;         // columns of the widest chunk (0: no sample runs the resize kernel)
+  int32_t taps;       // horizontal weights of a chunk
+  int32_t steps;      // source rows of a walk
+  int32_t cells_y;    // grid of the sample with the most cells
+  int32_t cells_x;
 };
 
 struct LaunchParams {
@@ -63,42 +69,30 @@ struct LaunchParams {
   const float* lut;           // [c_out][256] cast table, device
   int32_t pad_px;             // pad value as a pixel
   int32_t* status;            // device word, non-zero once a self-check failed
-  // shared memory of the resize passes (0 when no sample resizes)
-  int32_t src_tile_bytes;
-  int32_t mid_float4s;
-  int32_t weight_floats;
-  int32_t u_cap;              // bound on the source rows feeding four adjacent output rows
-  int32_t band_tiles;         // float32 kernel: tiles per CTA along a row band (set at launch)
-  int32_t bands_x;            // float32 kernel: CTAs per row band
-  int32_t fast_smem_bytes;    // float32 kernel: dynamic shared memory of the launch
-  int32_t pad_apart;          // float32 kernel: the rows below each post window are written by pad_fill_kernel
-  int32_t direct;             // some sample is kModeResizeDirect: resize_direct_kernel runs after the band kernel
-  int32_t starve_wait;        // test hook: the first pass of every band expects 16 bytes that no copy delivers
+  int32_t band_tiles;         // band kernel: tiles per CTA along a row band (set at launch)
+  int32_t bands_x;            // band kernel: CTAs per row band
+  int32_t bands;              // some sample is copied or rotated: the band kernel runs
+  WalkPlan walk;
+  int32_t pad_apart;          // the rows below each post window are written by pad_fill_kernel
+  int32_t direct;             // some sample is kModeResizeDirect: resize_direct_kernel runs last
+  int32_t starve_wait;        // test hook: every resize CTA first waits for 16 bytes that no copy delivers
 };
 
-// Shared-memory need of one resize pass, from the planner's conservative bounds.
-struct PassNeed {
-  int32_t src_bytes;
-  int32_t mid_float4s;
-  int32_t weight_floats;
-  int32_t u_cap;
-  int64_t sum_bytes;          // largest per-sample sum of the parts that grow with the pass (pass_bytes)
-  int64_t fast_smem_bytes;    // float32 kernel: largest per-sample shared-memory layout
-};
-
-// Dynamic shared memory of the float32 kernel for a sample with these needs
-// (c_out channels in the cast table).
-size_t fused_fast_layout_bytes(int c_out, int u_cap, int weight_floats, int mid_float4s, int src_tile_bytes);
-
-// Launch the band kernel that fits the parameters (float32, float32 after the
-// channel reduction, uint8, two channels), preceded by pad_fill_kernel when
-// p.pad_apart is set.
+// Launch the kernels the parameters call for: pad_fill_kernel when p.pad_apart
+// is set, the resize kernel, the band kernel, resize_direct_kernel.
 cudaError_t launch_fused_batch(const LaunchParams& p, cudaStream_t stream);
-cudaError_t launch_fused_fast(const LaunchParams& p, cudaStream_t stream);
+cudaError_t launch_resize_walk(const LaunchParams& p, cudaStream_t stream);
 
-// Decide whether a ragged batch's padding gets a launch of its own; call after
-// the planner filled `need` and the host copy of the sample table.
-void choose_kernel(LaunchParams& p, const PassNeed& need, const DevSample* host_samples, int n);
+// Whether the resize kernel can run a sample (mode kModeResize) at all.
+bool walk_fits(const DevSample& s, int channels);
+
+// Split the resize samples of a batch into CTAs (DevSample::walk_*) and size
+// the launch.
+void plan_walk(DevSample* samples, int n, int channels, WalkPlan& plan);
+
+// Which kernels a launch needs and their grids; call after plan_walk with the
+// host copy of the sample table.
+void choose_kernels(LaunchParams& p, const DevSample* host_samples, int n);
 
 // Conservative per-axis bounds used by the host planner.
 struct AxisPlan {
@@ -106,11 +100,5 @@ struct AxisPlan {
   int32_t extent;   // bound on source samples touched by `sub` outputs
 };
 AxisPlan plan_axis(int32_t n_src, int32_t n_dst, int32_t sub);
-
-// Bound on the shared memory of a pass over sub_h x sub_w outputs of an axis
-// pair; `fits` tells whether it respects the limits above.
-PassNeed plan_pass(
-    const AxisPlan& ay, const AxisPlan& ax, int32_t sub_h, int32_t sub_w, int32_t pre_h, int32_t pre_w, int32_t channels,
-    bool& fits);
 
 } // namespace mlxd

@@ -1,4 +1,4 @@
-// Device helpers shared by the two kernels of the library.
+// Device helpers shared by the kernels of the library.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -83,9 +83,96 @@ __device__ __forceinline__ void axis_taps(
   count = cnt;
 }
 
-__device__ __forceinline__ int quantise(float acc) {
-  const float r = __fadd_rn(acc, 0.5f);
-  return r < 0.0f ? 0 : (r > 255.0f ? 255 : (int)r);
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// Typed view of a shared-space address.
+template <typename T>
+__device__ __forceinline__ T* sp(unsigned a) {
+  return reinterpret_cast<T*>(__cvta_shared_to_generic(a));
+}
+
+// Two float lanes in one 64-bit register, the operand form of the packed
+// instructions; keeping values packed avoids repacking moves around them.
+typedef unsigned long long f32x2;
+
+// d = a * b + d on both lanes (each lane is an IEEE fused multiply-add,
+// identical to fmaf).
+__device__ __forceinline__ void ffma2(f32x2& d, f32x2 a, f32x2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+__device__ __forceinline__ f32x2 fmul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+// Bytes B0 and B1 of a word as two packed floats, exactly: each byte is placed
+// in the mantissa of 2^23 and 2^23 is subtracted (one packed add for both).
+template <int B0, int B1>
+__device__ __forceinline__ f32x2 bytes_to_f32x2(uint32_t word, f32x2 minus_two23) {
+  const float x0 = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540u + B0));
+  const float x1 = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540u + B1));
+  f32x2 r = pack2(x0, x1);
+  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(r) : "l"(minus_two23));
+  return r;
+}
+
+// (int)(acc + 0.5) clamped to [0, 255]: the float-to-uint8 conversion truncates
+// toward zero and saturates at both ends, which is that clamp.
+__device__ __forceinline__ unsigned quantise_sat(float acc) {
+  unsigned q;
+  asm("cvt.rzi.u8.f32 %0, %1;" : "=r"(q) : "f"(__fadd_rn(acc, 0.5f)));
+  return q;
+}
+
+// Shared-memory loads by 32-bit shared-space address plus a constant offset.
+// Spelling the inner loops with these keeps their address arithmetic to the
+// pointer increments written out in the loops.
+template <int OFF>
+__device__ __forceinline__ uint32_t lds_u32(unsigned a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFF));
+  return v;
+}
+
+template <int OFF>
+__device__ __forceinline__ void lds_v2u32(unsigned a, uint32_t& x, uint32_t& y) {
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2+%3];" : "=r"(x), "=r"(y) : "r"(a), "n"(OFF));
+}
+
+template <int OFF>
+__device__ __forceinline__ f32x2 lds_u64(unsigned a) {
+  f32x2 v;
+  asm volatile("ld.shared.u64 %0, [%1+%2];" : "=l"(v) : "r"(a), "n"(OFF));
+  return v;
+}
+
+template <int OFF>
+__device__ __forceinline__ void lds_v2u64(unsigned a, f32x2& x, f32x2& y) {
+  asm volatile("ld.shared.v2.u64 {%0, %1}, [%2+%3];" : "=l"(x), "=l"(y) : "r"(a), "n"(OFF));
+}
+
+// Channel reduction of one quantised pixel: 16.16 fixed point, truncating
+// division, clamped (core::image::channel_reduction,
+// mlx/data/core/image/ImageTransform.cpp:159-180).
+__device__ __forceinline__ unsigned gray_mix(const LaunchParams& p, unsigned r, unsigned g, unsigned b) {
+  int v = ((int)r * p.gray_m[0] + (int)g * p.gray_m[1] + (int)b * p.gray_m[2] + p.gray_bias) / 65536;
+  v = v <= 255 ? v : 255;
+  v = v >= 0 ? v : 0;
+  return (unsigned)v;
 }
 
 template <int CO>
@@ -116,6 +203,7 @@ __device__ __forceinline__ void fill_rect_f32(
   if (ya >= yb || xa >= xb) {
     return;
   }
+  const int n_threads = (int)blockDim.x;
   const int L = (xb - xa) * CO;
   const int ny = yb - ya;
   const size_t row_floats = (size_t)slot_w * CO;
@@ -126,8 +214,8 @@ __device__ __forceinline__ void fill_rect_f32(
     head = head > L ? L : head;
     const int nvec = (L - head) >> 2;
     if (nvec > 0) {
-      const int lanes_q = nvec >= kThreads ? kThreads : nvec;
-      const int phases = kThreads / lanes_q;
+      const int lanes_q = nvec >= n_threads ? n_threads : nvec;
+      const int phases = n_threads / lanes_q;
       const int r0 = (int)threadIdx.x / lanes_q;
       if (r0 < phases) {
         for (int q = (int)threadIdx.x - r0 * lanes_q; q < nvec; q += lanes_q) {
@@ -146,7 +234,7 @@ __device__ __forceinline__ void fill_rect_f32(
     // the few floats before the first and after the last aligned unit of each row
     const int tail = head + 4 * nvec;
     const int loose = head + (L - tail);
-    for (int i = threadIdx.x; i < ny * loose; i += kThreads) {
+    for (int i = threadIdx.x; i < ny * loose; i += n_threads) {
       const int ry = i / loose;
       const int k = i - ry * loose;
       const int j = k < head ? k : tail + (k - head);
@@ -155,7 +243,7 @@ __device__ __forceinline__ void fill_rect_f32(
     return;
   }
   const int Q = ((L + 3) >> 2) + 2;
-  for (int i = threadIdx.x; i < ny * Q; i += kThreads) {
+  for (int i = threadIdx.x; i < ny * Q; i += n_threads) {
     const int ry = i / Q;
     const int q = i - ry * Q;
     float* rowp = row0 + (size_t)ry * row_floats;
@@ -194,7 +282,7 @@ __device__ __forceinline__ void fill_rect_u8(
   const size_t row_bytes = (size_t)slot_w * CO;
   const unsigned w = (unsigned)(pad_px & 0xff) * 0x01010101u;
   const uint4 v = make_uint4(w, w, w, w);
-  for (int ry = (int)threadIdx.x >> 5; ry < ny; ry += kThreads >> 5) {     // a warp per row
+  for (int ry = (int)threadIdx.x >> 5; ry < ny; ry += (int)blockDim.x >> 5) {     // a warp per row
     uint8_t* rowp = base + (size_t)(ya + ry) * row_bytes + (size_t)xa * CO;
     const int mis = (int)(reinterpret_cast<uintptr_t>(rowp) & 15);
     int head = (16 - mis) & 15;

@@ -1,6 +1,5 @@
-// Host side of a launch: which kernels run it, and the planner's bounds on
-// what one resize pass needs on chip.  The kernels themselves are in
-// fused_fast.cu.
+// Host side of a launch: which kernels run it, and how the resize samples are
+// split into CTAs.
 //
 // Reference behaviour the kernels reproduce (paths inside mlx-data):
 //   resize             mlx/data/core/image/ImageTransform.cpp:41-62 (triangle filter, clamp to edge)
@@ -10,38 +9,36 @@
 //   channel_reduction  mlx/data/core/image/ImageTransform.cpp:142-182
 //   batch + pad        mlx/data/Array.cpp:465-498, mlx/data/core/BatchShape.cpp:26-45
 //   cast               README.md:55-57 (x.astype(float32) / 255 and its normalised form)
+#include <algorithm>
 #include <cmath>
 
 #include "fused_batch.h"
 
 namespace mlxd {
 
-cudaError_t launch_fused_batch(const LaunchParams& p, cudaStream_t stream) {
-  return launch_fused_fast(p, stream);
-}
-
-void choose_kernel(LaunchParams& p, const PassNeed& need, const DevSample* host_samples, int n) {
-  (void)need;
+void choose_kernels(LaunchParams& p, const DevSample* host_samples, int n) {
+  p.bands = 0;
+  p.direct = 0;
+  unsigned long long rows = 0, below = 0;
+  for (int i = 0; i < n; i++) {
+    const DevSample& s = host_samples[i];
+    p.bands |= s.mode != kModeResize;   // a direct sample's padding is the band kernel's too
+    p.direct |= s.mode == kModeResizeDirect;
+    rows += (unsigned long long)s.slot_h;
+    below += (unsigned long long)(s.slot_h > s.post_h ? s.slot_h - s.post_h : 0);
+  }
   // The rows below a sample's post window are one contiguous run of its slot;
   // when those runs are at least an eighth of the batch they get a linear fill
   // of their own (pad_fill_kernel), which writes at memory speed.
-  p.pad_apart = 0;
-  p.direct = 0;
+  p.pad_apart = n > 0 && below * 8 >= rows ? 1 : 0;
+  p.walk.cells_y = p.walk.cells_x = 0;
   for (int i = 0; i < n; i++) {
-    if (host_samples[i].mode == kModeResizeDirect) {
-      p.direct = 1;
+    const DevSample& s = host_samples[i];
+    if (s.mode == kModeResize) {
+      const int h = p.pad_apart ? s.post_h : s.slot_h;
+      p.walk.cells_y = std::max(p.walk.cells_y, (h + s.walk_rows - 1) / s.walk_rows);
+      p.walk.cells_x = std::max(p.walk.cells_x, s.walk_chunks + (s.slot_w - s.post_w + kWalkPadPx - 1) / kWalkPadPx);
     }
-  }
-  if (n > 0) {
-    unsigned long long rows = 0, below = 0;
-    for (int i = 0; i < n; i++) {
-      const int h = host_samples[i].slot_h;
-      const int ph = host_samples[i].post_h < h ? host_samples[i].post_h : h;
-      const int first = ((ph + kTileH - 1) / kTileH) * kTileH;
-      rows += (unsigned long long)h;
-      below += (unsigned long long)(first < h ? h - first : 0);
-    }
-    p.pad_apart = below * 8 >= rows ? 1 : 0;
   }
 }
 
@@ -62,27 +59,67 @@ AxisPlan plan_axis(int32_t n_src, int32_t n_dst, int32_t sub) {
   return a;
 }
 
-PassNeed plan_pass(
-    const AxisPlan& ay, const AxisPlan& ax, int32_t sub_h, int32_t sub_w, int32_t pre_h, int32_t pre_w, int32_t channels,
-    bool& fits) {
-  const long long rows = ay.extent < pre_h ? ay.extent : pre_h;
-  const long long cols = ax.extent < pre_w ? ax.extent : pre_w;
-  const long long wbytes = cols * channels;
-  const long long pitch = (wbytes + 49 + 15) & ~15LL;
-  const long long src = rows * pitch;
-  // every plane is padded by up to 7 columns on either side and one slot is
-  // skipped after every eight columns
-  const long long pad = (7 + channels - 1) / channels;
-  const long long pslots = (cols + 2 * pad) + (cols + 2 * pad) / 8 + 1;
-  const long long mid4 = ((sub_h + 3) / 4) * channels * pslots;   // one set of planes per group of four rows
-  const long long wts = (long long)sub_h * ay.cap + (long long)sub_w * ax.cap;
-  fits = src <= kSrcTileBytes && mid4 * 4 <= kMidFloats && wts <= kWeightFloats && rows <= kMaxStagedRows;
-  PassNeed n;
-  n.src_bytes = (int32_t)src;
-  n.mid_float4s = (int32_t)mid4;
-  n.weight_floats = (int32_t)wts;
-  n.u_cap = (int32_t)(ay.extent < pre_h + 2 * ay.cap ? ay.extent : pre_h + 2 * ay.cap);
-  return n;
+// Source bytes of `px` output columns, from the word that holds the first one.
+static long long walk_row_bytes(const DevSample& s, int channels, int px) {
+  const long long cols = std::min(plan_axis(s.pre_w, s.geom_w, px).extent, s.pre_w);
+  return cols * channels + 6;
+}
+
+// Steps of a walk over `rows` output rows: every source row once, again once
+// per output row whose neighbours on both sides reach it, one per output row
+// at least.  (Enlargements walk the two rows of every output row.)
+static long long walk_steps(const DevSample& s, int rows) {
+  const long long extent = plan_axis(s.pre_h, s.geom_h, rows).extent;
+  return s.pre_h <= s.geom_h ? 4LL * rows + 4 : extent + rows + 8;
+}
+
+bool walk_fits(const DevSample& s, int channels) {
+  return walk_row_bytes(s, channels, 1) <= kWalkRow && walk_steps(s, 1) <= kWalkMaxSteps &&
+      (long long)s.src_w * channels < (1LL << 31);
+}
+
+// Chunks of at most `px` columns and walks of at most `rows` rows, smaller
+// where the source footprint asks for it.
+static void split_walk(DevSample& s, int channels, int px, int rows) {
+  while (px > 1 && walk_row_bytes(s, channels, px) > kWalkRow) {
+    px--;
+  }
+  while (rows > 1 && walk_steps(s, rows) > kWalkMaxSteps / 4) {
+    rows /= 2;
+  }
+  s.walk_chunks = (s.post_w + px - 1) / px;
+  s.walk_px = (s.post_w + s.walk_chunks - 1) / s.walk_chunks;
+  s.walk_rows = rows;
+}
+
+void plan_walk(DevSample* samples, int n, int channels, WalkPlan& plan) {
+  // The largest cells that still give every one of the 148 SMs two CTAs.  A CTA
+  // builds its tables and walks 2 r source rows (shrink ratio r) before its first
+  // output row is complete, so smaller cells cost more as soon as the SMs have
+  // work: 512 frames of 1080x1920 to 512x512 take 1.37 ms in 128x32 cells, 1.46
+  // in 128x16, 1.58 in 64x32, 3.4 in 64x4; 32 images of 200-500 px to 224x224
+  // 32 us in 448 CTAs of 128x32 and in 1792 of 128x8, 52 us in 64x4.  One 480x640
+  // image to 224x224 fills no wave of any size and is quickest in the smallest
+  // cells: 14.4 us a call in 64x4, 18 in 128x8.
+  static const int kCells[][2] = {{128, 32}, {128, 16}, {128, 8}, {64, 8}, {64, 4}};
+  constexpr long long kWantCtas = 148 * 2;
+  for (const auto& cell : kCells) {
+    long long ctas = 0;
+    plan = WalkPlan{0, 0, 0, 0, 0};
+    for (int i = 0; i < n; i++) {
+      DevSample& s = samples[i];
+      if (s.mode == kModeResize) {
+        split_walk(s, channels, cell[0], cell[1]);
+        ctas += (long long)s.walk_chunks * ((s.post_h + s.walk_rows - 1) / s.walk_rows);
+        plan.px = std::max(plan.px, s.walk_px);
+        plan.taps = std::max(plan.taps, s.walk_px * s.cap_x);
+        plan.steps = std::max(plan.steps, (int32_t)walk_steps(s, s.walk_rows));
+      }
+    }
+    if (ctas == 0 || ctas >= kWantCtas) {
+      return;
+    }
+  }
 }
 
 } // namespace mlxd

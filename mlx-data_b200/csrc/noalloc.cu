@@ -122,22 +122,16 @@ extern "C" int mlxd_fused_batch_noalloc(
   p.lut = reinterpret_cast<const float*>(scratch + kTableBytes);
   p.status = reinterpret_cast<int32_t*>(scratch + kStatusOffset);
 
-  PassNeed need = PassNeed{0, 0, 0, 0, 0, 0};
   const size_t esize = p.out_f32 ? 4 : 1;
   const size_t slot_bytes = (size_t)batch->slot_h * batch->slot_w * p.c_out * esize;
-  rc = plan_into(samples, n, batch, table, need);
+  rc = plan_into(samples, n, batch, table, p.walk);
   if (rc != MLXD_OK) {
     return rc;
   }
   for (int i = 0; i < n; i++) {
     table[i].dst = static_cast<uint8_t*>(batch->dst) + slot_bytes * i;
   }
-  p.src_tile_bytes = need.src_bytes;
-  p.mid_float4s = need.mid_float4s;
-  p.weight_floats = need.weight_floats;
-  p.u_cap = need.u_cap;
-  p.fast_smem_bytes = (int32_t)need.fast_smem_bytes;
-  choose_kernel(p, need, table, n);
+  choose_kernels(p, table, n);
 
   // The scratch keeps whatever the previous call left.  Its status word is
   // read back first (the kernel of the previous call is ahead of this copy on
