@@ -81,8 +81,14 @@ bool walk_fits(const DevSample& s, int channels) {
 // Chunks of at most `px` columns and walks of at most `rows` rows, smaller
 // where the source footprint asks for it.
 static void split_walk(DevSample& s, int channels, int px, int rows) {
-  while (px > 1 && walk_row_bytes(s, channels, px) > kWalkRow) {
-    px--;
+  if (walk_row_bytes(s, channels, px) > kWalkRow) {
+    // (px + 1) * ratio + 3 source columns at most (plan_axis), then down to what fits
+    const double ratio = (double)s.pre_w / (double)s.geom_w;
+    const int guess = s.pre_w <= s.geom_w ? px : (int)(kWalkRow / channels / ratio);
+    px = std::max(1, std::min(px, guess));
+    while (px > 1 && walk_row_bytes(s, channels, px) > kWalkRow) {
+      px--;
+    }
   }
   while (rows > 1 && walk_steps(s, rows) > kWalkMaxSteps / 4) {
     rows /= 2;

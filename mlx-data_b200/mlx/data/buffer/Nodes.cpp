@@ -27,10 +27,14 @@ void FromVector::check() const {
 }
 
 Sample FromVector::get(int64_t idx) const {
+  return *peek(idx);
+}
+
+const Sample* FromVector::peek(int64_t idx) const {
   if (idx < 0 || idx >= static_cast<int64_t>(data_.size())) {
     throw std::out_of_range("FromVector: index out of range");
   }
-  return data_[idx];
+  return &data_[idx];
 }
 
 int64_t FromVector::size() const {
@@ -155,10 +159,17 @@ Sample Batch::get(int64_t idx) const {
     lo = starts_[idx];
     hi = starts_[idx + 1];
   }
-  std::vector<Sample> raw;
+  std::vector<Sample> made;   // never grows beyond its reserve: `raw` points into it
+  made.reserve(hi - lo);
+  std::vector<const Sample*> raw;
   raw.reserve(hi - lo);
   for (int64_t i = lo; i < hi; i++) {
-    raw.push_back(base_->get(i));
+    const Sample* held = base_->peek(i);
+    if (!held) {
+      made.push_back(base_->get(i));
+      held = &made.back();
+    }
+    raw.push_back(held);
   }
   return batcher_->run(raw);
 }

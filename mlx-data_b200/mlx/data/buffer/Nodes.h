@@ -20,6 +20,7 @@ class FromVector : public Buffer {
   explicit FromVector(const std::vector<Sample>& data);
   explicit FromVector(std::vector<Sample>&& data);
   Sample get(int64_t idx) const override;  // throws std::out_of_range
+  const Sample* peek(int64_t idx) const override;
   int64_t size() const override;
 
  private:

@@ -38,6 +38,8 @@ class Batcher {
 
   // Empty input gives an empty sample (end of stream).
   Sample run(const std::vector<Sample>& raw) const;
+  // The same for samples held elsewhere; they stay in place during the call.
+  Sample run(const std::vector<const Sample*>& raw) const;
 
   const std::vector<std::shared_ptr<op::FusableOp>>& ops() const { return ops_; }
   const std::unordered_map<std::string, double>& pad_values() const { return pad_values_; }

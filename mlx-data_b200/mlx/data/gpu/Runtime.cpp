@@ -500,16 +500,26 @@ std::shared_ptr<Array> Runtime::device_array(
 
 std::shared_ptr<Array> Runtime::batch(
     const std::vector<LazyImage>& images, double pad_value, const CastSpec* cast, const Placement& where) {
+  std::vector<const LazyImage*> at;
+  at.reserve(images.size());
+  for (auto& im : images) {
+    at.push_back(&im);
+  }
+  return batch(at, pad_value, cast, where);
+}
+
+std::shared_ptr<Array> Runtime::batch(
+    const std::vector<const LazyImage*>& images, double pad_value, const CastSpec* cast, const Placement& where) {
   if (images.empty()) {
     throw std::runtime_error("Array: cannot batch an empty list of arrays");
   }
   const int n = static_cast<int>(images.size());
-  const LazyImage& first = images.front();
+  const LazyImage& first = *images.front();
   int64_t max_h = 0, max_w = 0;
   int on_device = 0;
   std::vector<mlxd_sample_desc> descs(images.size());
   for (int i = 0; i < n; i++) {
-    const LazyImage& im = images[i];
+    const LazyImage& im = *images[i];
     if (im.source()->type() != UInt8) {
       throw std::invalid_argument("image must be of type UInt8");
     }

@@ -163,6 +163,8 @@ class Runtime {
   // One fused launch: every image's program, batch + pad, optional cast.
   // Result is [N, max_h, max_w, C] uint8, or float32 when cast is given.
   std::shared_ptr<Array> batch(
+      const std::vector<const LazyImage*>& images, double pad_value, const CastSpec* cast, const Placement& where);
+  std::shared_ptr<Array> batch(
       const std::vector<LazyImage>& images, double pad_value, const CastSpec* cast, const Placement& where);
 
   // Cast an existing uint8 array (any shape, last dimension = channels <= 4).
