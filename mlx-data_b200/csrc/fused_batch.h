@@ -17,6 +17,7 @@ constexpr int kWalkThreads = 128;
 constexpr int kWalkRow = 832;       // floats per row in shared memory: source bytes of a chunk, alignment included
 constexpr int kWalkMaxRows = 32;    // output rows per CTA
 constexpr int kWalkMaxSteps = 1024; // source rows walked per CTA
+constexpr int kPadChunks = 128;     // CTAs that fill the rows below one sample
 constexpr int kWalkPadPx = 256;     // columns per strip of padding
 
 // kModeResizeDirect: a resize whose taps do not fit one chunk of the resize
@@ -73,13 +74,14 @@ struct LaunchParams {
   int32_t bands_x;            // band kernel: CTAs per row band
   int32_t bands;              // some sample is copied or rotated: the band kernel runs
   WalkPlan walk;
-  int32_t pad_apart;          // the rows below each post window are written by pad_fill_kernel
+  int32_t pad_apart;          // the rows below each post window are filled apart from the cells around them
+  int32_t fill_every;         // resize kernel, then: every so many CTAs, from the first on, one of them fills
   int32_t direct;             // some sample is kModeResizeDirect: resize_direct_kernel runs last
   int32_t starve_wait;        // test hook: every resize CTA first waits for 16 bytes that no copy delivers
 };
 
-// Launch the kernels the parameters call for: pad_fill_kernel when p.pad_apart
-// is set, the resize kernel, the band kernel, resize_direct_kernel.
+// Launch the kernels the parameters call for: the resize kernel or, without a
+// resize and when p.pad_apart is set, pad_fill_kernel, the band kernel, resize_direct_kernel.
 cudaError_t launch_fused_batch(const LaunchParams& p, cudaStream_t stream);
 cudaError_t launch_resize_walk(const LaunchParams& p, cudaStream_t stream);
 

@@ -299,4 +299,108 @@ __device__ __forceinline__ void fill_rect_u8(
   }
 }
 
+// The padding below a sample of a ragged batch.  Rows of a slot are contiguous,
+// so everything below the sample's post
+// window down to the end of the slot is one contiguous run of floats: written
+// here as a linear fill (16-byte stores, consecutive threads on consecutive
+// addresses, kPadChunks CTAs per sample), which runs at memory speed - the
+// band kernels above, writing 16-row strips, reach about 60 % of that.  The
+// strips to the right of the post window stay with the band kernels.
+template <int CO>
+__device__ __forceinline__ void pad_below(const LaunchParams& p, unsigned block) {
+  const int n = (int)(block / kPadChunks);
+  const int chunk = (int)(block % kPadChunks);
+  if (n >= p.n) {
+    return;
+  }
+  const DevSample* s = p.samples + n;
+  const int slot_h = s->slot_h, slot_w = s->slot_w;
+  const int post_h = s->post_h < slot_h ? s->post_h : slot_h;
+  const int first_row = post_h;
+  if (first_row >= slot_h) {
+    return;
+  }
+  float padf[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    padf[c] = c < CO ? __ldg(p.lut + c * 256 + p.pad_px) : 0.0f;
+  }
+  const size_t row_floats = (size_t)slot_w * CO;
+  float* run = reinterpret_cast<float*>(s->dst) + (size_t)first_row * row_floats;   // starts on a pixel: channel 0
+  const size_t len = (size_t)(slot_h - first_row) * row_floats;
+  const size_t mis = (reinterpret_cast<uintptr_t>(run) >> 2) & 3;
+  size_t head = (4 - mis) & 3;
+  head = head > len ? len : head;
+  const size_t nvec = (len - head) >> 2;
+  // this CTA's share of the aligned units
+  const size_t q0 = nvec * (size_t)chunk / kPadChunks;
+  const size_t q1 = nvec * (size_t)(chunk + 1) / kPadChunks;
+  for (size_t q = q0 + threadIdx.x; q < q1; q += (int)blockDim.x) {
+    const size_t j = head + 4 * q;
+    const int m = (int)(j % CO);
+    *reinterpret_cast<float4*>(run + j) = make_float4(
+        pad_pick<CO>(padf, m), pad_pick<CO>(padf, (m + 1) % CO), pad_pick<CO>(padf, (m + 2) % CO),
+        pad_pick<CO>(padf, (m + 3) % CO));
+  }
+  if (chunk == 0) {
+    // the floats before the first and after the last aligned unit
+    const size_t tail = head + 4 * nvec;
+    for (size_t k = threadIdx.x; k < head + (len - tail); k += (int)blockDim.x) {
+      const size_t j = k < head ? k : tail + (k - head);
+      run[j] = pad_pick<CO>(padf, (int)(j % CO));
+    }
+  }
+}
+
+// The same for a uint8 batch: a linear fill of bytes.
+__device__ __forceinline__ void pad_below_u8(const LaunchParams& p, unsigned block) {
+  const int n = (int)(block / kPadChunks);
+  const int chunk = (int)(block % kPadChunks);
+  if (n >= p.n) {
+    return;
+  }
+  const DevSample* s = p.samples + n;
+  const int slot_h = s->slot_h, slot_w = s->slot_w;
+  const int post_h = s->post_h < slot_h ? s->post_h : slot_h;
+  const int first_row = post_h;
+  if (first_row >= slot_h) {
+    return;
+  }
+  const size_t row_bytes = (size_t)slot_w * p.c_out;
+  uint8_t* run = reinterpret_cast<uint8_t*>(s->dst) + (size_t)first_row * row_bytes;
+  const size_t len = (size_t)(slot_h - first_row) * row_bytes;
+  const size_t mis = reinterpret_cast<uintptr_t>(run) & 15;
+  size_t head = (16 - mis) & 15;
+  head = head > len ? len : head;
+  const size_t nvec = (len - head) >> 4;
+  const unsigned w = (unsigned)(p.pad_px & 0xff) * 0x01010101u;
+  const uint4 v = make_uint4(w, w, w, w);
+  const size_t q0 = nvec * (size_t)chunk / kPadChunks;
+  const size_t q1 = nvec * (size_t)(chunk + 1) / kPadChunks;
+  for (size_t q = q0 + threadIdx.x; q < q1; q += (int)blockDim.x) {
+    *reinterpret_cast<uint4*>(run + head + 16 * q) = v;
+  }
+  if (chunk == 0) {
+    const size_t tail = head + 16 * nvec;
+    for (size_t k = threadIdx.x; k < head + (len - tail); k += (int)blockDim.x) {
+      run[k < head ? k : tail + (k - head)] = (uint8_t)p.pad_px;
+    }
+  }
+}
+
+// Block `block` of n * kPadChunks.
+__device__ __forceinline__ void pad_below_any(const LaunchParams& p, unsigned block) {
+  if (!p.out_f32) {
+    pad_below_u8(p, block);
+  } else if (p.c_out == 3) {
+    pad_below<3>(p, block);
+  } else if (p.c_out == 1) {
+    pad_below<1>(p, block);
+  } else if (p.c_out == 2) {
+    pad_below<2>(p, block);
+  } else {
+    pad_below<4>(p, block);
+  }
+}
+
 } // namespace mlxd

@@ -29,7 +29,8 @@ void choose_kernels(LaunchParams& p, const DevSample* host_samples, int n) {
   }
   // The rows below a sample's post window are one contiguous run of its slot;
   // when those runs are at least an eighth of the batch they get a linear fill
-  // of their own (pad_fill_kernel), which writes at memory speed.
+  // of their own (CTAs of the resize kernel, else pad_fill_kernel), which writes
+  // at memory speed.
   p.pad_apart = n > 0 && below * 8 >= rows ? 1 : 0;
   p.walk.cells_y = p.walk.cells_x = 0;
   for (int i = 0; i < n; i++) {
