@@ -27,10 +27,10 @@ import numpy as np
 
 ROOT = os.path.dirname(os.path.abspath(__file__))
 NOMINAL_HBM_GBS = 8000.0
-# dram__bytes_read.sum + dram__bytes_write.sum of one fused_fast_kernel launch per
-# image of the workload, from an ncu capture of a 128-image launch (852.6 MB);
-# the traffic of this kernel grows in proportion to the image count.
-NCU_DRAM_BYTES_PER_IMAGE = {"c5": 852.6e6 / 128}
+# DRAM bytes per image of the workload: dram__bytes_read.sum of an ncu capture of one
+# resize_walk_kernel launch on 64 images (239.7 MB), plus the batch it writes, all of
+# which leaves L2 in a launch larger than that; both grow with the image count.
+NCU_DRAM_BYTES_PER_IMAGE = {"c5": 239.7e6 / 64 + 512 * 512 * 3 * 4}
 
 
 def load_package():
@@ -650,7 +650,7 @@ def main():
                          "frac_of_nominal_8tbs": achieved / NOMINAL_HBM_GBS,
                          "kernel_ms": kernel_ms, "algorithmic_bytes_per_launch": algo_per_launch,
                          "traffic": (NCU_DRAM_BYTES_PER_IMAGE[name] * batch if name in NCU_DRAM_BYTES_PER_IMAGE else None),
-                         "traffic_kind": "ncu dram bytes of a 128-image launch scaled by the image count"},
+                         "traffic_kind": "ncu dram bytes read by a 64-image launch scaled by the image count, plus the batch"},
             "cpu_baseline": cpu,
         }
         if checked is not None and not checked["ok"]:

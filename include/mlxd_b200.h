@@ -190,8 +190,8 @@ MLXD_API int mlxd_ctx_set_timing(mlxd_ctx* ctx, int on);
  *    (the call clears what must start at zero): two calls whose kernels can
  *    overlap on the GPU - different streams, or different host threads - race;
  *    order them on one stream;
- *  - the kernel's self-check word (a bounded wait that ran out, a shared-memory
- *    bound) is read back at the start of the NEXT call on the same stream,
+ *  - the kernel's self-check word (a resize chunk beyond its planned shared
+ *    memory, a bounded wait that ran out) is read back at the start of the NEXT call on the same stream,
  *    which then returns MLXD_ERR_DEVICE and launches nothing; after the last
  *    call of a run ask mlxd_noalloc_status. */
 #define MLXD_NOALLOC_MAX_SAMPLES 1024
@@ -224,9 +224,9 @@ MLXD_API int mlxd_fused_batch_on_stream(
     mlxd_ctx* ctx, void* cuda_stream, const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* batch);
 
 /* Self-check word of the kernels launched by mlxd_fused_batch_on_stream: waits
- * for `cuda_stream`, stores the word in *status (0 = clean; bit 1/2: a pass
- * larger than the planned shared memory, 4: a bounded wait on a bulk copy ran
- * out, 8: more filter rows than planned), clears it, and returns
+ * for `cuda_stream`, stores the word in *status (0 = clean; 8: a resize chunk with
+ * more source rows or bytes than planned, 4: a bounded wait ran out, which only
+ * the test hook MLXD_TEST_STARVE_WAIT does), clears it, and returns
  * MLXD_ERR_DEVICE when it was set.  The lanes of mlxd_fused_batch report the
  * same word through mlxd_batch_wait.  No counterpart in the reference, whose
  * CPU ops throw where they stand. */

@@ -27,9 +27,9 @@
 //
 // What bounds it (1080x1920x3 to 512x512, 512 images, 1.37 ms, before: 1.75 ms in
 // 16x64-pixel passes staged by bulk copies and filtered from there): the shared-
-// memory pipe, 87 % busy, of whose wavefronts the horizontal taps are about 45 %
+// memory pipe, 89 % busy, of whose wavefronts the horizontal taps are about 45 %
 // (half of them bank conflicts of columns 2.1 apart), the stores of the row pairs
-// 20 %; instructions per 16x64 pixels are 7.3 k, before 10.2 k.  Why this split:
+// 20 %; instructions per 16x64 pixels are 6.6 k, before 10.2 k.  Why this split:
 // a walk converts a byte once instead of once per pair of output rows that it
 // feeds, keeps no source footprint on chip beyond the rows in flight, and has two
 // barriers per four output rows.  The rows in flight lie in shared memory because
