@@ -17,6 +17,11 @@ constexpr int kWalkThreads = 128;
 constexpr int kWalkRow = 832;       // floats per row in shared memory: source bytes of a chunk, alignment included
 constexpr int kWalkMaxRows = 32;    // output rows per CTA
 constexpr int kWalkMaxSteps = 1024; // source rows walked per CTA
+constexpr int kWalkMaxPx = 128;     // output columns per CTA
+// Horizontal weights per CTA: px columns of floor(2r) + 2 taps.  A shrink by r has
+// px * r <= kWalkRow (the chunk's source columns), so 2 * kWalkRow + 2 * kWalkMaxPx
+// bounds them; an enlargement has 4 * kWalkMaxPx.
+constexpr int kWalkMaxTaps = 2 * kWalkRow + 2 * kWalkMaxPx;
 constexpr int kPadChunks = 128;     // CTAs that fill the rows below one sample
 constexpr int kWalkPadPx = 256;     // columns per strip of padding
 

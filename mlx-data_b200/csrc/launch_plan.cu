@@ -108,7 +108,7 @@ void plan_walk(DevSample* samples, int n, int channels, WalkPlan& plan) {
   // 32 us in 448 CTAs of 128x32 and in 1792 of 128x8, 52 us in 64x4.  One 480x640
   // image to 224x224 fills no wave of any size and is quickest in the smallest
   // cells: 14.4 us a call in 64x4, 18 in 128x8.
-  static const int kCells[][2] = {{128, 32}, {128, 16}, {128, 8}, {64, 8}, {64, 4}};
+  static const int kCells[][2] = {{kWalkMaxPx, 32}, {kWalkMaxPx, 16}, {kWalkMaxPx, 8}, {64, 8}, {64, 4}};
   constexpr long long kWantCtas = 148 * 2;
   for (const auto& cell : kCells) {
     long long ctas = 0;

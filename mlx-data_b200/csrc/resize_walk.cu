@@ -63,8 +63,8 @@ struct WalkSmem {
   unsigned hw;      // float [tap][walk_px]
 };
 
-__host__ __device__ inline size_t walk_layout(int c_out, const WalkPlan& w, unsigned base, WalkSmem* out) {
-  WalkSmem sm;
+__host__ __device__ constexpr size_t walk_layout(int c_out, const WalkPlan& w, unsigned base, WalkSmem* out) {
+  WalkSmem sm{};
   size_t off = 0;
   sm.mid = base;
   off += kMidBytes;
@@ -653,12 +653,18 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
   }
 }
 
+// No plan needs more shared memory than this.
+constexpr size_t kWalkMaxSmem = walk_layout(4, WalkPlan{kWalkMaxPx, kWalkMaxTaps, kWalkMaxSteps, 0, 0}, 0u, nullptr);
+
 template <int C, bool GRAY, bool U8>
 cudaError_t launch(const LaunchParams& p, unsigned blocks, size_t smem, cudaStream_t stream) {
-  // the attribute belongs to the kernel on the current device; only strong shrinks need it
+  // Only strong shrinks need more than the 48 KB that every kernel may have.  The
+  // limit belongs to the kernel on the current device and is shared by all host
+  // threads, so each of them sets the same value: one that set its own launch's
+  // need could lower the limit between another's setting and its launch.
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(
-        resize_walk_kernel<C, GRAY, U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        resize_walk_kernel<C, GRAY, U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkMaxSmem);
     if (e != cudaSuccess) {
       return e;
     }

@@ -1,0 +1,50 @@
+"""Two host threads that launch resizes of different shared-memory need at the
+same time: neither lowers the kernel's limit under the other."""
+import threading
+
+import numpy as np
+import pytest
+
+import chain
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("c", [1, 3, 4])
+def test_two_threads_of_strong_shrinks(pkg, ctx, oracle, c):
+    rows = (4, 5)   # from 2000: plans of 57 to 60 KB and of 51 to 54 KB
+    torch = pytest.importorskip("torch")
+    capi = pkg._capi
+    rng = np.random.default_rng(c)
+    img = rng.integers(0, 256, (2000, 24, c), dtype=np.uint8)
+    dev = torch.from_numpy(img).cuda()
+    torch.cuda.synchronize()
+    outs = [torch.zeros((1, h, 20, c), dtype=torch.float32, device="cuda") for h in rows]
+    torch.cuda.synchronize()
+    failed = []
+    start = threading.Barrier(2)
+
+    def work(lane):
+        h = rows[lane]
+        descs = np.zeros(1, pkg.SAMPLE_DTYPE)
+        chain.fill_descs(descs, 0, chain.reduce_chain(img.shape, [("image_resize", dict(key="image", w=20, h=h))]),
+                         dev.data_ptr())
+        bd = pkg.make_batch_desc(outs[lane].data_ptr(), h, 20, c, src_mem=capi.MEM_DEVICE, dst_mem=capi.MEM_DEVICE)
+        start.wait()
+        for i in range(3000):
+            try:
+                ctx.fused_batch(lane, descs, bd)
+            except pkg.MlxdError as e:
+                failed.append((lane, i, str(e)))
+                break
+        ctx.wait(lane)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+    for h, out in zip(rows, outs):
+        want = oracle.resize(img, 20, h).astype(np.float32) / np.float32(255)
+        assert np.array_equal(out[0].cpu().numpy(), want)
