@@ -138,8 +138,10 @@ Sample Batcher::run(const std::vector<const Sample*>& raw) const {
       run_op(lazy.back(), *op);
     }
   }
-  // 2. per key of the first sample: one batch tensor
+  // 2. per key of the first sample: one batch tensor.  Casts come after the batch in
+  // the chain: what they make goes in last, in their order, over a batch of that key.
   Sample out;
+  std::vector<std::shared_ptr<Array>> cast_results(casts_.size());
   std::vector<Entry*> col;
   std::vector<gpu::LazyImage> made;             // programs of entries that are plain arrays, or were computed on their own
   std::vector<const gpu::LazyImage*> images;
@@ -184,16 +186,11 @@ Sample Batcher::run(const std::vector<const Sample*>& raw) const {
         throw std::runtime_error("BatchShape: batched arrays expected to have consistent shapes");
       }
       bool replaced = false;
-      for (auto& c : casts_) {
-        if (c.ikey != key) {
-          continue;
-        }
-        auto f32 = gpu::Runtime::get().batch(images, pad, &c.spec, placement_);
-        if (c.okey.empty() || c.okey == key) {
-          out[key] = f32;
-          replaced = true;
-        } else {
-          out[c.okey] = f32;
+      for (size_t k = 0; k < casts_.size(); k++) {
+        const CastRequest& c = casts_[k];
+        if (c.ikey == key) {
+          cast_results[k] = gpu::Runtime::get().batch(images, pad, &c.spec, placement_);
+          replaced = replaced || c.okey.empty() || c.okey == key;
         }
       }
       if (!replaced) {
@@ -209,10 +206,15 @@ Sample Batcher::run(const std::vector<const Sample*>& raw) const {
     std::shared_ptr<Array> merged =
         dim == batch_dims_.end() ? array::batch(arrs, pad) : array::batch(arrs, dim->second, pad);
     out[key] = merged;
-    for (auto& c : casts_) {
-      if (c.ikey == key) {
-        out[c.okey.empty() ? key : c.okey] = gpu::Runtime::get().cast(merged, c.spec);
+    for (size_t k = 0; k < casts_.size(); k++) {
+      if (casts_[k].ikey == key) {
+        cast_results[k] = gpu::Runtime::get().cast(merged, casts_[k].spec);
       }
+    }
+  }
+  for (size_t k = 0; k < casts_.size(); k++) {
+    if (cast_results[k]) {
+      out[casts_[k].okey.empty() ? casts_[k].ikey : casts_[k].okey] = cast_results[k];
     }
   }
   return out;
