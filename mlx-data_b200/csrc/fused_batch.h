@@ -58,9 +58,14 @@ struct WalkPlan {
   int32_t px;         // columns of the widest chunk (0: no sample runs the resize kernel)
   int32_t taps;       // horizontal weights of a chunk
   int32_t steps;      // source rows of a walk
-  int32_t cells_y;    // grid of the sample with the most cells
-  int32_t cells_x;
+  int32_t cells_y;    // grid of cells of every sample, the most rows and the most columns of any of them;
+  int32_t cells_x;    // or 0 rows: cells_x CTAs per sample, which counts its own cells off
 };
+
+// Strips of padding beside the post window.
+__host__ __device__ inline int walk_strips(const DevSample& s) {
+  return (s.slot_w - s.post_w + kWalkPadPx - 1) / kWalkPadPx;
+}
 
 struct LaunchParams {
   const DevSample* samples;

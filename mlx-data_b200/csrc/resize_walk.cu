@@ -597,7 +597,8 @@ __device__ __noinline__ void starve(const LaunchParams& p, unsigned bar) {
 }
 
 // One cell: walk_rows rows x one chunk (or one strip of padding) of a slot.
-template <int C, bool GRAY, bool U8>
+// OWN: samples count their own cells off (WalkPlan::cells_y of 0).
+template <int C, bool GRAY, bool U8, bool OWN>
 __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __grid_constant__ LaunchParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int CO = GRAY ? 1 : C;
@@ -610,16 +611,25 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
     }
     t -= min(t / every + 1, fills);
   }
-  const int cx = t % p.walk.cells_x;
+  const unsigned cell = t % p.walk.cells_x;
   t /= p.walk.cells_x;
-  const int cy = t % p.walk.cells_y;
-  const DevSample& s = p.samples[t / p.walk.cells_y];
+  int cx = (int)cell;
+  int cy = OWN ? 0 : (int)(t % p.walk.cells_y);
+  const DevSample& s = p.samples[OWN ? t : t / p.walk.cells_y];
   if (s.mode != kModeResize) {
     return;   // the other kernels'
   }
   const int slot_h = s.slot_h, slot_w = s.slot_w, post_h = s.post_h, post_w = s.post_w;
-  const int y0 = cy * s.walk_rows;
   const int chunks = s.walk_chunks;
+  if (OWN) {
+    const unsigned cells_x = (unsigned)(chunks + walk_strips(s));
+    cx = (int)(cell % cells_x);
+    cy = (int)(cell / cells_x);
+    if (cy >= (slot_h + s.walk_rows - 1) / s.walk_rows) {
+      return;
+    }
+  }
+  const int y0 = cy * s.walk_rows;
   // the chunks share the post window's columns evenly; strips of kWalkPadPx behind it
   const bool strip = cx >= chunks;
   const int x0 = strip ? post_w + (cx - chunks) * kWalkPadPx : (int)((long long)post_w * cx / chunks);
@@ -656,28 +666,34 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
 // No plan needs more shared memory than this.
 constexpr size_t kWalkMaxSmem = walk_layout(4, WalkPlan{kWalkMaxPx, kWalkMaxTaps, kWalkMaxSteps, 0, 0}, 0u, nullptr);
 
-template <int C, bool GRAY, bool U8>
-cudaError_t launch(const LaunchParams& p, unsigned blocks, size_t smem, cudaStream_t stream) {
+template <int C, bool GRAY, bool U8, bool OWN>
+cudaError_t launch_kernel(const LaunchParams& p, unsigned blocks, size_t smem, cudaStream_t stream) {
   // Only strong shrinks need more than the 48 KB that every kernel may have.  The
   // limit belongs to the kernel on the current device and is shared by all host
   // threads, so each of them sets the same value: one that set its own launch's
   // need could lower the limit between another's setting and its launch.
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(
-        resize_walk_kernel<C, GRAY, U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkMaxSmem);
+        resize_walk_kernel<C, GRAY, U8, OWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkMaxSmem);
     if (e != cudaSuccess) {
       return e;
     }
   }
-  resize_walk_kernel<C, GRAY, U8><<<blocks, kWalkThreads, smem, stream>>>(p);
+  resize_walk_kernel<C, GRAY, U8, OWN><<<blocks, kWalkThreads, smem, stream>>>(p);
   return cudaGetLastError();
+}
+
+template <int C, bool GRAY, bool U8>
+cudaError_t launch(const LaunchParams& p, unsigned blocks, size_t smem, cudaStream_t stream) {
+  return p.walk.cells_y == 0 ? launch_kernel<C, GRAY, U8, true>(p, blocks, smem, stream)
+                          : launch_kernel<C, GRAY, U8, false>(p, blocks, smem, stream);
 }
 
 } // namespace
 
 cudaError_t launch_resize_walk(const LaunchParams& p_in, cudaStream_t stream) {
   LaunchParams p = p_in;
-  unsigned long long blocks = (unsigned long long)p.n * p.walk.cells_y * p.walk.cells_x;
+  unsigned long long blocks = (unsigned long long)p.n * std::max(p.walk.cells_y, 1) * p.walk.cells_x;
   if (blocks == 0) {
     return cudaSuccess;
   }
