@@ -191,7 +191,7 @@ MLXD_API int mlxd_ctx_set_timing(mlxd_ctx* ctx, int on);
  *    overlap on the GPU - different streams, or different host threads - race;
  *    order them on one stream;
  *  - the kernel's self-check word (a resize chunk beyond its planned shared
- *    memory, a bounded wait that ran out) is read back at the start of the NEXT call on the same stream,
+ *    memory) is read back at the start of the NEXT call on the same stream,
  *    which then returns MLXD_ERR_DEVICE and launches nothing; after the last
  *    call of a run ask mlxd_noalloc_status. */
 #define MLXD_NOALLOC_MAX_SAMPLES 1024
@@ -225,9 +225,8 @@ MLXD_API int mlxd_fused_batch_on_stream(
 
 /* Self-check word of the kernels launched by mlxd_fused_batch_on_stream: waits
  * for `cuda_stream`, stores the word in *status (0 = clean; 8: a resize chunk with
- * more source rows or bytes than planned, 4: a bounded wait ran out, which only
- * the test hook MLXD_TEST_STARVE_WAIT does), clears it, and returns
- * MLXD_ERR_DEVICE when it was set.  The lanes of mlxd_fused_batch report the
+ * more source rows or bytes than planned, whose rows were then not written), clears
+ * it, and returns MLXD_ERR_DEVICE when it was set.  The lanes of mlxd_fused_batch report the
  * same word through mlxd_batch_wait.  No counterpart in the reference, whose
  * CPU ops throw where they stand. */
 MLXD_API int mlxd_stream_status(mlxd_ctx* ctx, void* cuda_stream, int32_t* status);

@@ -207,7 +207,16 @@ int plan_samples(
     const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b,
     std::vector<DevSample>& out, WalkPlan& walk) {
   out.resize(n);
-  return plan_into(samples, n, b, out.data(), walk);
+  const int rc = plan_into(samples, n, b, out.data(), walk);
+  // Test hook (MLXD_TEST_SHORT_PLAN=1, read per launch): room for one step a walk.
+  // Every resize CTA that has more finds that before it copies or filters anything,
+  // sets the status word and returns, so the kernel's self-check and the way from it
+  // to the caller's error code can be exercised without a fault or a hang.
+  const char* hook = std::getenv("MLXD_TEST_SHORT_PLAN");
+  if (hook && hook[0] == '1' && walk.steps > 1) {
+    walk.steps = 1;
+  }
+  return rc;
 }
 
 // Source samples of an n_src -> n_dst axis that outputs [o_lo, o_hi) can read,
@@ -343,11 +352,6 @@ int prepare_launch(
   p.out_f32 = b->out_dtype == MLXD_F32;
   p.pad_px = (int32_t)(uint8_t)(int32_t)b->pad_value;
   p.status = ctx->d_status;   // callers point this at their lane's word
-  // Test hook (MLXD_TEST_STARVE_WAIT=1, read per launch): the resize bands'
-  // first bounded wait runs out, so the path from the kernel's status word to
-  // the caller's error code can be exercised without a fault or a hang.
-  const char* starve = std::getenv("MLXD_TEST_STARVE_WAIT");
-  p.starve_wait = (starve && starve[0] == '1') ? 1 : 0;
   if (p.out_f32) {
     if (!(b->divisor != 0.0f)) {
       return fail(MLXD_ERR_INVALID, "cast divisor must be non-zero");

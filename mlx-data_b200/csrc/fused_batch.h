@@ -87,7 +87,6 @@ struct LaunchParams {
   int32_t pad_apart;          // the rows below each post window are filled apart from the cells around them
   int32_t fill_every;         // resize kernel, then: every so many CTAs, from the first on, one of them fills
   int32_t direct;             // some sample is kModeResizeDirect: resize_direct_kernel runs last
-  int32_t starve_wait;        // test hook: every resize CTA first waits for 16 bytes that no copy delivers
 };
 
 // Launch the kernels the parameters call for: the resize kernel or, without a

@@ -568,34 +568,6 @@ __device__ __forceinline__ void walk_chunk(
   }
 }
 
-// Polls of an mbarrier before a wait gives up: about a second (a poll that finds
-// the phase incomplete returns after a few microseconds).
-constexpr unsigned kSpinLimit = 1u << 18;
-
-// Test hook (LaunchParams::starve_wait): a bounded wait for bytes that never
-// arrive runs out, to exercise the way from the status word to the caller's
-// error code.
-__device__ __noinline__ void starve(const LaunchParams& p, unsigned bar) {
-  if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], 16;" ::"r"(bar) : "memory");
-    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(bar) : "memory");
-    unsigned done = 0;
-    for (unsigned i = 0; i < kSpinLimit && !done; i++) {
-      asm volatile(
-          "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-          : "=r"(done)
-          : "r"(bar)
-          : "memory");
-    }
-    if (!done) {
-      atomicOr(p.status, 4);
-    }
-    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-  }
-  __syncthreads();
-}
-
 // One cell: walk_rows rows x one chunk (or one strip of padding) of a slot.
 // OWN: samples count their own cells off (WalkPlan::cells_y of 0).
 template <int C, bool GRAY, bool U8, bool OWN>
@@ -644,9 +616,6 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
   if (!strip && y0 < vy1) {
     WalkSmem sm;
     walk_layout(p.c_out, p.walk, smem_addr(smem_raw), &sm);
-    if (p.starve_wait) {
-      starve(p, sm.mid);
-    }
     walk_chunk<C, GRAY, U8>(s, p, sm, y0, vy1, x0, x1);
   }
   if (fill_y0 < fill_y1) {

@@ -1,7 +1,8 @@
 """Failure reporting without a fault: a lane wait that runs out of time, and a
-kernel whose bounded wait runs out (a test hook makes the first resize pass
-expect bytes that no copy delivers).  In both cases the caller gets an error
-code, nothing hangs, and the same context goes on to produce correct batches."""
+resize kernel that finds more source rows than its launch was planned for (a
+test hook understates the plan; the CTAs return before they filter anything).
+In both cases the caller gets an error code, nothing hangs, and the same context
+goes on to produce correct batches."""
 import os
 
 import numpy as np
@@ -50,20 +51,20 @@ def test_lane_wait_times_out_and_recovers(pkg, oracle):
         own.close()
 
 
-def test_bounded_wait_runs_out_is_reported_and_cleared(pkg, oracle):
+def test_walk_beyond_its_plan_is_reported_and_cleared(pkg, oracle):
     capi = pkg._capi
     own = pkg.Context(device=0, n_lanes=1)
     rng = np.random.default_rng(1)
-    samples = [{"image": rng.integers(0, 256, (60, 90, 3), dtype=np.uint8)}]     # one band, one pass
+    samples = [{"image": rng.integers(0, 256, (60, 90, 3), dtype=np.uint8)}]
     descs, fields = _descs(pkg, samples, OPS)
     out = np.zeros((1, 40, 48, 3), np.float32)
     bd = pkg.make_batch_desc(out, 40, 48, 3)
     try:
-        os.environ["MLXD_TEST_STARVE_WAIT"] = "1"
+        os.environ["MLXD_TEST_SHORT_PLAN"] = "1"
         try:
             own.fused_batch(0, descs, bd)
         finally:
-            os.environ.pop("MLXD_TEST_STARVE_WAIT", None)
+            os.environ.pop("MLXD_TEST_SHORT_PLAN", None)
         with pytest.raises(pkg.MlxdError) as e:
             own.wait(0)
         assert e.value.code == capi.ERR_DEVICE and "self-check" in str(e.value)
@@ -76,3 +77,29 @@ def test_bounded_wait_runs_out_is_reported_and_cleared(pkg, oracle):
         assert d.max() <= 1.0001 / 255 and (d > 0).mean() <= 1e-3
     finally:
         own.close()
+
+
+def test_walk_beyond_its_plan_on_a_stream(pkg, ctx, oracle):
+    """The rows that were not filtered keep what the batch held, the padding around them is written."""
+    torch = pytest.importorskip("torch")
+    capi = pkg._capi
+    stream = torch.cuda.current_stream().cuda_stream
+    img = np.random.default_rng(2).integers(0, 256, (200, 90, 3), dtype=np.uint8)
+    src = torch.from_numpy(img).cuda()
+    descs = np.zeros(1, pkg.SAMPLE_DTYPE)
+    chain.fill_descs(descs, 0, chain.reduce_chain(img.shape, OPS), src.data_ptr())
+    out = torch.full((1, 50, 300, 3), -1.0, device="cuda")
+    bd = pkg.make_batch_desc(out.data_ptr(), 50, 300, 3, pad_value=255.0, src_mem=capi.MEM_DEVICE, dst_mem=capi.MEM_DEVICE)
+    os.environ["MLXD_TEST_SHORT_PLAN"] = "1"
+    try:
+        ctx.fused_batch_on_stream(stream, descs, bd)
+    finally:
+        os.environ.pop("MLXD_TEST_SHORT_PLAN", None)
+    assert ctx.stream_status(stream) == 8
+    assert ctx.stream_status(stream) == 0
+    got = out[0].cpu().numpy()
+    assert (got[:40, :48] == -1).all() and (got[40:] == 1).all() and (got[:, 48:] == 1).all()
+    ctx.fused_batch_on_stream(stream, descs, bd)
+    assert ctx.stream_status(stream) == 0
+    want = oracle.resize(img, 48, 40).astype(np.float32) / np.float32(255)
+    assert np.array_equal(out[0, :40, :48].cpu().numpy(), want)
