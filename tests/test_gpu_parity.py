@@ -311,10 +311,10 @@ def test_float32_resize_cases(pkg, ctx, oracle, case, cast):
     _compare(got, want, True, cast)
 
 
-# ---------------------------------------------------------------- shrink ratios beyond the on-chip passes
-DIRECT_RESIZE_CASES = [
-    # one output row of these takes more source rows (2 * ratio + 1) than a pass can stage (192): every
-    # pixel is filtered from global memory by the kernel for such samples
+# ---------------------------------------------------------------- strong shrinks
+STRONG_SHRINK_CASES = [
+    # one output row of these takes 200 to 600 source rows: walks of one output row per CTA, chunks of a
+    # few columns (the shrinks that the resize kernel leaves to another are in test_gpu_resize_limits.py)
     ((1500, 1500), 3, [("image_resize", dict(key="image", w=12, h=12))]),
     ((2100, 64), 1, [("image_resize", dict(key="image", w=32, h=10))]),
     ((1300, 900), 4, [("image_random_h_flip", dict(key="image", prob=1.0)),
@@ -326,12 +326,12 @@ DIRECT_RESIZE_CASES = [
 ]
 
 
-@pytest.mark.parametrize("case", range(len(DIRECT_RESIZE_CASES)))
+@pytest.mark.parametrize("case", range(len(STRONG_SHRINK_CASES)))
 @pytest.mark.parametrize("cast", [None, (), "norm"])
-def test_resize_beyond_the_on_chip_footprint(pkg, ctx, oracle, case, cast):
-    """A batch of two such samples and one small image that takes the staged
-    passes, same chain: uint8, float32 and normalised float32 out."""
-    (h, w), c, ops = DIRECT_RESIZE_CASES[case]
+def test_strong_shrinks(pkg, ctx, oracle, case, cast):
+    """A batch of two such samples and one small image, same chain: uint8,
+    float32 and normalised float32 out."""
+    (h, w), c, ops = STRONG_SHRINK_CASES[case]
     rng = np.random.default_rng(500 + case)
     shapes = [(h, w), (h - 7, w - 3), (57, 64)]
     samples = [{"image": rng.integers(0, 256, (a, b, c), dtype=np.uint8)} for a, b in shapes]
@@ -342,7 +342,7 @@ def test_resize_beyond_the_on_chip_footprint(pkg, ctx, oracle, case, cast):
     _compare(got, want, True, cast)
 
 
-def test_resize_beyond_the_on_chip_footprint_gray(pkg, ctx, oracle):
+def test_strong_shrinks_gray(pkg, ctx, oracle):
     ops = [("image_resize", dict(key="image", w=14, h=9)),
            ("image_channel_reduction", dict(key="image", preset="default"))]
     rng = np.random.default_rng(77)
