@@ -26,9 +26,10 @@ constexpr int kPadChunks = 128;     // CTAs that fill the rows below one sample
 constexpr int kWalkPadPx = 256;     // columns per strip of padding
 
 // kModeResizeDirect: a resize whose taps do not fit one chunk of the resize
-// kernel (shrink ratios of about 100 and more along a row, 300 down the rows);
-// every output pixel is then filtered straight from global memory by
-// resize_direct_kernel.
+// kernel: one column's 2r + 2 source columns exceed kWalkRow bytes (shrink ratios r
+// above 412, 205, 136, 102 along a row for 1 to 4 channels) or one row's 2r + 11
+// steps exceed kWalkMaxSteps (above 506 down the rows).  Every output pixel is then
+// filtered straight from global memory by resize_direct_kernel.
 enum Mode : int32_t { kModeCopy = 0, kModeResize = 1, kModeAffine = 2, kModeResizeDirect = 3 };
 
 // One sample's program.  Coordinates name four nested images:

@@ -5,8 +5,9 @@
 // Copy and affine: one CTA per band of up to eight kTileH x kTileW tiles of one
 // sample's slot; the source is read through the read-only path, four pixels per
 // thread, and stored 16 bytes at a time; pad-only bands are plain 16-byte
-// stores.  The rows below a sample in a ragged batch go out through a linear
-// fill kernel.  A resize too strong for the resize kernel is filtered pixel by
+// stores.  The rows below a sample in a ragged batch go out through a linear fill
+// kernel when the launch has no resize (else CTAs of the resize kernel write them).
+// A resize too strong for the resize kernel is filtered pixel by
 // pixel from global memory by a kernel of its own.
 #include "fused_batch.h"
 #include "kernel_common.cuh"
@@ -173,54 +174,54 @@ __device__ void gather_rows(
         }
       }
     } else {
-    float out[4][CO];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      if (GRAY) {
-        out[j][0] = __uint_as_float(lds_u32<0>(lut_s + 4u * gray_mix(p, px[j][0], px[j][1 % C], px[j][2 % C])));
-      } else {
-#pragma unroll
-        for (int ch = 0; ch < C; ch++) {
-          out[j][ch % CO] = __uint_as_float(lds_u32<0>(lut_s + (unsigned)ch * 1024u + 4u * px[j][ch]));
-        }
-      }
-    }
-    float* dst = base + ((size_t)(y0 + ry) * s.slot_w + x_first) * CO;
-    if (vec_ok && npx == 4) {
-      const float* o = &out[0][0];
-#pragma unroll
-      for (int k = 0; k < CO; k++) {
-        reinterpret_cast<float4*>(dst)[k] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
-      }
-    } else if (CO > 1 && npx == 4) {
-      // A row that starts off a 16-byte boundary (odd widths).  Single floats alone, a
-      // lane's 4 * CO apart from the next lane's, bring each 32-byte sector to L2 once per
-      // float in it: 64 mirrored images of 719x1279x3 487 us a pass, 259 with these units.
-      const float* o = &out[0][0];
-      switch ((reinterpret_cast<uintptr_t>(dst) >> 2) & 3) {
-        case 0:
-          store_run<4 * CO, 0>(dst, o);
-          break;
-        case 1:
-          store_run<4 * CO, 3>(dst, o);
-          break;
-        case 2:
-          store_run<4 * CO, 2>(dst, o);
-          break;
-        default:
-          store_run<4 * CO, 1>(dst, o);
-      }
-    } else {
+      float out[4][CO];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        if (j < npx) {
+        if (GRAY) {
+          out[j][0] = __uint_as_float(lds_u32<0>(lut_s + 4u * gray_mix(p, px[j][0], px[j][1 % C], px[j][2 % C])));
+        } else {
 #pragma unroll
-          for (int ch = 0; ch < CO; ch++) {
-            dst[j * CO + ch] = out[j][ch];
+          for (int ch = 0; ch < C; ch++) {
+            out[j][ch % CO] = __uint_as_float(lds_u32<0>(lut_s + (unsigned)ch * 1024u + 4u * px[j][ch]));
           }
         }
       }
-    }
+      float* dst = base + ((size_t)(y0 + ry) * s.slot_w + x_first) * CO;
+      if (vec_ok && npx == 4) {
+        const float* o = &out[0][0];
+#pragma unroll
+        for (int k = 0; k < CO; k++) {
+          reinterpret_cast<float4*>(dst)[k] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
+        }
+      } else if (CO > 1 && npx == 4) {
+        // A row that starts off a 16-byte boundary (odd widths).  Single floats alone, a
+        // lane's 4 * CO apart from the next lane's, bring each 32-byte sector to L2 once per
+        // float in it: 64 mirrored images of 719x1279x3 487 us a pass, 259 with these units.
+        const float* o = &out[0][0];
+        switch ((reinterpret_cast<uintptr_t>(dst) >> 2) & 3) {
+          case 0:
+            store_run<4 * CO, 0>(dst, o);
+            break;
+          case 1:
+            store_run<4 * CO, 3>(dst, o);
+            break;
+          case 2:
+            store_run<4 * CO, 2>(dst, o);
+            break;
+          default:
+            store_run<4 * CO, 1>(dst, o);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          if (j < npx) {
+#pragma unroll
+            for (int ch = 0; ch < CO; ch++) {
+              dst[j * CO + ch] = out[j][ch];
+            }
+          }
+        }
+      }
     }
   }
 }
@@ -266,7 +267,7 @@ __device__ void run_band(const LaunchParams& p, float* lut_s) {
     }
   };
   if (!has_valid) {
-    // bands below the post window are pad_fill_kernel's when it runs
+    // bands below the post window are filled apart when p.pad_apart is set
     if (!(p.pad_apart && y0 >= s.post_h)) {
       pad_rect(y0, y1, x0, x1);
     }
@@ -340,15 +341,15 @@ __global__ void __launch_bounds__(kThreads, 3) fused_fast_gray_kernel(const Laun
 
 } // namespace
 
-// ---- resizes whose taps do not fit the on-chip passes ---------------------------------
+// ---- resizes whose taps do not fit a chunk of the resize kernel ------------------------
 //
 // One thread per pixel of the post window, every tap read from global memory.
-// The arithmetic is that of the band kernel, value by value: per source column
-// the vertical sum (first tap a product, then multiply-adds in tap order, taps
-// outside the window reading the clamped row), then the horizontal
-// multiply-adds over those sums in tap order onto zero, weights tent / sum
-// with the sum taken in tap order.  Such samples are rare and small on the
-// output side (a shrink ratio of 60 or more), so nothing is staged or shared.
+// The arithmetic is that of the resize kernel, value by value: per source column
+// the vertical sum (multiply-adds in tap order, the first of them a product, taps
+// outside the window reading the clamped row), then the horizontal multiply-adds
+// over those sums in tap order onto zero, weights tent / sum with the sum taken in
+// tap order.  Such samples are rare and small on the output side (walk_fits: shrink
+// ratios above 100 along a row, 500 down the rows), so nothing is staged or shared.
 template <int C>
 __device__ void direct_pixel(const DevSample& s, const LaunchParams& p, int ox, int oy) {
   const Axis ay = make_axis(s.pre_h, s.geom_h);

@@ -55,34 +55,6 @@ __device__ __forceinline__ float axis_tent(const Axis& a, float u, int i) {
   return v > 0.0f ? v : 0.0f;
 }
 
-// Tap range and normalised weights of output sample o; at most cap taps.
-__device__ __forceinline__ void axis_taps(
-    int n, int m, int o, int cap, int& first, int& count, float* w) {
-  if (n == m) {
-    first = o;
-    count = 1;
-    w[0] = 1.0f;
-    return;
-  }
-  const Axis a = make_axis(n, m);
-  const float u = axis_center(a, o);
-  int lo, hi;
-  axis_range(a, o, lo, hi);
-  int cnt = hi - lo + 1;
-  cnt = cnt > cap ? cap : cnt;
-  float sum = 0.0f;
-  for (int k = 0; k < cnt; k++) {
-    const float v = axis_tent(a, u, lo + k);
-    w[k] = v;
-    sum = __fadd_rn(sum, v);
-  }
-  for (int k = 0; k < cnt; k++) {
-    w[k] = __fdiv_rn(w[k], sum);
-  }
-  first = lo;
-  count = cnt;
-}
-
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -101,12 +73,6 @@ typedef unsigned long long f32x2;
 // identical to fmaf).
 __device__ __forceinline__ void ffma2(f32x2& d, f32x2 a, f32x2 b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-
-__device__ __forceinline__ f32x2 fmul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
 }
 
 __device__ __forceinline__ f32x2 pack2(float lo, float hi) {
@@ -300,12 +266,12 @@ __device__ __forceinline__ void fill_rect_u8(
 }
 
 // The padding below a sample of a ragged batch.  Rows of a slot are contiguous,
-// so everything below the sample's post
-// window down to the end of the slot is one contiguous run of floats: written
-// here as a linear fill (16-byte stores, consecutive threads on consecutive
-// addresses, kPadChunks CTAs per sample), which runs at memory speed - the
-// band kernels above, writing 16-row strips, reach about 60 % of that.  The
-// strips to the right of the post window stay with the band kernels.
+// so everything below the sample's post window down to the end of the slot is one
+// contiguous run of floats: written here as a linear fill (16-byte stores,
+// consecutive threads on consecutive addresses, kPadChunks CTAs per sample), which
+// runs at memory speed (7.7 TB/s; the 16-row strips of the band kernel 4.5).  The
+// strips to the right of the post window are the band kernel's, or cells of the
+// resize kernel.
 template <int CO>
 __device__ __forceinline__ void pad_below(const LaunchParams& p, unsigned block) {
   const int n = (int)(block / kPadChunks);
