@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kThreads, 3) fused_fast_u8_kernel(const Launch
 }
 
 __global__ void __launch_bounds__(kThreads, 6) pad_fill_kernel(const LaunchParams p) {
-  pad_below_any(p, blockIdx.x);
+  pad_below_any<kThreads>(p, blockIdx.x);
 }
 
 // Launches that end in the channel reduction: three channels in, one out.  A

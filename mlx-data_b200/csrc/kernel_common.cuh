@@ -271,8 +271,9 @@ __device__ __forceinline__ void fill_rect_u8(
 // consecutive threads on consecutive addresses, kPadChunks CTAs per sample), which
 // runs at memory speed (7.7 TB/s; the 16-row strips of the band kernel 4.5).  The
 // strips to the right of the post window are the band kernel's, or cells of the
-// resize kernel.
-template <int CO>
+// resize kernel.  THREADS is a CTA's thread count: read from blockDim, it made the
+// fill kernel spill (64 images of 64x64 in slots of 4000x100: 99.3 us a pass, 96.5 so).
+template <int CO, int THREADS>
 __device__ __forceinline__ void pad_below(const LaunchParams& p, unsigned block) {
   const int n = (int)(block / kPadChunks);
   const int chunk = (int)(block % kPadChunks);
@@ -301,7 +302,7 @@ __device__ __forceinline__ void pad_below(const LaunchParams& p, unsigned block)
   // this CTA's share of the aligned units
   const size_t q0 = nvec * (size_t)chunk / kPadChunks;
   const size_t q1 = nvec * (size_t)(chunk + 1) / kPadChunks;
-  for (size_t q = q0 + threadIdx.x; q < q1; q += (int)blockDim.x) {
+  for (size_t q = q0 + threadIdx.x; q < q1; q += THREADS) {
     const size_t j = head + 4 * q;
     const int m = (int)(j % CO);
     *reinterpret_cast<float4*>(run + j) = make_float4(
@@ -311,7 +312,7 @@ __device__ __forceinline__ void pad_below(const LaunchParams& p, unsigned block)
   if (chunk == 0) {
     // the floats before the first and after the last aligned unit
     const size_t tail = head + 4 * nvec;
-    for (size_t k = threadIdx.x; k < head + (len - tail); k += (int)blockDim.x) {
+    for (size_t k = threadIdx.x; k < head + (len - tail); k += THREADS) {
       const size_t j = k < head ? k : tail + (k - head);
       run[j] = pad_pick<CO>(padf, (int)(j % CO));
     }
@@ -319,6 +320,7 @@ __device__ __forceinline__ void pad_below(const LaunchParams& p, unsigned block)
 }
 
 // The same for a uint8 batch: a linear fill of bytes.
+template <int THREADS>
 __device__ __forceinline__ void pad_below_u8(const LaunchParams& p, unsigned block) {
   const int n = (int)(block / kPadChunks);
   const int chunk = (int)(block % kPadChunks);
@@ -343,29 +345,30 @@ __device__ __forceinline__ void pad_below_u8(const LaunchParams& p, unsigned blo
   const uint4 v = make_uint4(w, w, w, w);
   const size_t q0 = nvec * (size_t)chunk / kPadChunks;
   const size_t q1 = nvec * (size_t)(chunk + 1) / kPadChunks;
-  for (size_t q = q0 + threadIdx.x; q < q1; q += (int)blockDim.x) {
+  for (size_t q = q0 + threadIdx.x; q < q1; q += THREADS) {
     *reinterpret_cast<uint4*>(run + head + 16 * q) = v;
   }
   if (chunk == 0) {
     const size_t tail = head + 16 * nvec;
-    for (size_t k = threadIdx.x; k < head + (len - tail); k += (int)blockDim.x) {
+    for (size_t k = threadIdx.x; k < head + (len - tail); k += THREADS) {
       run[k < head ? k : tail + (k - head)] = (uint8_t)p.pad_px;
     }
   }
 }
 
 // Block `block` of n * kPadChunks.
+template <int THREADS>
 __device__ __forceinline__ void pad_below_any(const LaunchParams& p, unsigned block) {
   if (!p.out_f32) {
-    pad_below_u8(p, block);
+    pad_below_u8<THREADS>(p, block);
   } else if (p.c_out == 3) {
-    pad_below<3>(p, block);
+    pad_below<3, THREADS>(p, block);
   } else if (p.c_out == 1) {
-    pad_below<1>(p, block);
+    pad_below<1, THREADS>(p, block);
   } else if (p.c_out == 2) {
-    pad_below<2>(p, block);
+    pad_below<2, THREADS>(p, block);
   } else {
-    pad_below<4>(p, block);
+    pad_below<4, THREADS>(p, block);
   }
 }
 
