@@ -669,10 +669,10 @@ cudaError_t launch_resize_walk(const LaunchParams& p_in, cudaStream_t stream) {
   if (p.pad_apart) {
     // Filling is bound by memory writes, walking by the SMs: the fill CTAs go
     // among the others, evenly, instead of into a launch of their own.  64 images
-    // of 160-1024 px padded to the largest (2 GB written): 384 us a pass; in a launch
-    // before this one, when it took 398, 449.  Where they are more than the walking CTAs (small slots) all of
-    // them come first: 64 images of 100-400 px, shorter side 128, 74 us a pass, 256 of
-    // 30-120 px, shorter side 32, 87.
+    // of 160-1024 px padded to the largest (2 GB written): 384 us a pass (in a
+    // launch before this one, when it took 398: 449).  Where they are more than
+    // the walking CTAs (small slots) all of them come first: 64 images of 100-400
+    // px, shorter side 128, 74 us a pass, 256 of 30-120 px, shorter side 32, 87.
     const unsigned long long fills = (unsigned long long)p.n * kPadChunks;
     blocks += fills;
     p.fill_every = (int32_t)std::max<unsigned long long>(1, std::min<unsigned long long>(blocks / fills, 1u << 30));
