@@ -173,8 +173,13 @@ int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, 
       if (d.pre_w == d.geom_w && d.pre_h == d.geom_h) {
         s.mode = kModeCopy;  // identity on both axes
       } else {
-        s.mode = walk_fits(s, b->channels) ? kModeResize : kModeResizeDirect;
         s.cap_x = plan_axis(s.pre_w, s.geom_w, 1).cap;
+        s.mode = resize_mode(s, b->channels);
+        // the divisions of make_axis(), correctly rounded here as there
+        s.axis_x[0] = (float)s.pre_w / (float)s.geom_w;
+        s.axis_x[1] = std::min(1.0f, (float)s.geom_w / (float)s.pre_w);
+        s.axis_y[0] = (float)s.pre_h / (float)s.geom_h;
+        s.axis_y[1] = std::min(1.0f, (float)s.geom_h / (float)s.pre_h);
       }
     } else if (d.geom == MLXD_GEOM_AFFINE) {
       s.mode = kModeAffine;
@@ -192,29 +197,30 @@ int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, 
   return MLXD_OK;
 }
 
-int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, DevSample* out, WalkPlan& walk) {
+int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, DevSample* out, ResizePlan& plan) {
   for (int i = 0; i < n; i++) {
     const int rc = plan_one_sample(samples[i], i, b, out[i]);
     if (rc != MLXD_OK) {
       return rc;
     }
   }
-  plan_walk(out, n, b->channels, walk);
+  plan_resize(out, n, b->channels, plan);
   return MLXD_OK;
 }
 
 int plan_samples(
     const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b,
-    std::vector<DevSample>& out, WalkPlan& walk) {
+    std::vector<DevSample>& out, ResizePlan& plan) {
   out.resize(n);
-  const int rc = plan_into(samples, n, b, out.data(), walk);
+  const int rc = plan_into(samples, n, b, out.data(), plan);
   // Test hook (MLXD_TEST_SHORT_PLAN=1, read per launch): room for one step a walk.
   // Every resize CTA that has more finds that before it copies or filters anything,
   // sets the status word and returns, so the kernel's self-check and the way from it
   // to the caller's error code can be exercised without a fault or a hang.
   const char* hook = std::getenv("MLXD_TEST_SHORT_PLAN");
-  if (hook && hook[0] == '1' && walk.steps > 1) {
-    walk.steps = 1;
+  if (rc == MLXD_OK && hook && hook[0] == '1') {
+    plan.strip.steps = std::min(plan.strip.steps, 1);
+    plan.wide.steps = std::min(plan.wide.steps, 1);
   }
   return rc;
 }
@@ -242,7 +248,7 @@ void needed_region(const DevSample& s, int margin, int32_t& r0, int32_t& r1, int
     rhi = (int64_t)s.post_y + s.post_h;
     clo = s.post_x;
     chi = (int64_t)s.post_x + s.post_w;
-  } else if (s.mode == kModeResize || s.mode == kModeResizeDirect) {
+  } else if (s.mode != kModeAffine) {   // the resizes
     axis_span(s.pre_h, s.geom_h, s.post_y, (int64_t)s.post_y + s.post_h, margin, rlo, rhi);
     axis_span(s.pre_w, s.geom_w, s.post_x, (int64_t)s.post_x + s.post_w, margin, clo, chi);
     if (s.pre_flip) {
@@ -396,11 +402,12 @@ int enqueue_on_lane(
   }
   std::vector<DevSample> dev;
   p.status = lane.d_status;
-  rc = plan_samples(samples, n, batch, dev, p.walk);
+  ResizePlan plan;
+  rc = plan_samples(samples, n, batch, dev, plan);
   if (rc != MLXD_OK) {
     return rc;
   }
-  choose_kernels(p, dev.data(), n);
+  choose_kernels(p, plan, dev.data(), n);
   const size_t esize = p.out_f32 ? 4 : 1;
   const size_t slot_bytes = (size_t)batch->slot_h * batch->slot_w * p.c_out * esize;
   const size_t out_bytes = slot_bytes * n;
@@ -430,7 +437,7 @@ int enqueue_on_lane(
 
   // Stage host sources: only the rows the chain reads, each block 256-byte aligned.
   struct Piece {
-    size_t offset, row_bytes, rows, from_pitch;
+    size_t offset, row_bytes, rows, from_pitch, first_row;
     const uint8_t* from;
   };
   std::vector<Piece> pieces;
@@ -499,7 +506,7 @@ int enqueue_on_lane(
       stage_bytes += (pieces[i].row_bytes * pieces[i].rows + 255) & ~(size_t)255;
       dev[i].src_w = c1 - c0;
       dev[i].pre_x -= c0;
-      dev[i].r0_staged = r0;
+      pieces[i].first_row = (size_t)r0;
     }
     rc = arena_reserve(ctx, lane.d_src, stage_bytes + 256, false, lane.stream);
     if (rc != MLXD_OK) {
@@ -508,7 +515,7 @@ int enqueue_on_lane(
     for (int i = 0; i < n; i++) {
       // Base of a virtual image whose rows from r0 on are the staged block.
       dev[i].src = static_cast<const uint8_t*>(lane.d_src.ptr) + pieces[i].offset -
-          pieces[i].row_bytes * (size_t)dev[i].r0_staged;
+          pieces[i].row_bytes * pieces[i].first_row;
     }
   }
   uint8_t* out_base = static_cast<uint8_t*>(batch->dst);
@@ -634,7 +641,7 @@ int enqueue_on_lane(
   if (timed) {
     MLXD_CUDA(cudaEventRecord(lane.k_begin[slot], lane.stream));
   }
-  MLXD_CUDA(launch_fused_batch(p, lane.stream));
+  MLXD_CUDA(launch_fused_batch(p, plan, lane.stream));
   if (timed) {
     MLXD_CUDA(cudaEventRecord(lane.k_end[slot], lane.stream));
     lane.k_pending[slot] = true;

@@ -120,7 +120,7 @@ namespace mlxd {
 // filled by the caller).  Returns MLXD_OK or an error with the message set.
 int plan_samples(
     const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b,
-    std::vector<DevSample>& out, WalkPlan& walk);
+    std::vector<DevSample>& out, ResizePlan& plan);
 
 // One rectangle of a host source that gather.cu packs into device memory:
 // `rows` rows of `row_bytes` bytes, `src_pitch` apart at the source (a pointer
@@ -145,7 +145,7 @@ cudaError_t launch_gather_rows(const GatherPiece* table_dev, int n, uint32_t tot
 // One sample of plan_samples, without its share of the launch.
 int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, DevSample& out);
 // plan_samples into caller-owned storage of n entries.
-int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, DevSample* out, WalkPlan& walk);
+int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, DevSample* out, ResizePlan& plan);
 
 // The cast table of a batch descriptor: table[c * 256 + v], c < c_out.
 void compute_cast_table(const mlxd_batch_desc* b, int c_out, float* table);

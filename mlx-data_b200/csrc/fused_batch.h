@@ -12,7 +12,23 @@ constexpr int kTileH = 16;    // copy and affine bands: output rows per CTA
 constexpr int kTileW = 64;    // and output pixels per tile
 constexpr int kThreads = 256;
 
-// Resize kernel (resize_walk.cu).
+// Resize kernel (resize_strip.cu): a warp walks down a strip of output columns.
+constexpr int kStripThreads = 128;
+constexpr int kStripCtas = 5;         // per SM
+constexpr int kStripRow = 241;        // source bytes of a strip: 16 units of 16 bytes, whichever byte of a unit they start at
+constexpr int kStripMaxRows = 32;     // output rows per warp
+constexpr int kStripSlots = 14;       // source rows of a part, which are in shared memory together
+constexpr int kStripMaxSteps = 320;   // steps of a warp's walk
+constexpr int kStripMaxPx = 256;      // output columns per strip
+// Horizontal weights per strip: 32 * ceil(px / 32) columns of floor(2r) + 2 taps.  A
+// shrink by r has px * r <= kStripRow, so 2 * 241 + 2 * 256 columns and taps bound them
+// twice over; below 32 columns r is at most kStripRow / (kStripMinPx + 1).
+// A strip of fewer columns is left to resize_walk.cu: a shrink along a row alone by 6 (12
+// columns a strip) is 5 % faster in strips, by 12 (5 columns) 7 % and by 15 (4) 45 % slower.
+constexpr int kStripMinPx = 8;
+constexpr int kStripMaxTaps = 32 * (2 * kStripRow / (kStripMinPx + 1) + 4);
+
+// Resize kernel for strong shrinks (resize_walk.cu): a CTA walks down a chunk of columns.
 constexpr int kWalkThreads = 128;
 constexpr int kWalkRow = 832;       // floats per row in shared memory: source bytes of a chunk, alignment included
 constexpr int kWalkMaxRows = 32;    // output rows per CTA
@@ -30,7 +46,8 @@ constexpr int kWalkPadPx = 256;     // columns per strip of padding
 // above 412, 205, 136, 102 along a row for 1 to 4 channels) or one row's 2r + 11
 // steps exceed kWalkMaxSteps (above 506 down the rows).  Every output pixel is then
 // filtered straight from global memory by resize_direct_kernel.
-enum Mode : int32_t { kModeCopy = 0, kModeResize = 1, kModeAffine = 2, kModeResizeDirect = 3 };
+// kModeResizeWide: a resize that is too strong for resize_strip.cu.
+enum Mode : int32_t { kModeCopy = 0, kModeResize = 1, kModeAffine = 2, kModeResizeDirect = 3, kModeResizeWide = 4 };
 
 // One sample's program.  Coordinates name four nested images:
 //   source [src_h, src_w] -> pre window [pre_h, pre_w] (+mirror)
@@ -47,20 +64,46 @@ struct __align__(16) DevSample {
   int32_t mode;
   int32_t pre_flip, post_flip;
   int32_t cap_x;          // resize: bound on the horizontal tap count
-  int32_t walk_px;        // resize kernel: most output columns of a chunk,
-  int32_t walk_chunks;    // chunks that share the post window's columns,
-  int32_t walk_rows;      // output rows per CTA
-  float mx[6];
-  int32_t r0_staged;      // host use: first source row held by the staged copy
+  int32_t walk_px;        // resize kernels: most output columns of a strip (chunk),
+  int32_t walk_chunks;    // strips that share the post window's columns,
+  int32_t walk_rows;      // output rows per warp (CTA)
+  union {
+    float mx[6];          // affine
+    struct {
+      float axis_x[2], axis_y[2];   // resize_strip.cu: Axis::ratio and Axis::fs
+    };
+  };
+  int32_t walk_part;      // resize_strip.cu: output rows whose source rows are in shared memory together, 1, 2 or 4
 };
 
 // What the resize kernel of one launch is sized by: the largest needs of its samples.
+struct StripPlan {
+  int32_t columns;    // columns of the widest strip, a multiple of 32 (0: no sample runs the kernel)
+  int32_t taps;       // horizontal weights of a strip
+  int32_t steps;      // steps of a warp's walk
+  int32_t slots;      // source rows of a part
+  int32_t cells_y;    // grid of cells of every sample, the most rows and the most columns of any of them;
+  int32_t cells_x;    // or 0 rows: cells_x CTAs per sample, which counts its own cells off
+  // with LaunchParams::pad_apart, set at launch: CTAs that walk; the first blocks, which hold
+  // all of these; and the share of those blocks that fill, times 2^32
+  uint32_t walks, mixed_blocks, fill_ratio;
+  int32_t linear;        // blocks are numbered through, not by three coordinates (set at launch)
+};
+
+// The same for the resize kernel of strong shrinks.
 struct WalkPlan {
   int32_t px;         // columns of the widest chunk (0: no sample runs the resize kernel)
   int32_t taps;       // horizontal weights of a chunk
   int32_t steps;      // source rows of a walk
   int32_t cells_y;    // grid of cells of every sample, the most rows and the most columns of any of them;
   int32_t cells_x;    // or 0 rows: cells_x CTAs per sample, which counts its own cells off
+};
+
+// Both, and the samples the second one runs for.
+struct ResizePlan {
+  StripPlan strip;
+  WalkPlan wide;
+  int32_t first_wide, wides;   // all of them are among these samples
 };
 
 // Strips of padding beside the post window.
@@ -84,27 +127,28 @@ struct LaunchParams {
   int32_t band_tiles;         // band kernel: tiles per CTA along a row band (set at launch)
   int32_t bands_x;            // band kernel: CTAs per row band
   int32_t bands;              // some sample is copied or rotated: the band kernel runs
-  WalkPlan walk;
+  WalkPlan walk;              // resize_walk.cu: ResizePlan::wide
   int32_t pad_apart;          // the rows below each post window are filled apart from the cells around them
-  int32_t fill_every;         // resize kernel, then: every so many CTAs, from the first on, one of them fills
+  int32_t fill_every;         // resize kernels, then: every so many CTAs, from the first on, one of them fills
   int32_t direct;             // some sample is kModeResizeDirect: resize_direct_kernel runs last
 };
 
 // Launch the kernels the parameters call for: the resize kernel or, without a
 // resize and when p.pad_apart is set, pad_fill_kernel, the band kernel, resize_direct_kernel.
-cudaError_t launch_fused_batch(const LaunchParams& p, cudaStream_t stream);
-cudaError_t launch_resize_walk(const LaunchParams& p, cudaStream_t stream);
+cudaError_t launch_fused_batch(const LaunchParams& p, const ResizePlan& plan, cudaStream_t stream);
+cudaError_t launch_resize_strip(const LaunchParams& p, const StripPlan& plan, cudaStream_t stream);
+cudaError_t launch_resize_walk(const LaunchParams& p, bool fills_padding, cudaStream_t stream);
 
-// Whether the resize kernel can run a sample (mode kModeResize) at all.
-bool walk_fits(const DevSample& s, int channels);
+// The kernel that runs a resize.
+Mode resize_mode(const DevSample& s, int channels);
 
 // Split the resize samples of a batch into CTAs (DevSample::walk_*) and size
-// the launch.
-void plan_walk(DevSample* samples, int n, int channels, WalkPlan& plan);
+// the launches.
+void plan_resize(DevSample* samples, int n, int channels, ResizePlan& plan);
 
-// Which kernels a launch needs and their grids; call after plan_walk with the
+// Which kernels a launch needs and their grids; call after plan_resize with the
 // host copy of the sample table.
-void choose_kernels(LaunchParams& p, const DevSample* host_samples, int n);
+void choose_kernels(LaunchParams& p, ResizePlan& plan, const DevSample* host_samples, int n);
 
 // Conservative per-axis bounds used by the host planner.
 struct AxisPlan {

@@ -237,8 +237,8 @@ __device__ void run_band(const LaunchParams& p, float* lut_s) {
   if (n >= p.n) {
     return;
   }
-  if (p.samples[n].mode == kModeResize) {
-    return;   // the resize kernel's
+  if (p.samples[n].mode == kModeResize || p.samples[n].mode == kModeResizeWide) {
+    return;   // the resize kernels'
   }
   const DevSample s = p.samples[n];
   const int y0 = ty * kTileH;
@@ -497,19 +497,31 @@ static cudaError_t launch_bands(LaunchParams p, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_fused_batch(const LaunchParams& p, cudaStream_t stream) {
+cudaError_t launch_fused_batch(const LaunchParams& p, const ResizePlan& plan, cudaStream_t stream) {
   if (p.n <= 0) {
     return cudaSuccess;
   }
-  if (p.pad_apart && p.walk.px == 0) {   // the resize kernel fills the padding itself
+  const bool strips = plan.strip.columns > 0, wides = plan.wide.px > 0;
+  if (p.pad_apart && !strips && !wides) {   // a resize kernel fills the padding itself
     pad_fill_kernel<<<(unsigned)p.n * kPadChunks, kThreads, 0, stream>>>(p);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
       return e;
     }
   }
-  if (p.walk.px > 0) {
-    const cudaError_t e = launch_resize_walk(p, stream);
+  if (strips) {
+    const cudaError_t e = launch_resize_strip(p, plan.strip, stream);
+    if (e != cudaSuccess) {
+      return e;
+    }
+  }
+  if (wides) {
+    LaunchParams q = p;
+    if (strips) {
+      q.samples += plan.first_wide;
+      q.n = plan.wides;
+    }
+    const cudaError_t e = launch_resize_walk(q, !strips, stream);
     if (e != cudaSuccess) {
       return e;
     }

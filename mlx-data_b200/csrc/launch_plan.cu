@@ -16,34 +16,16 @@
 
 namespace mlxd {
 
-void choose_kernels(LaunchParams& p, const DevSample* host_samples, int n) {
-  p.bands = 0;
-  p.direct = 0;
-  unsigned long long rows = 0, below = 0;
-  for (int i = 0; i < n; i++) {
-    const DevSample& s = host_samples[i];
-    p.bands |= s.mode != kModeResize;   // a direct sample's padding is the band kernel's too
-    p.direct |= s.mode == kModeResizeDirect;
-    rows += (unsigned long long)s.slot_h;
-    below += (unsigned long long)(s.slot_h > s.post_h ? s.slot_h - s.post_h : 0);
-  }
-  // The rows below a sample's post window are one contiguous run of its slot;
-  // when those runs are at least an eighth of the batch they get a linear fill
-  // of their own (CTAs of the resize kernel, else pad_fill_kernel), which writes
-  // at memory speed.
-  p.pad_apart = n > 0 && below * 8 >= rows ? 1 : 0;
-  p.walk.cells_y = p.walk.cells_x = 0;
-  long long own = 0;
-  for (int i = 0; i < n; i++) {
-    const DevSample& s = host_samples[i];
-    if (s.mode == kModeResize) {
-      const int h = p.pad_apart ? s.post_h : s.slot_h;
-      const int cells_y = (h + s.walk_rows - 1) / s.walk_rows;
-      const int cells_x = s.walk_chunks + walk_strips(s);
-      p.walk.cells_y = std::max(p.walk.cells_y, cells_y);
-      p.walk.cells_x = std::max(p.walk.cells_x, cells_x);
-      own = std::max(own, (long long)cells_y * cells_x);
-    }
+// The grid of one resize kernel: `rows` and `columns` of cells of a sample.
+namespace {
+struct Cells {
+  int32_t y = 0, x = 0;
+  long long own = 0;   // of the largest sample
+
+  void add(int rows, int columns) {
+    y = std::max(y, rows);
+    x = std::max(x, columns);
+    own = std::max(own, (long long)rows * columns);
   }
   // A tall strong shrink beside a wide one would multiply the rows of the one by the
   // columns of the other, for every sample: 1022 images of 32-120 px, one of 22400x60
@@ -51,10 +33,47 @@ void choose_kernels(LaunchParams& p, const DevSample* host_samples, int n) {
   // sample counts its own cells.  That costs each CTA a division by its sample's count
   // (128 images enlarged to 224x224: 58 us a pass instead of 55), so it is left to batches
   // whose common grid has twice the cells of the largest sample.
-  if ((long long)p.walk.cells_y * p.walk.cells_x >= 2 * own && own <= 0x7fffffff) {
-    p.walk.cells_y = 0;
-    p.walk.cells_x = (int32_t)own;
+  void put(int32_t& cells_y, int32_t& cells_x) const {
+    const bool each = (long long)y * x >= 2 * own && own <= 0x7fffffff;
+    cells_y = each ? 0 : y;
+    cells_x = each ? (int32_t)own : x;
   }
+};
+} // namespace
+
+void choose_kernels(LaunchParams& p, ResizePlan& plan, const DevSample* host_samples, int n) {
+  p.bands = 0;
+  p.direct = 0;
+  unsigned long long rows = 0, below = 0;
+  for (int i = 0; i < n; i++) {
+    const DevSample& s = host_samples[i];
+    p.bands |= s.mode != kModeResize && s.mode != kModeResizeWide;   // a direct sample's padding is the band kernel's too
+    p.direct |= s.mode == kModeResizeDirect;
+    rows += (unsigned long long)s.slot_h;
+    below += (unsigned long long)(s.slot_h > s.post_h ? s.slot_h - s.post_h : 0);
+  }
+  // The rows below a sample's post window are one contiguous run of its slot;
+  // when those runs are at least an eighth of the batch they get a linear fill
+  // of their own (CTAs of a resize kernel, else pad_fill_kernel), which writes
+  // at memory speed.
+  p.pad_apart = n > 0 && below * 8 >= rows ? 1 : 0;
+  Cells strip, wide;
+  plan.first_wide = plan.wides = 0;
+  for (int i = 0; i < n; i++) {
+    const DevSample& s = host_samples[i];
+    const int h = p.pad_apart ? s.post_h : s.slot_h;
+    if (s.mode == kModeResize) {
+      const int cell_rows = s.walk_rows * (kStripThreads / 32);
+      strip.add((h + cell_rows - 1) / cell_rows, s.walk_chunks + walk_strips(s));
+    } else if (s.mode == kModeResizeWide) {
+      wide.add((h + s.walk_rows - 1) / s.walk_rows, s.walk_chunks + walk_strips(s));
+      plan.first_wide = plan.wides == 0 ? i : plan.first_wide;
+      plan.wides = i + 1 - plan.first_wide;
+    }
+  }
+  strip.put(plan.strip.cells_y, plan.strip.cells_x);
+  wide.put(plan.wide.cells_y, plan.wide.cells_x);
+  p.walk = plan.wide;
 }
 
 AxisPlan plan_axis(int32_t n_src, int32_t n_dst, int32_t sub) {
@@ -88,9 +107,75 @@ static long long walk_steps(const DevSample& s, int rows) {
   return s.pre_h <= s.geom_h ? 4LL * rows + 4 : extent + rows + 8;
 }
 
-bool walk_fits(const DevSample& s, int channels) {
-  return walk_row_bytes(s, channels, 1) <= kWalkRow && walk_steps(s, 1) <= kWalkMaxSteps &&
-      (long long)s.src_w * channels < (1LL << 31);
+// Source bytes of `px` output columns of a strip.  The last of them is centred
+// (px - 1) ratios behind the first, and both reach one radius further; two more
+// columns cover the ends' fractions and the float32 rounding of the kernel.
+static long long strip_bytes(const DevSample& s, int channels, int px) {
+  const double ratio = (double)s.pre_w / (double)s.geom_w;
+  const long long cols = (long long)std::ceil((px - 1) * ratio + 2.0 * std::max(1.0, ratio)) + 2;
+  return std::min<long long>(cols, s.pre_w) * channels;
+}
+
+// The widest strip that fits; 0 when not even one column does.
+static int strip_most_px(const DevSample& s, int channels) {
+  const int most = std::min(s.post_w, kStripMaxPx);
+  if ((long long)s.pre_w * channels <= kStripRow) {
+    return most;
+  }
+  const double ratio = (double)s.pre_w / (double)s.geom_w;
+  const int guess = (int)((kStripRow / channels - 2 - 2.0 * std::max(1.0, ratio)) / ratio) + 1;
+  int px = std::max(0, std::min(most, guess));
+  while (px > 0 && strip_bytes(s, channels, px) > kStripRow) {
+    px--;
+  }
+  return px;
+}
+
+// Bound on the source rows that `rows` output rows read.
+static int strip_span(const DevSample& s, int rows) {
+  const double ratio = (double)s.pre_h / (double)s.geom_h;
+  return (int)std::min(1e6, (rows - 1) * ratio + 2.0 * std::max(1.0, ratio)) + 2;
+}
+
+Mode resize_mode(const DevSample& s, int channels) {
+  if ((long long)s.src_w * channels >= (1LL << 31)) {
+    return kModeResizeDirect;
+  }
+  const int px = strip_most_px(s, channels);
+  if (px >= std::min(s.post_w, kStripMinPx) && s.cap_x * 32 * ((px + 31) / 32) <= kStripMaxTaps &&
+      strip_span(s, 1) <= kStripSlots) {
+    return kModeResize;
+  }
+  return walk_row_bytes(s, channels, 1) <= kWalkRow && walk_steps(s, 1) <= kWalkMaxSteps ? kModeResizeWide
+                                                                                          : kModeResizeDirect;
+}
+
+// Instructions of a warp per stage of four output rows of a strip `px` columns wide,
+// as measured by taking parts of the kernel away: the steps down the source rows,
+// then passes of 32 columns.
+static double stage_cost(const DevSample& s, int px) {
+  const double rx = (double)s.pre_w / (double)s.geom_w, ry = (double)s.pre_h / (double)s.geom_h;
+  const double vertical = 4.0 * std::max(ry, 1.5) * 30.0 + 150.0;
+  const double pass = (2.0 * std::max(rx, 1.0) + 1.0) * 17.0 + 90.0;
+  return vertical + (px + 31) / 32 * pass;
+}
+
+// How many strips: the fewer, the fewer walks down the source rows; the horizontal
+// half works on 32 columns at a time, so strips of whole 32s waste no lanes.
+static void split_strips(DevSample& s, int channels) {
+  const int most = strip_most_px(s, channels);
+  double best = 0.0;
+  int chosen = 0;
+  for (int passes = (most + 31) / 32; passes > 0; passes--) {
+    const int strips = (s.post_w + std::min(most, 32 * passes) - 1) / std::min(most, 32 * passes);
+    const double cost = strips * stage_cost(s, (s.post_w + strips - 1) / strips);
+    if (chosen == 0 || cost < best) {
+      best = cost;
+      chosen = strips;
+    }
+  }
+  s.walk_px = (s.post_w + chosen - 1) / chosen;
+  s.walk_chunks = (s.post_w + s.walk_px - 1) / s.walk_px;
 }
 
 // Chunks of at most `px` columns and walks of at most `rows` rows, smaller
@@ -113,16 +198,54 @@ static void split_walk(DevSample& s, int channels, int px, int rows) {
   s.walk_rows = rows;
 }
 
-void plan_walk(DevSample* samples, int n, int channels, WalkPlan& plan) {
+static void plan_strips(DevSample* samples, int n, int channels, StripPlan& plan) {
+  constexpr int kWarps = kStripThreads / 32;
+  constexpr double kWarpsAtOnce = 148 * kStripCtas * kWarps;
+  plan = StripPlan{};
+  double total = 0.0;
+  for (int i = 0; i < n; i++) {
+    DevSample& s = samples[i];
+    if (s.mode == kModeResize) {
+      split_strips(s, channels);
+      s.walk_part = strip_span(s, 4) <= kStripSlots ? 4 : strip_span(s, 2) <= kStripSlots ? 2 : 1;
+      const int columns = (s.walk_px + 31) / 32 * 32;
+      plan.columns = std::max(plan.columns, columns);
+      plan.taps = std::max(plan.taps, columns * s.cap_x);
+      plan.slots = std::max(plan.slots, strip_span(s, s.walk_part));
+      total += (double)s.walk_chunks * ((s.post_h + 3) / 4) * stage_cost(s, s.walk_px);
+    }
+  }
+  if (total == 0.0) {
+    return;
+  }
+  // Walks of about the same work in all samples, so that a large or strongly shrunk one
+  // does not hold up the end: one and a half rounds of them over the device's warps, but
+  // not below kLeast, about three times what a walk's tables take, as long as all warps
+  // have one.  96 images of 240-640 px to 224x224: 51 us a pass so, 56 in one round, 66
+  // where every walk has 8 rows; 256 of 256-800 px: 121, 125 in two and a half rounds,
+  // 149 in eight.
+  constexpr double kRounds = 1.5, kLeast = 2500.0;
+  const double walk = std::max(total / kWarpsAtOnce / kRounds, std::min(total / kWarpsAtOnce, kLeast));
+  for (int i = 0; i < n; i++) {
+    DevSample& s = samples[i];
+    if (s.mode != kModeResize) {
+      continue;
+    }
+    const int stages = (int)std::min(8.0, std::max(1.0, walk / stage_cost(s, s.walk_px)));
+    // as few CTAs as that makes, with the rows dealt evenly, in fours
+    const int down = (s.post_h + 4 * stages * kWarps - 1) / (4 * stages * kWarps);
+    int rows = ((s.post_h + down * kWarps - 1) / (down * kWarps) + 3) / 4 * 4;
+    while (rows > 4 && walk_steps(s, rows) > kStripMaxSteps) {
+      rows -= 4;
+    }
+    s.walk_rows = rows;
+    plan.steps = std::max(plan.steps, (int32_t)walk_steps(s, rows));
+  }
+}
+
+static void plan_wide(DevSample* samples, int n, int channels, WalkPlan& plan) {
   // The largest cells that still give every one of a B200's 148 SMs two CTAs (another
-  // count would only choose other cells).  A CTA
-  // builds its tables and walks 2 r source rows (shrink ratio r) before its first
-  // output row is complete, so smaller cells cost more as soon as the SMs have
-  // work: 512 frames of 1080x1920 to 512x512 take 1.37 ms in 128x32 cells, 1.46
-  // in 128x16, 1.58 in 64x32, 3.4 in 64x4; 32 images of 200-500 px to 224x224
-  // 32 us in 448 CTAs of 128x32 and in 1792 of 128x8, 52 us in 64x4.  One 480x640
-  // image to 224x224 fills no wave of any size and is quickest in the smallest
-  // cells: 14.4 us a call in 64x4, 18 in 128x8.
+  // count would only choose other cells).
   static const int kCells[][2] = {{kWalkMaxPx, 32}, {kWalkMaxPx, 16}, {kWalkMaxPx, 8}, {64, 8}, {64, 4}};
   constexpr long long kWantCtas = 148 * 2;
   for (const auto& cell : kCells) {
@@ -130,7 +253,7 @@ void plan_walk(DevSample* samples, int n, int channels, WalkPlan& plan) {
     plan = WalkPlan{0, 0, 0, 0, 0};
     for (int i = 0; i < n; i++) {
       DevSample& s = samples[i];
-      if (s.mode == kModeResize) {
+      if (s.mode == kModeResizeWide) {
         split_walk(s, channels, cell[0], cell[1]);
         ctas += (long long)s.walk_chunks * ((s.post_h + s.walk_rows - 1) / s.walk_rows);
         plan.px = std::max(plan.px, s.walk_px);
@@ -142,6 +265,11 @@ void plan_walk(DevSample* samples, int n, int channels, WalkPlan& plan) {
       return;
     }
   }
+}
+
+void plan_resize(DevSample* samples, int n, int channels, ResizePlan& plan) {
+  plan_strips(samples, n, channels, plan.strip);
+  plan_wide(samples, n, channels, plan.wide);
 }
 
 } // namespace mlxd

@@ -124,14 +124,15 @@ extern "C" int mlxd_fused_batch_noalloc(
 
   const size_t esize = p.out_f32 ? 4 : 1;
   const size_t slot_bytes = (size_t)batch->slot_h * batch->slot_w * p.c_out * esize;
-  rc = plan_into(samples, n, batch, table, p.walk);
+  ResizePlan plan;
+  rc = plan_into(samples, n, batch, table, plan);
   if (rc != MLXD_OK) {
     return rc;
   }
   for (int i = 0; i < n; i++) {
     table[i].dst = static_cast<uint8_t*>(batch->dst) + slot_bytes * i;
   }
-  choose_kernels(p, table, n);
+  choose_kernels(p, plan, table, n);
 
   // The scratch keeps whatever the previous call left.  Its status word is
   // read back first (the kernel of the previous call is ahead of this copy on
@@ -157,7 +158,7 @@ extern "C" int mlxd_fused_batch_noalloc(
              (int)previous_status);
     return fail(MLXD_ERR_DEVICE, msg);
   }
-  MLXD_CUDA(launch_fused_batch(p, stream));
+  MLXD_CUDA(launch_fused_batch(p, plan, stream));
   return MLXD_OK;
 }
 

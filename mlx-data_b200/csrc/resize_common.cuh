@@ -1,0 +1,95 @@
+// What the two resize kernels share: packed float arithmetic, quantisation and
+// the way of four finished rows into the batch tensor.
+#pragma once
+
+#include "fused_batch.h"
+#include "kernel_common.cuh"
+
+namespace mlxd {
+
+// d = a * b + c on both lanes.
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// (int)(acc + 0.5) of both lanes as the low mantissa bits of 2^23 + that
+// integer.  acc is never negative and at most 255 (1 + 1e-4) here - pixels
+// times weights that sum to 1 within the rounding of a few hundred terms - so
+// acc + 0.5 < 256 and the clamp to [0, 255] of the definition never acts.
+__device__ __forceinline__ void quantise2(f32x2 acc, unsigned& q0, unsigned& q1) {
+  const f32x2 half = pack2(0.5f, 0.5f), two23 = pack2(8388608.0f, 8388608.0f);
+  f32x2 t;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(acc), "l"(half));
+  asm("add.rz.f32x2 %0, %1, %2;" : "=l"(t) : "l"(t), "l"(two23));
+  float a, b;
+  unpack2(t, a, b);
+  q0 = __float_as_uint(a);
+  q1 = __float_as_uint(b);
+}
+
+constexpr unsigned kTwo23Bits = 0x4B000000u;
+
+__device__ __forceinline__ void sts_v4(unsigned a, float x, float y, float z, float w) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+
+template <int OFF>
+__device__ __forceinline__ void lds_v4u32(unsigned a, uint32_t& x, uint32_t& y, uint32_t& z, uint32_t& w) {
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4+%5];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(a), "n"(OFF));
+}
+
+// One output column of four rows: filter sums acc[2 * c + h] (rows 2h and 2h + 1
+// of channel c) quantised, reduced to grey, cast and stored.  `at` is the first
+// row's place in the batch tensor in elements; the first `rows` rows are stored.
+template <int C, bool GRAY, bool U8>
+__device__ __forceinline__ void store_column(
+    const LaunchParams& p, unsigned lut, const f32x2 (&acc)[2 * C], int rows, void* dst, size_t at, size_t row_stride,
+    bool vec_ok) {
+  constexpr int CO = GRAY ? 1 : C;
+  unsigned q[4][C];   // 2^23 bits + value
+#pragma unroll
+  for (int ch = 0; ch < C; ch++) {
+    quantise2(acc[2 * ch], q[0][ch], q[1][ch]);
+    quantise2(acc[2 * ch + 1], q[2][ch], q[3][ch]);
+  }
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+    if (r < rows) {   // (rows beyond the last hold anything: they must not index the cast table)
+      if (U8) {
+        uint8_t* d = reinterpret_cast<uint8_t*>(dst) + at + r * row_stride;
+        if (GRAY) {
+          d[0] = (uint8_t)gray_mix(p, q[r][0] & 0xffu, q[r][1 % C] & 0xffu, q[r][2 % C] & 0xffu);
+        } else {
+#pragma unroll
+          for (int ch = 0; ch < C; ch++) {
+            d[ch] = (uint8_t)q[r][ch];
+          }
+        }
+      } else {
+        float v[CO];
+        if (GRAY) {
+          v[0] = __uint_as_float(
+              lds_u32<0>(lut + 4u * gray_mix(p, q[r][0] & 0xffu, q[r][1 % C] & 0xffu, q[r][2 % C] & 0xffu)));
+        } else {
+#pragma unroll
+          for (int ch = 0; ch < C; ch++) {
+            v[ch % CO] = __uint_as_float(lds_u32<0>((lut + 1024u * ch - 4u * kTwo23Bits) + 4u * q[r][ch]));
+          }
+        }
+        float* d = reinterpret_cast<float*>(dst) + at + r * row_stride;
+        if (CO == 4 && vec_ok) {
+          *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1 % CO], v[2 % CO], v[3 % CO]);
+        } else {
+#pragma unroll
+          for (int ch = 0; ch < CO; ch++) {
+            d[ch] = v[ch];
+          }
+        }
+      }
+    }
+  }
+}
+
+} // namespace mlxd

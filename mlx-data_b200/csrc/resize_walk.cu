@@ -1,4 +1,4 @@
-// The resize kernel: one CTA of kWalkThreads walks down one chunk of output
+// The resize kernel of strong shrinks (kModeResizeWide): one CTA of kWalkThreads walks down one chunk of output
 // columns (walk_px of them at most) of one sample, walk_rows output rows, in
 // stages of four rows.
 //
@@ -41,6 +41,7 @@
 
 #include "fused_batch.h"
 #include "kernel_common.cuh"
+#include "resize_common.cuh"
 
 namespace mlxd {
 namespace {
@@ -84,39 +85,6 @@ __host__ __device__ constexpr size_t walk_layout(int c_out, const WalkPlan& w, u
     *out = sm;
   }
   return (off + 15) & ~(size_t)15;
-}
-
-// d = a * b + c on both lanes.
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
-// (int)(acc + 0.5) of both lanes as the low mantissa bits of 2^23 + that
-// integer.  acc is never negative and at most 255 (1 + 1e-4) here - pixels
-// times weights that sum to 1 within the rounding of a few hundred terms - so
-// acc + 0.5 < 256 and the clamp to [0, 255] of the definition never acts.
-__device__ __forceinline__ void quantise2(f32x2 acc, unsigned& q0, unsigned& q1) {
-  const f32x2 half = pack2(0.5f, 0.5f), two23 = pack2(8388608.0f, 8388608.0f);
-  f32x2 t;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(acc), "l"(half));
-  asm("add.rz.f32x2 %0, %1, %2;" : "=l"(t) : "l"(t), "l"(two23));
-  float a, b;
-  unpack2(t, a, b);
-  q0 = __float_as_uint(a);
-  q1 = __float_as_uint(b);
-}
-
-constexpr unsigned kTwo23Bits = 0x4B000000u;
-
-__device__ __forceinline__ void sts_v4(unsigned a, float x, float y, float z, float w) {
-  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
-}
-
-template <int OFF>
-__device__ __forceinline__ void lds_v4u32(unsigned a, uint32_t& x, uint32_t& y, uint32_t& z, uint32_t& w) {
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4+%5];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(a), "n"(OFF));
 }
 
 // One thread's filter state.
@@ -313,11 +281,10 @@ __device__ __forceinline__ void walk_stages(const DevSample& s, const LaunchPara
       fetch<SHIFT>(k, lds_u32<16>(e), (int)lds_u32<20>(e), (unsigned)j * kSlotBytes);
     }
   }
-  float* const out = reinterpret_cast<float*>(s.dst);
-  uint8_t* const out8 = reinterpret_cast<uint8_t*>(s.dst);
   const size_t row_stride = (size_t)s.slot_w * CO;
   const bool post_flip = s.post_flip != 0;
-  const bool vec_ok = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  void* const dst = s.dst;   // (a copy: the stores could otherwise have changed it)
+  const bool vec_ok = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
   const unsigned hstep = (unsigned)s.walk_px * 4u;
   const int tap_step = c.pre_flip ? -8 * C : 8 * C;
   const unsigned mid = c.sm.mid;
@@ -352,50 +319,9 @@ __device__ __forceinline__ void walk_stages(const DevSample& s, const LaunchPara
           wq += hstep;
         }
       }
-      unsigned q[4][C];   // 2^23 bits + value
-#pragma unroll
-      for (int ch = 0; ch < C; ch++) {
-        quantise2(acc[2 * ch], q[0][ch], q[1][ch]);
-        quantise2(acc[2 * ch + 1], q[2][ch], q[3][ch]);
-      }
       const int ox = post_flip ? c.x1 - 1 - x : c.x0 + x;
-      const size_t at = (size_t)(c.y0 + r0) * row_stride + (size_t)ox * CO;
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        if (r < rows) {   // (rows beyond the last hold anything: they must not index the cast table)
-          if (U8) {
-            uint8_t* d = out8 + at + r * row_stride;
-            if (GRAY) {
-              d[0] = (uint8_t)gray_mix(p, q[r][0] & 0xffu, q[r][1 % C] & 0xffu, q[r][2 % C] & 0xffu);
-            } else {
-#pragma unroll
-              for (int ch = 0; ch < C; ch++) {
-                d[ch] = (uint8_t)q[r][ch];
-              }
-            }
-          } else {
-            float v[CO];
-            if (GRAY) {
-              v[0] = __uint_as_float(lds_u32<0>(
-                  c.sm.lut + 4u * gray_mix(p, q[r][0] & 0xffu, q[r][1 % C] & 0xffu, q[r][2 % C] & 0xffu)));
-            } else {
-#pragma unroll
-              for (int ch = 0; ch < C; ch++) {
-                v[ch % CO] = __uint_as_float(lds_u32<0>((c.sm.lut + 1024u * ch - 4u * kTwo23Bits) + 4u * q[r][ch]));
-              }
-            }
-            float* d = out + at + r * row_stride;
-            if (CO == 4 && vec_ok) {
-              *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1 % CO], v[2 % CO], v[3 % CO]);
-            } else {
-#pragma unroll
-              for (int ch = 0; ch < CO; ch++) {
-                d[ch] = v[ch];
-              }
-            }
-          }
-        }
-      }
+      store_column<C, GRAY, U8>(
+          p, c.sm.lut, acc, rows, dst, (size_t)(c.y0 + r0) * row_stride + (size_t)ox * CO, row_stride, vec_ok);
     }
     __syncthreads();
   }
@@ -575,7 +501,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int CO = GRAY ? 1 : C;
   unsigned t = blockIdx.x;
-  if (p.pad_apart) {
+  if (p.pad_apart && p.fill_every > 0) {   // (0: the other resize kernel fills)
     const unsigned fills = (unsigned)p.n * kPadChunks, every = (unsigned)p.fill_every;
     if (t % every == 0 && t / every < fills) {
       pad_below_any<kWalkThreads>(p, t / every);
@@ -588,7 +514,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
   int cx = (int)cell;
   int cy = OWN ? 0 : (int)(t % p.walk.cells_y);
   const DevSample& s = p.samples[OWN ? t : t / p.walk.cells_y];
-  if (s.mode != kModeResize) {
+  if (s.mode != kModeResizeWide) {
     return;   // the other kernels'
   }
   const int slot_h = s.slot_h, slot_w = s.slot_w, post_h = s.post_h, post_w = s.post_w;
@@ -660,13 +586,14 @@ cudaError_t launch(const LaunchParams& p, unsigned blocks, size_t smem, cudaStre
 
 } // namespace
 
-cudaError_t launch_resize_walk(const LaunchParams& p_in, cudaStream_t stream) {
+cudaError_t launch_resize_walk(const LaunchParams& p_in, bool fills_padding, cudaStream_t stream) {
   LaunchParams p = p_in;
+  p.fill_every = 0;
   unsigned long long blocks = (unsigned long long)p.n * std::max(p.walk.cells_y, 1) * p.walk.cells_x;
   if (blocks == 0) {
     return cudaSuccess;
   }
-  if (p.pad_apart) {
+  if (p.pad_apart && fills_padding) {
     // Filling is bound by memory writes, walking by the SMs: the fill CTAs go
     // among the others, evenly, instead of into a launch of their own.  64 images
     // of 160-1024 px padded to the largest (2 GB written): 384 us a pass (in a
