@@ -174,12 +174,12 @@ int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, 
         s.mode = kModeCopy;  // identity on both axes
       } else {
         s.cap_x = plan_axis(s.pre_w, s.geom_w, 1).cap;
-        s.mode = resize_mode(s, b->channels);
         // the divisions of make_axis(), correctly rounded here as there
         s.axis_x[0] = (float)s.pre_w / (float)s.geom_w;
         s.axis_x[1] = std::min(1.0f, (float)s.geom_w / (float)s.pre_w);
         s.axis_y[0] = (float)s.pre_h / (float)s.geom_h;
         s.axis_y[1] = std::min(1.0f, (float)s.geom_h / (float)s.pre_h);
+        s.mode = resize_mode(s, b->channels);
       }
     } else if (d.geom == MLXD_GEOM_AFFINE) {
       s.mode = kModeAffine;

@@ -24,8 +24,8 @@ constexpr int kStripMaxPx = 256;      // output columns per strip
 // shrink by r has px * r <= kStripRow, so 2 * 241 + 2 * 256 columns and taps bound them
 // twice over; below 32 columns r is at most kStripRow / (kStripMinPx + 1).
 // A strip of fewer columns is left to resize_walk.cu: a shrink along a row alone by 6 (12
-// columns a strip) is 5 % faster in strips, by 12 (5 columns) 7 % and by 15 (4) 45 % slower.
-constexpr int kStripMinPx = 8;
+// columns a strip) is 6 % faster in strips, by 7 (10 columns) 25 % slower, by 15 (4) 45 %.
+constexpr int kStripMinPx = 11;
 constexpr int kStripMaxTaps = 32 * (2 * kStripRow / (kStripMinPx + 1) + 4);
 
 // Resize kernel for strong shrinks (resize_walk.cu): a CTA walks down a chunk of columns.
@@ -139,8 +139,8 @@ cudaError_t launch_fused_batch(const LaunchParams& p, const ResizePlan& plan, cu
 cudaError_t launch_resize_strip(const LaunchParams& p, const StripPlan& plan, cudaStream_t stream);
 cudaError_t launch_resize_walk(const LaunchParams& p, bool fills_padding, cudaStream_t stream);
 
-// The kernel that runs a resize.
-Mode resize_mode(const DevSample& s, int channels);
+// The kernel that runs a resize, axis_x and axis_y in place.
+Mode resize_mode(DevSample& s, int channels);
 
 // Split the resize samples of a batch into CTAs (DevSample::walk_*) and size
 // the launches.

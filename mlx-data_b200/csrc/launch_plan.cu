@@ -111,7 +111,7 @@ static long long walk_steps(const DevSample& s, int rows) {
 // (px - 1) ratios behind the first, and both reach one radius further; two more
 // columns cover the ends' fractions and the float32 rounding of the kernel.
 static long long strip_bytes(const DevSample& s, int channels, int px) {
-  const double ratio = (double)s.pre_w / (double)s.geom_w;
+  const double ratio = s.axis_x[0];
   const long long cols = (long long)std::ceil((px - 1) * ratio + 2.0 * std::max(1.0, ratio)) + 2;
   return std::min<long long>(cols, s.pre_w) * channels;
 }
@@ -122,7 +122,7 @@ static int strip_most_px(const DevSample& s, int channels) {
   if ((long long)s.pre_w * channels <= kStripRow) {
     return most;
   }
-  const double ratio = (double)s.pre_w / (double)s.geom_w;
+  const double ratio = s.axis_x[0];
   const int guess = (int)((kStripRow / channels - 2 - 2.0 * std::max(1.0, ratio)) / ratio) + 1;
   int px = std::max(0, std::min(most, guess));
   while (px > 0 && strip_bytes(s, channels, px) > kStripRow) {
@@ -133,15 +133,16 @@ static int strip_most_px(const DevSample& s, int channels) {
 
 // Bound on the source rows that `rows` output rows read.
 static int strip_span(const DevSample& s, int rows) {
-  const double ratio = (double)s.pre_h / (double)s.geom_h;
+  const double ratio = s.axis_y[0];
   return (int)std::min(1e6, (rows - 1) * ratio + 2.0 * std::max(1.0, ratio)) + 2;
 }
 
-Mode resize_mode(const DevSample& s, int channels) {
+Mode resize_mode(DevSample& s, int channels) {
   if ((long long)s.src_w * channels >= (1LL << 31)) {
     return kModeResizeDirect;
   }
   const int px = strip_most_px(s, channels);
+  s.walk_px = px;   // for split_strips
   if (px >= std::min(s.post_w, kStripMinPx) && s.cap_x * 32 * ((px + 31) / 32) <= kStripMaxTaps &&
       strip_span(s, 1) <= kStripSlots) {
     return kModeResize;
@@ -154,7 +155,7 @@ Mode resize_mode(const DevSample& s, int channels) {
 // as measured by taking parts of the kernel away: the steps down the source rows,
 // then passes of 32 columns.
 static double stage_cost(const DevSample& s, int px) {
-  const double rx = (double)s.pre_w / (double)s.geom_w, ry = (double)s.pre_h / (double)s.geom_h;
+  const double rx = s.axis_x[0], ry = s.axis_y[0];
   const double vertical = 4.0 * std::max(ry, 1.5) * 30.0 + 150.0;
   const double pass = (2.0 * std::max(rx, 1.0) + 1.0) * 17.0 + 90.0;
   return vertical + (px + 31) / 32 * pass;
@@ -162,8 +163,8 @@ static double stage_cost(const DevSample& s, int px) {
 
 // How many strips: the fewer, the fewer walks down the source rows; the horizontal
 // half works on 32 columns at a time, so strips of whole 32s waste no lanes.
-static void split_strips(DevSample& s, int channels) {
-  const int most = strip_most_px(s, channels);
+static void split_strips(DevSample& s) {
+  const int most = s.walk_px;
   double best = 0.0;
   int chosen = 0;
   for (int passes = (most + 31) / 32; passes > 0; passes--) {
@@ -198,7 +199,7 @@ static void split_walk(DevSample& s, int channels, int px, int rows) {
   s.walk_rows = rows;
 }
 
-static void plan_strips(DevSample* samples, int n, int channels, StripPlan& plan) {
+static void plan_strips(DevSample* samples, int n, StripPlan& plan) {
   constexpr int kWarps = kStripThreads / 32;
   constexpr double kWarpsAtOnce = 148 * kStripCtas * kWarps;
   plan = StripPlan{};
@@ -206,7 +207,7 @@ static void plan_strips(DevSample* samples, int n, int channels, StripPlan& plan
   for (int i = 0; i < n; i++) {
     DevSample& s = samples[i];
     if (s.mode == kModeResize) {
-      split_strips(s, channels);
+      split_strips(s);
       s.walk_part = strip_span(s, 4) <= kStripSlots ? 4 : strip_span(s, 2) <= kStripSlots ? 2 : 1;
       const int columns = (s.walk_px + 31) / 32 * 32;
       plan.columns = std::max(plan.columns, columns);
@@ -268,7 +269,24 @@ static void plan_wide(DevSample* samples, int n, int channels, WalkPlan& plan) {
 }
 
 void plan_resize(DevSample* samples, int n, int channels, ResizePlan& plan) {
-  plan_strips(samples, n, channels, plan.strip);
+  // With four channels all units of a pixel column lie in one half of the banks, so that
+  // the columns of a shrink of two or three meet in one or two of eight places: 96 images
+  // to 224x224 take 133 us a pass in strips at 2:1 and 110 in resize_walk.cu, 178 and 148
+  // at 3:1 (78 and 83 at 1.6:1, and at 4:1, where that kernel's columns meet too, 27 and
+  // 35).  Decided for the batch: 128 images of 256-800 px, both kinds, take 160 us when
+  // either kernel gets its own, 150 in strips, 137 in resize_walk.cu.
+  int resizes = 0, meet = 0;
+  for (int i = 0; channels == 4 && i < n; i++) {
+    resizes += samples[i].mode == kModeResize;
+    meet += samples[i].mode == kModeResize && samples[i].axis_x[0] > 1.75f && samples[i].axis_x[0] < 3.5f;
+  }
+  for (int i = 0; 4 * meet > resizes && i < n; i++) {
+    DevSample& s = samples[i];
+    if (s.mode == kModeResize && walk_row_bytes(s, channels, 1) <= kWalkRow && walk_steps(s, 1) <= kWalkMaxSteps) {
+      s.mode = kModeResizeWide;
+    }
+  }
+  plan_strips(samples, n, plan.strip);
   plan_wide(samples, n, channels, plan.wide);
 }
 

@@ -31,11 +31,13 @@ def test_rows_of_a_part(pkg, ctx, oracle, h, c):
     _check(pkg, ctx, oracle, [(h, 64), (h, 65), (h, 66), (h, 67), (20, 71)], c, ops, seed=h + c)
 
 
-# along a row: around eight columns of a strip (2r + 7r + 2 source columns in 241 bytes)
-@pytest.mark.parametrize("c,ratio", [(1, 26), (1, 27.5), (2, 13), (2, 13.5), (3, 8.5), (3, 9), (4, 6.2), (4, 6.7)])
+# along a row: around eleven columns of a strip (2r + 10r + 2 source columns in 241 bytes), and the
+# shrinks in between that four channels leave to the other kernel
+@pytest.mark.parametrize("c,ratio", [(1, 19.5), (1, 20.5), (2, 9.4), (2, 9.9), (3, 6.3), (3, 6.7), (4, 4.6), (4, 5),
+                                     (4, 1.7), (4, 1.8), (4, 3.4), (4, 3.6)])
 def test_columns_of_a_strip(pkg, ctx, oracle, c, ratio):
-    w = int(9 * ratio)
-    ops = [("image_resize", dict(key="image", w=9, h=11)), ("image_random_h_flip", dict(key="image", prob=0.5))]
+    w = int(12 * ratio)
+    ops = [("image_resize", dict(key="image", w=12, h=11)), ("image_random_h_flip", dict(key="image", prob=0.5))]
     _check(pkg, ctx, oracle, [(13, w + k) for k in range(-9, 10, 3)] + [(12, 60)], c, ops, seed=c)
 
 
