@@ -28,9 +28,9 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 NOMINAL_HBM_GBS = 8000.0
 # DRAM bytes per image of the workload: dram__bytes_read.sum of an ncu capture of one
-# resize_walk_kernel launch on 64 images (239.7 MB), plus the batch it writes, all of
+# resize_strip_kernel launch on 64 images (239.4 MB), plus the batch it writes, all of
 # which leaves L2 in a launch larger than that; both grow with the image count.
-NCU_DRAM_BYTES_PER_IMAGE = {"c5": 239.7e6 / 64 + 512 * 512 * 3 * 4}
+NCU_DRAM_BYTES_PER_IMAGE = {"c5": 239.4e6 / 64 + 512 * 512 * 3 * 4}
 
 
 def load_package():

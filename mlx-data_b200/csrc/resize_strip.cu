@@ -25,19 +25,19 @@
 // out times 2^-22 and the horizontal weights are kept times 2^22 - powers of two
 // throughout, so every rounding falls as without them.
 //
-// What bounds it (1080x1920x3 to 512x512, 512 images: 1.18 ms; 1.37 in resize_walk.cu,
-// which runs a whole CTA down 832 bytes): latency of shared memory and of the stages'
-// copies at 20 warps an SM, instruction issue a little over 55 %, the shared-memory
-// pipe two thirds busy (resize_walk.cu: 89 %).  Per 32 columns x 4 rows a warp executes
-// 790 instructions (830): 310 on the steps, 260 on taps and stores, 110 on copies and
-// the skeleton of a stage, the rest on tables.  Why this split: two 4-byte cp.async a
-// row cost the pipe nine wavefronts, one 16-byte cp.async for two rows about two a row;
-// a unit of four rows halves the loads of the taps, and dealing columns to lanes by
-// bank takes most of their conflicts; a CTA-wide walk meets two barriers a stage and
-// leaves warps idle where a chunk's words are no multiple of its 128 lanes.  Five CTAs
-// per SM at 96 registers: six spill (1.55 ms), four wait (1.36).  The tables of a CTA
-// took a fifth of the time before the taps of a pass were shared by its warps, the steps
-// dealt flat over the lanes and the axes' ratios divided on the host (1.25 ms).
+// What bounds it (1080x1920x3 to 512x512, 512 images: 1.17 ms; 1.37 in resize_walk.cu,
+// which runs a whole CTA down 832 bytes): the shared-memory pipe, 76 % busy (89 there),
+// and its latency at 20 warps an SM; instructions issue in 58 % of the cycles.  Per 32
+// columns x 4 rows a warp executes 780 instructions (830), about 310 of them on the
+// steps, 260 on taps and stores, 110 on copies and the skeleton of a stage.  Why this
+// split: two 4-byte cp.async a row cost the pipe nine wavefronts, one 16-byte cp.async
+// for two rows about two a row; a unit of four rows halves the loads of the taps, and
+// dealing columns to lanes by bank takes most of their conflicts; a CTA-wide walk meets
+// two barriers a stage and leaves warps idle where a chunk's words are no multiple of its
+// 128 lanes.  Five CTAs per SM at 96 registers: six spill (1.55 ms), four wait (1.36).
+// The tables of a CTA took a fifth of the time before the taps of a pass were shared by
+// its warps, the steps dealt flat over the lanes and the axes' ratios divided on the
+// host (1.25 ms).
 #include <algorithm>
 
 #include "fused_batch.h"
