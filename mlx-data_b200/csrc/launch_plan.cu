@@ -226,21 +226,37 @@ static void plan_strips(DevSample* samples, int n, StripPlan& plan) {
   // where every walk has 8 rows; 256 of 256-800 px: 121, 125 in two and a half rounds,
   // 149 in eight.
   constexpr double kRounds = 1.5, kLeast = 2500.0;
-  const double walk = std::max(total / kWarpsAtOnce / kRounds, std::min(total / kWarpsAtOnce, kLeast));
-  for (int i = 0; i < n; i++) {
-    DevSample& s = samples[i];
-    if (s.mode != kModeResize) {
-      continue;
+  double walk = std::max(total / kWarpsAtOnce / kRounds, std::min(total / kWarpsAtOnce, kLeast));
+  for (;;) {
+    long long ctas = 0;
+    bool longest = true;
+    plan.steps = 0;
+    for (int i = 0; i < n; i++) {
+      DevSample& s = samples[i];
+      if (s.mode != kModeResize) {
+        continue;
+      }
+      const int stages = (int)std::min(8.0, std::max(1.0, walk / stage_cost(s, s.walk_px)));
+      longest = longest && stages == 8;
+      // as few CTAs as that makes, with the rows dealt evenly, in fours
+      const int down = (s.post_h + 4 * stages * kWarps - 1) / (4 * stages * kWarps);
+      int rows = ((s.post_h + down * kWarps - 1) / (down * kWarps) + 3) / 4 * 4;
+      while (rows > 4 && walk_steps(s, rows) > kStripMaxSteps) {
+        rows -= 4;
+      }
+      s.walk_rows = rows;
+      plan.steps = std::max(plan.steps, (int32_t)walk_steps(s, rows));
+      ctas += (long long)s.walk_chunks * ((s.post_h + rows * kWarps - 1) / (rows * kWarps));
     }
-    const int stages = (int)std::min(8.0, std::max(1.0, walk / stage_cost(s, s.walk_px)));
-    // as few CTAs as that makes, with the rows dealt evenly, in fours
-    const int down = (s.post_h + 4 * stages * kWarps - 1) / (4 * stages * kWarps);
-    int rows = ((s.post_h + down * kWarps - 1) / (down * kWarps) + 3) / 4 * 4;
-    while (rows > 4 && walk_steps(s, rows) > kStripMaxSteps) {
-      rows -= 4;
+    // A small batch: whole CTAs make the one round a little more than one, which takes as
+    // long as two; longer walks until it is one.  4 and 8 images of 900x1100 px, shorter
+    // side 224: 20.5 and 28.9 us a pass before, 18.4 and 24.6 so (896 CTAs for 740 places
+    // in the second); beyond 1.3 rounds it costs more than it gives (32 images of 200-500
+    // px to 224x224, 1.4 rounds: 23.9 and 24.4).
+    if (walk > kLeast || ctas <= 148 * kStripCtas || 10 * ctas > 13 * 148 * kStripCtas || longest) {
+      return;
     }
-    s.walk_rows = rows;
-    plan.steps = std::max(plan.steps, (int32_t)walk_steps(s, rows));
+    walk *= 1.15;
   }
 }
 
