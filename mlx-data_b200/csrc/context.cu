@@ -226,7 +226,8 @@ int plan_samples(
 }
 
 // Source samples of an n_src -> n_dst axis that outputs [o_lo, o_hi) can read,
-// widened by `margin` on both sides and clipped to the axis.
+// widened by `margin` on both sides (none: the exact span, for statistics) and clipped
+// to the axis.
 static void axis_span(int64_t n_src, int64_t n_dst, int64_t o_lo, int64_t o_hi, int margin, int64_t& lo, int64_t& hi) {
   if (n_src == n_dst) {
     lo = o_lo;
@@ -236,6 +237,10 @@ static void axis_span(int64_t n_src, int64_t n_dst, int64_t o_lo, int64_t o_hi, 
     const double radius = ratio > 1.0 ? ratio : 1.0;
     lo = (int64_t)std::floor((o_lo + 0.5) * ratio - 0.5 - radius) - margin;
     hi = (int64_t)std::ceil((o_hi - 0.5) * ratio - 0.5 + radius) + 1 + margin;
+    if (margin > 0) {
+      lo -= axis_slack((int32_t)n_src);
+      hi += axis_slack((int32_t)n_src);
+    }
   }
   lo = std::max<int64_t>(lo, 0);
   hi = std::min<int64_t>(hi, n_src);

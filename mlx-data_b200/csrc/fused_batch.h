@@ -150,6 +150,14 @@ void plan_resize(DevSample* samples, int n, int channels, ResizePlan& plan);
 // host copy of the sample table.
 void choose_kernels(LaunchParams& p, ResizePlan& plan, const DevSample* host_samples, int n);
 
+// Samples by which the distance of two taps of an axis of n source samples can exceed
+// its exact value, beyond the one that the bounds below always add: a tap's position
+// goes through at most four float32 roundings (and the ratio's), each of them half a
+// unit in the last place of n, together below n * 2^-22, at either end.
+__host__ __device__ constexpr int32_t axis_slack(int32_t n) {
+  return n >> 21;
+}
+
 // Conservative per-axis bounds used by the host planner.
 struct AxisPlan {
   int32_t cap;      // tap-count bound

@@ -78,18 +78,19 @@ void choose_kernels(LaunchParams& p, ResizePlan& plan, const DevSample* host_sam
 
 AxisPlan plan_axis(int32_t n_src, int32_t n_dst, int32_t sub) {
   AxisPlan a;
+  const int32_t slack = axis_slack(n_src);
   if (n_src <= n_dst) {
-    a.cap = 4;
-    a.extent = sub + 4;
+    a.cap = 4 + slack;
+    a.extent = sub + 4 + slack;
     return a;
   }
   // Output o reads taps ceil(u - R) .. floor(u + R) with u = (o + 0.5) * ratio - 0.5
   // and R = ratio: at most floor(2R) + 1 of them, and `sub` consecutive
   // outputs span at most (sub - 1) * ratio + 2R + 1 source samples.  One more
-  // of each covers the float32 rounding of u and R in the kernel.
+  // of each and the slack cover the float32 rounding of u and R in the kernel.
   const double ratio = (double)n_src / (double)n_dst;
-  a.cap = (int32_t)std::floor(2.0 * ratio) + 2;
-  a.extent = (int32_t)std::ceil((double)(sub - 1) * ratio + 2.0 * ratio) + 2;
+  a.cap = (int32_t)std::floor(2.0 * ratio) + 2 + slack;
+  a.extent = (int32_t)std::ceil((double)(sub - 1) * ratio + 2.0 * ratio) + 2 + slack;
   return a;
 }
 
@@ -101,18 +102,25 @@ static long long walk_row_bytes(const DevSample& s, int channels, int px) {
 
 // Steps of a walk over `rows` output rows: every source row once, again once
 // per output row whose neighbours on both sides reach it, one per output row
-// at least.  (Enlargements walk the two rows of every output row.)
+// at least.  (Enlargements walk the two rows of every output row.)  Rounding lets
+// neighbours reach that much further into each other.
 static long long walk_steps(const DevSample& s, int rows) {
   const long long extent = plan_axis(s.pre_h, s.geom_h, rows).extent;
-  return s.pre_h <= s.geom_h ? 4LL * rows + 4 : extent + rows + 8;
+  const long long again = (long long)rows * axis_slack(s.pre_h);
+  return again + (s.pre_h <= s.geom_h ? 4LL * rows + 4 : extent + rows + 8);
+}
+
+// Whether one output column and one output row fit a chunk of resize_walk.cu.
+static bool walk_fits(const DevSample& s, int channels) {
+  return walk_row_bytes(s, channels, 1) <= kWalkRow && walk_steps(s, 1) <= kWalkMaxSteps && s.cap_x <= kWalkMaxTaps;
 }
 
 // Source bytes of `px` output columns of a strip.  The last of them is centred
 // (px - 1) ratios behind the first, and both reach one radius further; two more
-// columns cover the ends' fractions and the float32 rounding of the kernel.
+// columns and the slack cover the ends' fractions and the float32 rounding of the kernel.
 static long long strip_bytes(const DevSample& s, int channels, int px) {
   const double ratio = s.axis_x[0];
-  const long long cols = (long long)std::ceil((px - 1) * ratio + 2.0 * std::max(1.0, ratio)) + 2;
+  const long long cols = (long long)std::ceil((px - 1) * ratio + 2.0 * std::max(1.0, ratio)) + 2 + axis_slack(s.pre_w);
   return std::min<long long>(cols, s.pre_w) * channels;
 }
 
@@ -134,7 +142,7 @@ static int strip_most_px(const DevSample& s, int channels) {
 // Bound on the source rows that `rows` output rows read.
 static int strip_span(const DevSample& s, int rows) {
   const double ratio = s.axis_y[0];
-  return (int)std::min(1e6, (rows - 1) * ratio + 2.0 * std::max(1.0, ratio)) + 2;
+  return (int)std::min(1e6, (rows - 1) * ratio + 2.0 * std::max(1.0, ratio)) + 2 + axis_slack(s.pre_h);
 }
 
 Mode resize_mode(DevSample& s, int channels) {
@@ -147,8 +155,7 @@ Mode resize_mode(DevSample& s, int channels) {
       strip_span(s, 1) <= kStripSlots) {
     return kModeResize;
   }
-  return walk_row_bytes(s, channels, 1) <= kWalkRow && walk_steps(s, 1) <= kWalkMaxSteps ? kModeResizeWide
-                                                                                          : kModeResizeDirect;
+  return walk_fits(s, channels) ? kModeResizeWide : kModeResizeDirect;
 }
 
 // Instructions of a warp per stage of four output rows of a strip `px` columns wide,
@@ -182,6 +189,7 @@ static void split_strips(DevSample& s) {
 // Chunks of at most `px` columns and walks of at most `rows` rows, smaller
 // where the source footprint asks for it.
 static void split_walk(DevSample& s, int channels, int px, int rows) {
+  px = std::min(px, kWalkMaxTaps / s.cap_x);   // (acts on axes with slack alone)
   if (walk_row_bytes(s, channels, px) > kWalkRow) {
     // (px + 1) * ratio + 3 source columns at most (plan_axis), then down to what fits
     const double ratio = (double)s.pre_w / (double)s.geom_w;
@@ -298,7 +306,7 @@ void plan_resize(DevSample* samples, int n, int channels, ResizePlan& plan) {
   }
   for (int i = 0; 4 * meet > resizes && i < n; i++) {
     DevSample& s = samples[i];
-    if (s.mode == kModeResize && walk_row_bytes(s, channels, 1) <= kWalkRow && walk_steps(s, 1) <= kWalkMaxSteps) {
+    if (s.mode == kModeResize && walk_fits(s, channels)) {
       s.mode = kModeResizeWide;
     }
   }

@@ -60,3 +60,18 @@ def test_far_beyond_both_in_ragged_slots(pkg, ctx, oracle, c):
     ops = [("image_random_h_flip", dict(key="image", prob=0.5)), ("image_resize_smallest_side", dict(key="image", size=3)),
            ("image_random_h_flip", dict(key="image", prob=0.5))]
     _check(pkg, ctx, oracle, [(1700, 1700), (1700, 2300), (5, 3), (40, 70), (3, 8), (1530, 1280)], c, ops, seed=c)
+
+
+# (along which axis, source and result, channels): the planner's bounds have to hold float32 positions that
+# are a sample or two off at this distance from the image's edge
+@pytest.mark.parametrize("axis,n,m,c", [("y", 9716434, 8426337, 1), ("y", 9489329, 6289399, 1), ("y", 8597653, 3954443, 1),
+                                        ("x", 8865487, 9554784, 3), ("x", 9446063, 2688457, 3)])
+def test_sides_beyond_the_integers_of_float32(pkg, oracle, axis, n, m, c):
+    img = np.random.default_rng(n).integers(0, 256, (n, 2, c) if axis == "y" else (2, n, c), dtype=np.uint8)
+    w, h = (2, m) if axis == "y" else (m, 2)
+    own = pkg.Context(device=0, n_lanes=1)
+    try:
+        got = own.image_resize(img, w, h)
+    finally:
+        own.close()
+    assert np.array_equal(got, oracle.resize(img, w, h))
