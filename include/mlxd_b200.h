@@ -219,7 +219,13 @@ MLXD_API int mlxd_batch_wait(mlxd_ctx* ctx, int lane, int timeout_ms);
 
 /* Same work for device-resident sources and destination, launched on the
  * caller's CUDA stream (a cudaStream_t passed as void*; NULL is the default
- * stream).  Nothing is copied except the descriptors. */
+ * stream).  Nothing is copied except the descriptors.
+ *
+ * A stream under capture gets the call as nodes of the graph: the descriptors become
+ * the graph's own, in an allocation node, so such a graph follows the rules of graphs
+ * with memory nodes (one instance at a time, no child graph).  A replay reads the
+ * sources and writes the destination given here, and sets the self-check word of this
+ * context, which therefore has to outlive the graph; it is not timed. */
 MLXD_API int mlxd_fused_batch_on_stream(
     mlxd_ctx* ctx, void* cuda_stream, const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* batch);
 

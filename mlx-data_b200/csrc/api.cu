@@ -1,6 +1,7 @@
 // extern "C" entry points declared in include/mlxd_b200.h.
 #include <cstring>
 #include <new>
+#include <optional>
 
 #include "context.h"
 
@@ -270,9 +271,18 @@ int mlxd_fused_batch_on_stream(
   std::vector<DevSample> dev;
   mlxd_batch_desc b = *batch;
   Lane& ring = *ctx->lanes[ctx->n_user_lanes + 1];
-  LutUse table_in_use(ctx);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  MLXD_CUDA(cudaStreamIsCapturing(stream, &capture));
+  const bool captured = capture != cudaStreamCaptureStatusNone;
+  std::optional<LutUse> table_in_use;
   LaunchParams p;
-  int rc = prepare_launch(ctx, &b, n, p);
+  int rc;
+  if (captured) {
+    rc = describe_launch(&b, n, p);
+  } else {
+    table_in_use.emplace(ctx);
+    rc = prepare_launch(ctx, &b, n, p);
+  }
   if (rc != MLXD_OK) {
     return rc;
   }
@@ -294,6 +304,15 @@ int mlxd_fused_batch_on_stream(
   }
   ctx->algo_src += algo_src;
   ctx->algo_dst += slot_bytes * n;
+  if (captured) {
+    rc = capture_batch(p, plan, dev.data(), &b, stream);
+    if (rc == MLXD_OK) {
+      ctx->batches += 1;
+      ctx->samples += n;
+      ctx->launches += 1;
+    }
+    return rc;
+  }
   std::lock_guard<std::mutex> guard(ring.mu);
   const int slot = ring.next_slot;
   ring.next_slot = (slot + 1) % kDescSlots;
@@ -301,26 +320,21 @@ int mlxd_fused_batch_on_stream(
   // means neither the copy nor the kernel still needs the tables.
   MLXD_CUDA(cudaEventSynchronize(ring.desc_copied[slot]));
   harvest_timing(ctx, ring, slot, true);
-  rc = arena_reserve(ctx, ring.h_desc[slot], sizeof(DevSample) * n, true, nullptr);
-  if (rc != MLXD_OK) {
-    return rc;
-  }
-  rc = arena_reserve(ctx, ring.d_desc[slot], sizeof(DevSample) * n, false, nullptr);
+  const size_t table_bytes = sizeof(DevSample) * n;
+  rc = arena_reserve(ctx, ring.d_desc[slot], table_bytes, false, nullptr);
   if (rc != MLXD_OK) {
     return rc;
   }
   // A table of at most 64 KB is taken from ordinary memory: the driver copies it into
   // the command stream before the call returns, which costs a pass 2 us where a copy
   // from page-locked memory, started by a copy engine, costs 6 (32 to 240 samples
-  // ahead of a kernel of 20 us).  A stream under capture would read the memory again
-  // whenever its graph runs, so there the table comes from the slot's block.
-  const size_t table_bytes = sizeof(DevSample) * n;
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (table_bytes <= 64 * 1024) {
-    MLXD_CUDA(cudaStreamIsCapturing(stream, &capture));
-  }
+  // ahead of a kernel of 20 us).
   const void* table = dev.data();
-  if (table_bytes > 64 * 1024 || capture != cudaStreamCaptureStatusNone) {
+  if (table_bytes > 64 * 1024) {
+    rc = arena_reserve(ctx, ring.h_desc[slot], table_bytes, true, nullptr);
+    if (rc != MLXD_OK) {
+      return rc;
+    }
     std::memcpy(ring.h_desc[slot].ptr, dev.data(), table_bytes);
     table = ring.h_desc[slot].ptr;
   }

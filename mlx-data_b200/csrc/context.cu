@@ -335,8 +335,7 @@ int get_lut(mlxd_ctx* ctx, const mlxd_batch_desc* b, int c_out, const float** lu
   return MLXD_OK;
 }
 
-int prepare_launch(
-    mlxd_ctx* ctx, const mlxd_batch_desc* b, int n, LaunchParams& p) {
+int describe_launch(const mlxd_batch_desc* b, int n, LaunchParams& p) {
   if (b->channels < 1 || b->channels > 4) {
     return fail(MLXD_ERR_INVALID, "image: channels must be 0 < c <= 4");
   }
@@ -362,17 +361,18 @@ int prepare_launch(
   p.gray_bias = b->gray_bias;
   p.out_f32 = b->out_dtype == MLXD_F32;
   p.pad_px = (int32_t)(uint8_t)(int32_t)b->pad_value;
-  p.status = ctx->d_status;   // callers point this at their lane's word
-  if (p.out_f32) {
-    if (!(b->divisor != 0.0f)) {
-      return fail(MLXD_ERR_INVALID, "cast divisor must be non-zero");
-    }
-    int rc = get_lut(ctx, b, p.c_out, &p.lut);
-    if (rc != MLXD_OK) {
-      return rc;
-    }
+  if (p.out_f32 && !(b->divisor != 0.0f)) {
+    return fail(MLXD_ERR_INVALID, "cast divisor must be non-zero");
   }
   return MLXD_OK;
+}
+
+int prepare_launch(mlxd_ctx* ctx, const mlxd_batch_desc* b, int n, LaunchParams& p) {
+  const int rc = describe_launch(b, n, p);
+  if (rc != MLXD_OK || !p.out_f32) {
+    return rc;
+  }
+  return get_lut(ctx, b, p.c_out, &p.lut);
 }
 
 // Threads that pack one batch's pageable sources (the caller included):

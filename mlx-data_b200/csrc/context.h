@@ -150,8 +150,14 @@ int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, 
 // The cast table of a batch descriptor: table[c * 256 + v], c < c_out.
 void compute_cast_table(const mlxd_batch_desc* b, int c_out, float* table);
 
-// Launch-wide parameters (cast table included) from a batch descriptor.
+// Launch-wide parameters from a batch descriptor, without the cast table, and with it.
+int describe_launch(const mlxd_batch_desc* b, int n, LaunchParams& p);
 int prepare_launch(mlxd_ctx* ctx, const mlxd_batch_desc* b, int n, LaunchParams& p);
+
+// The launch of a described and planned batch as nodes of the graph that `stream` is
+// being captured into, tables included.
+int capture_batch(
+    LaunchParams& p, const ResizePlan& plan, const DevSample* samples, const mlxd_batch_desc* batch, cudaStream_t stream);
 
 // Device cast table for a batch descriptor (cached per context).
 int get_lut(mlxd_ctx* ctx, const mlxd_batch_desc* b, int c_out, const float** lut);
