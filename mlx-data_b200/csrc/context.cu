@@ -142,7 +142,7 @@ static int check_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc*
   return MLXD_OK;
 }
 
-int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, DevSample& out) {
+int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, const DevSample* before, DevSample& out) {
   {
     int rc = check_sample(d, i, b, b->slot_h, b->slot_w);
     if (rc != MLXD_OK) {
@@ -173,13 +173,18 @@ int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, 
       if (d.pre_w == d.geom_w && d.pre_h == d.geom_h) {
         s.mode = kModeCopy;  // identity on both axes
       } else {
-        s.cap_x = plan_axis(s.pre_w, s.geom_w, 1).cap;
-        // the divisions of make_axis(), correctly rounded here as there
-        s.axis_x[0] = (float)s.pre_w / (float)s.geom_w;
-        s.axis_x[1] = std::min(1.0f, (float)s.geom_w / (float)s.pre_w);
-        s.axis_y[0] = (float)s.pre_h / (float)s.geom_h;
-        s.axis_y[1] = std::min(1.0f, (float)s.geom_h / (float)s.pre_h);
-        s.mode = resize_mode(s, b->channels);
+        if (before && is_resize(*before) && s.pre_w == before->pre_w && s.pre_h == before->pre_h &&
+            s.geom_w == before->geom_w && s.geom_h == before->geom_h && s.post_w == before->post_w &&
+            s.src_w == before->src_w) {
+          // like the sample before it, as in a batch of frames
+          std::memcpy(s.mx, before->mx, sizeof(s.mx));
+          s.cap_x = before->cap_x;
+          s.walk_px = before->walk_px;
+          s.mode = before->mode;
+        } else {
+          set_axes(s);
+          s.mode = resize_mode(s, b->channels);
+        }
       }
     } else if (d.geom == MLXD_GEOM_AFFINE) {
       s.mode = kModeAffine;
@@ -199,7 +204,7 @@ int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, 
 
 int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, DevSample* out, ResizePlan& plan) {
   for (int i = 0; i < n; i++) {
-    const int rc = plan_one_sample(samples[i], i, b, out[i]);
+    const int rc = plan_one_sample(samples[i], i, b, i > 0 ? &out[i - 1] : nullptr, out[i]);
     if (rc != MLXD_OK) {
       return rc;
     }

@@ -142,8 +142,10 @@ const uint8_t* pinned_registry_lookup(const void* host);
 
 cudaError_t launch_gather_rows(const GatherPiece* table_dev, int n, uint32_t total_rows, cudaStream_t stream);
 
-// One sample of plan_samples, without its share of the launch.
-int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, DevSample& out);
+// One sample of plan_samples, without its share of the launch; `before` is the sample
+// planned before it, if any.
+int plan_one_sample(
+    const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, const DevSample* before, DevSample& out);
 // plan_samples into caller-owned storage of n entries.
 int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, DevSample* out, ResizePlan& plan);
 

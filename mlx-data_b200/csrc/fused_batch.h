@@ -70,7 +70,8 @@ struct __align__(16) DevSample {
   union {
     float mx[6];          // affine
     struct {
-      float axis_x[2], axis_y[2];   // resize_strip.cu: Axis::ratio and Axis::fs
+      float axis_x[2], axis_y[2];   // resizes: Axis::ratio and Axis::fs
+      float stage_cost;             // the planner's, of four output rows of a strip
     };
   };
   int32_t walk_part;      // resize_strip.cu: output rows whose source rows are in shared memory together, 1, 2 or 4
@@ -106,6 +107,10 @@ struct ResizePlan {
   int32_t first_wide, wides;   // all of them are among these samples
 };
 
+__host__ __device__ inline bool is_resize(const DevSample& s) {
+  return s.mode == kModeResize || s.mode == kModeResizeWide || s.mode == kModeResizeDirect;
+}
+
 // Strips of padding beside the post window.
 __host__ __device__ inline int walk_strips(const DevSample& s) {
   return (s.slot_w - s.post_w + kWalkPadPx - 1) / kWalkPadPx;
@@ -139,7 +144,11 @@ cudaError_t launch_fused_batch(const LaunchParams& p, const ResizePlan& plan, cu
 cudaError_t launch_resize_strip(const LaunchParams& p, const StripPlan& plan, cudaStream_t stream);
 cudaError_t launch_resize_walk(const LaunchParams& p, bool fills_padding, cudaStream_t stream);
 
-// The kernel that runs a resize, axis_x and axis_y in place.
+// axis_x, axis_y (the divisions of make_axis(), correctly rounded here as there) and
+// cap_x of a resize.
+void set_axes(DevSample& s);
+
+// The kernel that runs a resize, its axes set.
 Mode resize_mode(DevSample& s, int channels);
 
 // Split the resize samples of a batch into CTAs (DevSample::walk_*) and size

@@ -115,13 +115,14 @@ static bool walk_fits(const DevSample& s, int channels) {
   return walk_row_bytes(s, channels, 1) <= kWalkRow && walk_steps(s, 1) <= kWalkMaxSteps && s.cap_x <= kWalkMaxTaps;
 }
 
-// Source bytes of `px` output columns of a strip.  The last of them is centred
+// Source columns of `px` output columns of a strip.  The last of them is centred
 // (px - 1) ratios behind the first, and both reach one radius further; two more
 // columns and the slack cover the ends' fractions and the float32 rounding of the kernel.
-static long long strip_bytes(const DevSample& s, int channels, int px) {
-  const double ratio = s.axis_x[0];
-  const long long cols = (long long)std::ceil((px - 1) * ratio + 2.0 * std::max(1.0, ratio)) + 2 + axis_slack(s.pre_w);
-  return std::min<long long>(cols, s.pre_w) * channels;
+static int strip_columns(const DevSample& s, int px) {
+  const float ratio = s.axis_x[0];
+  const float span = std::min(1e6f, (float)(px - 1) * ratio + 2.0f * std::max(1.0f, ratio));
+  const int whole = (int)span;
+  return whole + (whole < span) + 2 + axis_slack(s.pre_w);
 }
 
 // The widest strip that fits; 0 when not even one column does.
@@ -130,10 +131,11 @@ static int strip_most_px(const DevSample& s, int channels) {
   if ((long long)s.pre_w * channels <= kStripRow) {
     return most;
   }
-  const double ratio = s.axis_x[0];
-  const int guess = (int)((kStripRow / channels - 2 - 2.0 * std::max(1.0, ratio)) / ratio) + 1;
-  int px = std::max(0, std::min(most, guess));
-  while (px > 0 && strip_bytes(s, channels, px) > kStripRow) {
+  const int columns = kStripRow / channels;
+  const float ratio = s.axis_x[0];
+  const float guess = ((float)(columns - 2) - 2.0f * std::max(1.0f, ratio)) / ratio + 1.0f;
+  int px = guess < (float)most ? std::max(0, (int)guess) : most;
+  while (px > 0 && strip_columns(s, px) > columns) {
     px--;
   }
   return px;
@@ -141,8 +143,28 @@ static int strip_most_px(const DevSample& s, int channels) {
 
 // Bound on the source rows that `rows` output rows read.
 static int strip_span(const DevSample& s, int rows) {
-  const double ratio = s.axis_y[0];
-  return (int)std::min(1e6, (rows - 1) * ratio + 2.0 * std::max(1.0, ratio)) + 2 + axis_slack(s.pre_h);
+  const float ratio = s.axis_y[0];
+  return (int)std::min(1e6f, (float)(rows - 1) * ratio + 2.0f * std::max(1.0f, ratio)) + 2 + axis_slack(s.pre_h);
+}
+
+// walk_steps() from the ratio in the sample's record.
+static int strip_steps(const DevSample& s, int rows) {
+  const int slack = axis_slack(s.pre_h);
+  if (s.pre_h <= s.geom_h) {
+    return rows * (4 + slack) + 4;
+  }
+  const float span = (float)(rows + 1) * s.axis_y[0];
+  const int whole = (int)span;
+  return whole + (whole < span) + slack + 2 + rows * (1 + slack) + 8;
+}
+
+void set_axes(DevSample& s) {
+  s.axis_x[0] = (float)s.pre_w / (float)s.geom_w;
+  s.axis_x[1] = s.pre_w > s.geom_w ? std::min(1.0f, (float)s.geom_w / (float)s.pre_w) : 1.0f;
+  s.axis_y[0] = (float)s.pre_h / (float)s.geom_h;
+  s.axis_y[1] = s.pre_h > s.geom_h ? std::min(1.0f, (float)s.geom_h / (float)s.pre_h) : 1.0f;
+  // plan_axis(): floor(2r) + 2 taps, which rounding r to a float cannot make fewer
+  s.cap_x = (s.pre_w > s.geom_w ? (int32_t)(2.0f * s.axis_x[0]) + 2 : 4) + axis_slack(s.pre_w);
 }
 
 Mode resize_mode(DevSample& s, int channels) {
@@ -158,32 +180,40 @@ Mode resize_mode(DevSample& s, int channels) {
   return walk_fits(s, channels) ? kModeResizeWide : kModeResizeDirect;
 }
 
-// Instructions of a warp per stage of four output rows of a strip `px` columns wide,
-// as measured by taking parts of the kernel away: the steps down the source rows,
-// then passes of 32 columns.
-static double stage_cost(const DevSample& s, int px) {
-  const double rx = s.axis_x[0], ry = s.axis_y[0];
-  const double vertical = 4.0 * std::max(ry, 1.5) * 30.0 + 150.0;
-  const double pass = (2.0 * std::max(rx, 1.0) + 1.0) * 17.0 + 90.0;
-  return vertical + (px + 31) / 32 * pass;
+// Instructions of a warp per stage of four output rows of a strip, as measured by taking
+// parts of the kernel away: the steps down the source rows, then passes of 32 columns.
+static float stage_rows_cost(const DevSample& s) {
+  return std::max(s.axis_y[0], 1.5f) * 120.0f + 150.0f;
+}
+
+static float stage_pass_cost(const DevSample& s) {
+  return std::max(s.axis_x[0], 1.0f) * 34.0f + 107.0f;
 }
 
 // How many strips: the fewer, the fewer walks down the source rows; the horizontal
-// half works on 32 columns at a time, so strips of whole 32s waste no lanes.
+// half works on 32 columns at a time, so strips of whole 32s waste no lanes.  More
+// strips than the least can at best save the passes above `whole`, which most often
+// does not make up for one more walk: then nothing else is tried.
 static void split_strips(DevSample& s) {
   const int most = s.walk_px;
-  double best = 0.0;
-  int chosen = 0;
-  for (int passes = (most + 31) / 32; passes > 0; passes--) {
-    const int strips = (s.post_w + std::min(most, 32 * passes) - 1) / std::min(most, 32 * passes);
-    const double cost = strips * stage_cost(s, (s.post_w + strips - 1) / strips);
-    if (chosen == 0 || cost < best) {
+  const float rows = stage_rows_cost(s), pass = stage_pass_cost(s);
+  const int least = most >= s.post_w ? 1 : (s.post_w + most - 1) / most;
+  const int whole = (s.post_w + 31) >> 5;
+  s.walk_px = least == 1 ? s.post_w : (s.post_w + least - 1) / least;
+  const int passes = (s.walk_px + 31) >> 5;
+  float best = (float)least * (rows + (float)passes * pass);
+  const float bound = (float)(least + 1) * rows + (float)whole * pass;
+  for (int p = passes - 1; p > 0 && best > bound; p--) {
+    const int strips = (s.post_w + 32 * p - 1) / (32 * p);
+    const int px = (s.post_w + strips - 1) / strips;
+    const float cost = (float)strips * (rows + (float)((px + 31) >> 5) * pass);
+    if (cost < best) {
       best = cost;
-      chosen = strips;
+      s.walk_px = px;
     }
   }
-  s.walk_px = (s.post_w + chosen - 1) / chosen;
-  s.walk_chunks = (s.post_w + s.walk_px - 1) / s.walk_px;
+  s.walk_chunks = s.walk_px == s.post_w ? 1 : (s.post_w + s.walk_px - 1) / s.walk_px;
+  s.stage_cost = rows + (float)((s.walk_px + 31) >> 5) * pass;
 }
 
 // Chunks of at most `px` columns and walks of at most `rows` rows, smaller
@@ -209,20 +239,34 @@ static void split_walk(DevSample& s, int channels, int px, int rows) {
 
 static void plan_strips(DevSample* samples, int n, StripPlan& plan) {
   constexpr int kWarps = kStripThreads / 32;
-  constexpr double kWarpsAtOnce = 148 * kStripCtas * kWarps;
+  constexpr float kWarpsAtOnce = 148 * kStripCtas * kWarps;
   plan = StripPlan{};
   double total = 0.0;
+  const DevSample* last = nullptr;   // the sample before: like ones are split once
+  int last_most = 0;
   for (int i = 0; i < n; i++) {
     DevSample& s = samples[i];
-    if (s.mode == kModeResize) {
+    if (s.mode != kModeResize) {
+      continue;
+    }
+    const int most = s.walk_px;
+    if (last && most == last_most && s.post_w == last->post_w && s.pre_h == last->pre_h && s.axis_x[0] == last->axis_x[0] &&
+        s.axis_y[0] == last->axis_y[0]) {
+      s.walk_px = last->walk_px;
+      s.walk_chunks = last->walk_chunks;
+      s.walk_part = last->walk_part;
+      s.stage_cost = last->stage_cost;
+    } else {
       split_strips(s);
       s.walk_part = strip_span(s, 4) <= kStripSlots ? 4 : strip_span(s, 2) <= kStripSlots ? 2 : 1;
-      const int columns = (s.walk_px + 31) / 32 * 32;
-      plan.columns = std::max(plan.columns, columns);
-      plan.taps = std::max(plan.taps, columns * s.cap_x);
       plan.slots = std::max(plan.slots, strip_span(s, s.walk_part));
-      total += (double)s.walk_chunks * ((s.post_h + 3) / 4) * stage_cost(s, s.walk_px);
     }
+    const int columns = (s.walk_px + 31) / 32 * 32;
+    plan.columns = std::max(plan.columns, columns);
+    plan.taps = std::max(plan.taps, columns * s.cap_x);
+    total += (double)(s.walk_chunks * ((s.post_h + 3) / 4)) * s.stage_cost;
+    last = &s;
+    last_most = most;
   }
   if (total == 0.0) {
     return;
@@ -233,28 +277,38 @@ static void plan_strips(DevSample* samples, int n, StripPlan& plan) {
   // have one.  96 images of 240-640 px to 224x224: 51 us a pass so, 56 in one round, 66
   // where every walk has 8 rows; 256 of 256-800 px: 121, 125 in two and a half rounds,
   // 149 in eight.
-  constexpr double kRounds = 1.5, kLeast = 2500.0;
-  double walk = std::max(total / kWarpsAtOnce / kRounds, std::min(total / kWarpsAtOnce, kLeast));
+  constexpr float kRounds = 1.5f, kLeast = 2500.0f;
+  const float each = (float)total / kWarpsAtOnce;
+  float walk = std::max(each / kRounds, std::min(each, kLeast));
   for (;;) {
     long long ctas = 0;
     bool longest = true;
     plan.steps = 0;
+    int stages = 0, post_h = 0, even = 0, down = 0;   // of the sample before
     for (int i = 0; i < n; i++) {
       DevSample& s = samples[i];
       if (s.mode != kModeResize) {
         continue;
       }
-      const int stages = (int)std::min(8.0, std::max(1.0, walk / stage_cost(s, s.walk_px)));
+      const int most = (int)std::min(8.0f, std::max(1.0f, walk / s.stage_cost));
+      if (most != stages || s.post_h != post_h) {
+        // as few CTAs as that makes, with the rows dealt evenly, in fours
+        stages = most;
+        post_h = s.post_h;
+        down = (post_h + 4 * kWarps * stages - 1) / (4 * kWarps * stages);
+        even = (post_h + 4 * kWarps * down - 1) / (4 * kWarps * down) * 4;
+        down = (post_h + even * kWarps - 1) / (even * kWarps);
+      }
       longest = longest && stages == 8;
-      // as few CTAs as that makes, with the rows dealt evenly, in fours
-      const int down = (s.post_h + 4 * stages * kWarps - 1) / (4 * stages * kWarps);
-      int rows = ((s.post_h + down * kWarps - 1) / (down * kWarps) + 3) / 4 * 4;
-      while (rows > 4 && walk_steps(s, rows) > kStripMaxSteps) {
+      int rows = even;
+      int steps = strip_steps(s, rows);
+      while (rows > 4 && steps > kStripMaxSteps) {
         rows -= 4;
+        steps = strip_steps(s, rows);
       }
       s.walk_rows = rows;
-      plan.steps = std::max(plan.steps, (int32_t)walk_steps(s, rows));
-      ctas += (long long)s.walk_chunks * ((s.post_h + rows * kWarps - 1) / (rows * kWarps));
+      plan.steps = std::max(plan.steps, steps);
+      ctas += s.walk_chunks * (long long)(rows == even ? down : (post_h + rows * kWarps - 1) / (rows * kWarps));
     }
     // A small batch: whole CTAs make the one round a little more than one, which takes as
     // long as two; longer walks until it is one.  4 and 8 images of 900x1100 px, shorter
@@ -264,7 +318,7 @@ static void plan_strips(DevSample* samples, int n, StripPlan& plan) {
     if (walk > kLeast || ctas <= 148 * kStripCtas || 10 * ctas > 13 * 148 * kStripCtas || longest) {
       return;
     }
-    walk *= 1.15;
+    walk *= 1.15f;
   }
 }
 
