@@ -546,7 +546,9 @@ __device__ __forceinline__ void walk_cell(
     const unsigned below = (1u << lane) - 1u;
     const unsigned less = (at & 4 ? ~b2 : 0u) | (e2 & ((at & 2 ? ~b1 : 0u) | (e1 & (at & 1 ? ~b0 : 0u))));
     const int place = valid ? __popc(all & (less | (e2 & e1 & e0 & below))) : __popc(all) + __popc(~all & below);
-    const int e = pass * 32 + (place & 3) * 8 + (place >> 2);
+    // In an enlargement neighbouring columns read the same pixels, which one access serves:
+    // there they stay together (141 images of 41x41x4 to 174x174: 61.8 us dealt, 41.4 so).
+    const int e = pass * 32 + (ax.ratio < 1.0f ? lane : (place & 3) * 8 + (place >> 2));
     if (share == 0) {
       uint32_t* hx = sp<uint32_t>(c.hx + 8u * (unsigned)e);
       hx[0] = (uint32_t)((at * 16) & 0xffff) | ((uint32_t)cnt << 16);

@@ -60,3 +60,10 @@ def test_rows_that_start_at_any_byte(pkg, ctx, oracle):
     for cut in range(5):
         ops = [("image_center_crop", dict(key="image", w=100 + cut, h=60)), ("image_resize", dict(key="image", w=90, h=44))]
         _check(pkg, ctx, oracle, [(70, 120 + k) for k in range(6)], 3, ops, seed=cut, casts=(None,))
+
+
+# which lane takes which column: an enlargement's stay in order, a shrink's are dealt
+@pytest.mark.parametrize("c", [1, 2, 3, 4])
+def test_order_of_columns(pkg, ctx, oracle, c):
+    ops = [("image_random_h_flip", dict(key="image", prob=0.5)), ("image_resize", dict(key="image", w=70, h=21))]
+    _check(pkg, ctx, oracle, [(20, w) for w in (1, 5, 34, 35, 36, 69, 70, 71, 72, 141)], c, ops, seed=c)
