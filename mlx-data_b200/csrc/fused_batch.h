@@ -28,7 +28,8 @@ constexpr int kStripMaxPx = 256;      // output columns per strip
 constexpr int kStripMinPx = 11;
 constexpr int kStripMaxTaps = 32 * (2 * kStripRow / (kStripMinPx + 1) + 4);
 
-// Resize kernel for strong shrinks (resize_walk.cu): a CTA walks down a chunk of columns.
+// Resize kernel of strong shrinks and what goes with them (resize_walk.cu): a CTA walks down
+// a chunk of columns.
 constexpr int kWalkThreads = 128;
 constexpr int kWalkRow = 832;       // floats per row in shared memory: source bytes of a chunk, alignment included
 constexpr int kWalkMaxRows = 32;    // output rows per CTA
@@ -46,7 +47,8 @@ constexpr int kWalkPadPx = 256;     // columns per strip of padding
 // above 412, 205, 136, 102 along a row for 1 to 4 channels) or one row's 2r + 11
 // steps exceed kWalkMaxSteps (above 506 down the rows).  Every output pixel is then
 // filtered straight from global memory by resize_direct_kernel.
-// kModeResizeWide: a resize that is too strong for resize_strip.cu.
+// kModeResizeWide: a resize that resize_walk.cu runs: one too strong for resize_strip.cu, or
+// one of a batch that goes there (launch_plan.cu: choose_resize_kernel).
 enum Mode : int32_t { kModeCopy = 0, kModeResize = 1, kModeAffine = 2, kModeResizeDirect = 3, kModeResizeWide = 4 };
 
 // One sample's program.  Coordinates name four nested images:
@@ -91,7 +93,7 @@ struct StripPlan {
   int32_t linear;        // blocks are numbered through, not by three coordinates (set at launch)
 };
 
-// The same for the resize kernel of strong shrinks.
+// The same for resize_walk.cu.
 struct WalkPlan {
   int32_t px;         // columns of the widest chunk (0: no sample runs the resize kernel)
   int32_t taps;       // horizontal weights of a chunk

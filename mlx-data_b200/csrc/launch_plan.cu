@@ -322,11 +322,12 @@ static void plan_strips(DevSample* samples, int n, StripPlan& plan) {
   }
 }
 
+// Two CTAs for every one of a B200's 148 SMs (another count would only choose other cells).
+constexpr long long kWideWantCtas = 148 * 2;
+
 static void plan_wide(DevSample* samples, int n, int channels, WalkPlan& plan) {
-  // The largest cells that still give every one of a B200's 148 SMs two CTAs (another
-  // count would only choose other cells).
+  // The largest cells that still give every SM two CTAs.
   static const int kCells[][2] = {{kWalkMaxPx, 32}, {kWalkMaxPx, 16}, {kWalkMaxPx, 8}, {64, 8}, {64, 4}};
-  constexpr long long kWantCtas = 148 * 2;
   for (const auto& cell : kCells) {
     long long ctas = 0;
     plan = WalkPlan{0, 0, 0, 0, 0};
@@ -340,30 +341,130 @@ static void plan_wide(DevSample* samples, int n, int channels, WalkPlan& plan) {
         plan.steps = std::max(plan.steps, (int32_t)walk_steps(s, s.walk_rows));
       }
     }
-    if (ctas == 0 || ctas >= kWantCtas) {
+    if (ctas == 0 || ctas >= kWideWantCtas) {
       return;
     }
   }
 }
 
-void plan_resize(DevSample* samples, int n, int channels, ResizePlan& plan) {
-  // With four channels all units of a pixel column lie in one half of the banks, so that
-  // the columns of a shrink of two or three meet in one or two of eight places: 96 images
-  // to 224x224 take 133 us a pass in strips at 2:1 and 110 in resize_walk.cu, 178 and 148
-  // at 3:1 (78 and 83 at 1.6:1, and at 4:1, where that kernel's columns meet too, 27 and
-  // 35).  Decided for the batch: 128 images of 256-800 px, both kinds, take 160 us when
-  // either kernel gets its own, 150 in strips, 137 in resize_walk.cu.
-  int resizes = 0, meet = 0;
-  for (int i = 0; channels == 4 && i < n; i++) {
-    resizes += samples[i].mode == kModeResize;
-    meet += samples[i].mode == kModeResize && samples[i].axis_x[0] > 1.75f && samples[i].axis_x[0] < 3.5f;
-  }
-  for (int i = 0; 4 * meet > resizes && i < n; i++) {
-    DevSample& s = samples[i];
-    if (s.mode == kModeResize && walk_fits(s, channels)) {
-      s.mode = kModeResizeWide;
+// Chunks of resize_walk.cu across a resize, as split_walk() makes them but for a column
+// or two, and the warps of a chunk that have a word of its source rows.
+static int wide_chunks(const DevSample& s, int channels, int& warps) {
+  const float ratio = s.axis_x[0], reach = 2.0f * std::max(ratio, 1.0f);
+  const float columns = (float)((kWalkRow - 6) / channels - 2);
+  const int px = (int)std::max(1.0f, std::min((float)kWalkMaxPx, (columns - reach) / ratio + 1.0f));
+  const int chunks = (s.post_w + px - 1) / px;
+  const float width = (float)((s.post_w + chunks - 1) / chunks - 1) * ratio + reach + 1.0f;
+  warps = ((int)std::min((float)s.pre_w, width) * channels + 255) / 256;
+  return chunks;
+}
+
+// What a resize adds to a launch of either kernel, in picoseconds: per strip (chunk) and
+// stage of four output rows the steps down the source rows, then the passes of 32
+// columns (the warps of the chunk, which all wait for the busiest).  Fitted to 1376 uniform
+// batches of 1 to 1024 images, 0.2:1 to 8:1, 1 to 4 channels, both output types, timed in
+// both kernels: they hold to 12 % in the mean; the strips' are a tenth lower, since a batch
+// in doubt is theirs.  With four channels all units of a pixel column lie in one half of
+// the banks, where the columns of a shrink meet.
+static float strip_time(const DevSample& s, int channels) {
+  const float rx = s.axis_x[0], ry = std::max(s.axis_y[0], 1.5f);
+  const float pass = channels < 4 ? 180.0f + 65.0f * std::max(rx, 1.0f) : rx < 1.0f ? 400.0f : 640.0f + 110.0f * rx;
+  return (float)(s.walk_chunks * ((s.post_h + 3) / 4)) * (420.0f * ry + (float)((s.walk_px + 31) >> 5) * pass);
+}
+
+static float wide_time(const DevSample& s, int channels) {
+  int warps;
+  const int chunks = wide_chunks(s, channels, warps);
+  return (float)(chunks * ((s.post_h + 3) / 4)) * (760.0f * std::max(s.axis_y[0], 1.5f) + 1100.0f * (float)warps);
+}
+
+// A batch that resize_walk.cu has to run a part of: whether it should run all of it.  Two
+// kernels run one after the other and each leaves the GPU part empty at its end: two
+// launches took 1.13 times as long as one over 143 batches of shrinks by 1 to 12 (2 images
+// 24.3 us and 15.0, 262 images 499 and 407).  Two are better where one launch
+// - would be flooded: every sample gets as many cells as the largest, and an empty CTA takes
+//   0.8 ns (255 images of 256-500 px, one 20000x300, one 300x20000, to 224x224: 201 000 CTAs,
+//   387 us in one launch, 228 in two);
+// - would fill less than one round of CTAs with the longest walks, of 32 rows, while the
+//   strong shrinks by themselves are cut into short ones (plan_wide): 173 images shrunk by 1
+//   to 4 and three by more, to 41x41: 38.7 us in one, 31.0 in two; 17 to 231x231 49.7 and 41.5.
+static bool one_launch(const DevSample* samples, int n, int channels) {
+  float cells = 0.0f, most = 0.0f, strong = 0.0f;
+  int resizes = 0;
+  for (int i = 0; i < n; i++) {
+    const DevSample& s = samples[i];
+    if (s.mode == kModeResize || s.mode == kModeResizeWide) {
+      int warps;
+      const float rows = std::max(1.0f, std::min((float)kWalkMaxRows, (float)(kWalkMaxSteps / 4) / std::max(s.axis_y[0], 1.0f)));
+      const float chunks = (float)wide_chunks(s, channels, warps);
+      const float own = chunks * std::ceil((float)s.post_h / rows);
+      cells += own;
+      most = std::max(most, own);
+      strong += s.mode == kModeResizeWide ? chunks * std::ceil((float)s.post_h / std::min(rows, 16.0f)) : 0.0f;
+      resizes++;
     }
   }
+  const float grid = most * (float)resizes;
+  const bool flooded = grid > 4.0f * cells && grid > 32768.0f;
+  const bool part_filled = cells >= kWideWantCtas && cells < 2.2f * kWideWantCtas && strong < kWideWantCtas;
+  return !flooded && !part_filled;
+}
+
+// Which kernel runs a resize that both can, decided for the batch.  One with strong
+// shrinks: one_launch().  Any other goes where it takes less time, into strips when in
+// doubt: what small launches take beyond the sums is a few us less there.  Up to three
+// channels strips win by 1.0 to 2.5 where the image shrinks by less than three, so the
+// times are made up only when a quarter of a batch shrinks by more (512 images of 748x748x3
+// to 136x136: 564 us in strips, 386 in resize_walk.cu; 564 of 507x507x3 to 136x136, bytes,
+// 339 and 276).
+static void choose_resize_kernel(DevSample* samples, int n, int channels) {
+  int strips = 0, strong = 0, doubt = 0;
+  for (int i = 0; i < n; i++) {
+    const DevSample& s = samples[i];
+    const int can = s.mode == kModeResize;
+    strips += can;
+    doubt += can & ((channels == 4) | (s.axis_x[0] >= 3.0f) | (s.axis_y[0] >= 3.0f));
+    strong += s.mode == kModeResizeWide;
+  }
+  if (strips == 0 || (strong == 0 && 4 * doubt <= strips)) {
+    return;
+  }
+  if (strong > 0) {
+    if (!one_launch(samples, n, channels)) {
+      return;
+    }
+  } else {
+    constexpr float kInDoubt = 3e6f;
+    float in_strips = 0.0f, in_wide = 0.0f, strip = 0.0f, wide = 0.0f;
+    const DevSample* last = nullptr;
+    for (int i = 0; i < n; i++) {
+      DevSample& s = samples[i];
+      if (s.mode != kModeResize) {
+        continue;
+      }
+      if (!last || s.post_w != last->post_w || s.post_h != last->post_h || s.axis_x[0] != last->axis_x[0] ||
+          s.axis_y[0] != last->axis_y[0] || s.pre_w != last->pre_w) {
+        split_strips(s);
+        strip = strip_time(s, channels);
+        wide = wide_time(s, channels);
+        last = &s;
+      }
+      in_strips += strip;
+      in_wide += wide;
+    }
+    if (in_strips < in_wide + kInDoubt) {
+      return;
+    }
+  }
+  for (int i = 0; i < n; i++) {
+    if (samples[i].mode == kModeResize && walk_fits(samples[i], channels)) {
+      samples[i].mode = kModeResizeWide;
+    }
+  }
+}
+
+void plan_resize(DevSample* samples, int n, int channels, ResizePlan& plan) {
+  choose_resize_kernel(samples, n, channels);
   plan_strips(samples, n, plan.strip);
   plan_wide(samples, n, channels, plan.wide);
 }

@@ -1,6 +1,6 @@
-// The resize kernel of strong shrinks (kModeResizeWide): one CTA of kWalkThreads walks down one chunk of output
-// columns (walk_px of them at most) of one sample, walk_rows output rows, in
-// stages of four rows.
+// The resize kernel of strong shrinks and of the batches with them (kModeResizeWide): one
+// CTA of kWalkThreads walks down one chunk of output columns (walk_px of them at most) of
+// one sample, walk_rows output rows, in stages of four rows.
 //
 // Vertical half of a stage.  A thread owns two 32-bit words of the chunk's
 // source bytes (eight byte columns) and walks down the source rows.  Each warp
