@@ -68,7 +68,7 @@ enum mlxd_mem { MLXD_MEM_HOST = 0, MLXD_MEM_DEVICE = 1 };
  * caller opted in; at this level the caller is expected to know.
  */
 typedef struct mlxd_sample_desc {
-  const uint8_t* src; /* [src_h, src_w, C] */
+  const uint8_t* src; /* [src_h, src_w, C]; device memory is read in the aligned 16-byte units that hold its bytes */
   int32_t src_h, src_w;
   int32_t pre_x, pre_y, pre_w, pre_h;
   int32_t pre_flip;

@@ -1,14 +1,14 @@
-// The kernels around the resize kernel (resize_walk.cu): copy (crop / flip /
+// The kernels around the resize kernels (resize_strip.cu, resize_walk.cu): copy (crop / flip /
 // batch only) and nearest-neighbour affine bands, padding of ragged batches,
-// and resizes whose taps fit no chunk of the resize kernel.
+// and resizes whose taps fit no chunk of resize_walk.cu.
 //
 // Copy and affine: one CTA per band of up to eight kTileH x kTileW tiles of one
 // sample's slot; the source is read through the read-only path, four pixels per
 // thread, and stored 16 bytes at a time; pad-only bands are plain 16-byte
 // stores.  The rows below a sample in a ragged batch go out through a linear fill
-// kernel when the launch has no resize (else CTAs of the resize kernel write them).
-// A resize too strong for the resize kernel is filtered pixel by
-// pixel from global memory by a kernel of its own.
+// kernel when the launch has no resize (else CTAs of a resize kernel write them).
+// A resize too strong for both resize kernels is filtered pixel by pixel from
+// global memory by a kernel of its own.
 #include "fused_batch.h"
 #include "kernel_common.cuh"
 
@@ -341,14 +341,14 @@ __global__ void __launch_bounds__(kThreads, 3) fused_fast_gray_kernel(const Laun
 
 } // namespace
 
-// ---- resizes whose taps do not fit a chunk of the resize kernel ------------------------
+// ---- resizes whose taps do not fit a chunk of resize_walk.cu ------------------------------
 //
 // One thread per pixel of the post window, every tap read from global memory.
-// The arithmetic is that of the resize kernel, value by value: per source column
+// The arithmetic is that of the resize kernels, value by value: per source column
 // the vertical sum (multiply-adds in tap order, the first of them a product, taps
 // outside the window reading the clamped row), then the horizontal multiply-adds
 // over those sums in tap order onto zero, weights tent / sum with the sum taken in
-// tap order.  Such samples are rare and small on the output side (walk_fits: shrink
+// tap order.  Such samples are rare and small on the output side (launch_plan.cu: walk_fits: shrink
 // ratios above 100 along a row, 500 down the rows), so nothing is staged or shared.
 template <int C>
 __device__ void direct_pixel(const DevSample& s, const LaunchParams& p, int ox, int oy) {

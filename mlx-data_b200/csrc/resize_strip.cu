@@ -34,7 +34,8 @@
 // for two rows about two a row; a unit of four rows halves the loads of the taps, and
 // dealing columns to lanes by bank takes most of their conflicts; a CTA-wide walk meets
 // two barriers a stage and leaves warps idle where a chunk's words are no multiple of its
-// 128 lanes.  Five CTAs per SM at 96 registers: six spill (1.55 ms), four wait (1.36).
+// 128 lanes.  Five CTAs per SM at 96 registers, for which most instances of one to three
+// channels spill 4 to 8 bytes; six spill the walk (1.55 ms), four wait (1.36).
 // The tables of a CTA took a fifth of the time before the taps of a pass were shared by
 // its warps, the steps dealt flat over the lanes and the axes' ratios divided on the
 // host (1.25 ms).
