@@ -103,3 +103,33 @@ def test_walk_beyond_its_plan_on_a_stream(pkg, ctx, oracle):
     assert ctx.stream_status(stream) == 0
     want = oracle.resize(img, 48, 40).astype(np.float32) / np.float32(255)
     assert np.array_equal(out[0, :40, :48].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("h", [200, 1600], ids=["resize_strip", "resize_walk"])
+@pytest.mark.parametrize("c", [1, 3, 4])
+def test_walk_beyond_its_plan_of_either_kernel(pkg, ctx, oracle, h, c):
+    """A shrink by 5 down the rows of two images runs in strips, one by 40 in the kernel of strong
+    shrinks: each refuses and recovers."""
+    torch = pytest.importorskip("torch")
+    capi = pkg._capi
+    stream = torch.cuda.current_stream().cuda_stream
+    imgs = [np.random.default_rng(k).integers(0, 256, (h, 90, c), dtype=np.uint8) for k in range(2)]
+    src = [torch.from_numpy(a).cuda() for a in imgs]
+    descs = np.zeros(2, pkg.SAMPLE_DTYPE)
+    for i, (a, t) in enumerate(zip(imgs, src)):
+        chain.fill_descs(descs, i, chain.reduce_chain(a.shape, OPS), t.data_ptr())
+    out = torch.full((2, 40, 300, c), -1.0, device="cuda")
+    bd = pkg.make_batch_desc(out.data_ptr(), 40, 300, c, pad_value=255.0, src_mem=capi.MEM_DEVICE, dst_mem=capi.MEM_DEVICE)
+    os.environ["MLXD_TEST_SHORT_PLAN"] = "1"
+    try:
+        ctx.fused_batch_on_stream(stream, descs, bd)
+    finally:
+        os.environ.pop("MLXD_TEST_SHORT_PLAN", None)
+    assert ctx.stream_status(stream) == 8
+    got = out.cpu().numpy()
+    assert (got[:, :, :48] == -1).all() and (got[:, :, 48:] == 1).all()
+    ctx.fused_batch_on_stream(stream, descs, bd)
+    assert ctx.stream_status(stream) == 0
+    for i, a in enumerate(imgs):
+        want = oracle.resize(a, 48, 40).astype(np.float32) / np.float32(255)
+        assert np.array_equal(out[i, :, :48].cpu().numpy(), want)
