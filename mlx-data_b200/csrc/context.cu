@@ -148,7 +148,7 @@ int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, 
     if (rc != MLXD_OK) {
       return rc;
     }
-    DevSample s;
+    DevSample& s = out;
     std::memset(&s, 0, sizeof(s));
     s.src = d.src;
     s.src_h = d.src_h;
@@ -197,7 +197,6 @@ int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, 
       s.post_flip ^= 1;
       s.post_x = s.geom_w - s.post_x - s.post_w;
     }
-    out = s;
   }
   return MLXD_OK;
 }
@@ -230,22 +229,35 @@ int plan_samples(
   return rc;
 }
 
+// floor() and ceil() without a library call.
+static int64_t floor_to(double x) {
+  const int64_t t = (int64_t)x;
+  return t - (x < (double)t);
+}
+
+static int64_t ceil_to(double x) {
+  const int64_t t = (int64_t)x;
+  return t + (x > (double)t);
+}
+
 // Source samples of an n_src -> n_dst axis that outputs [o_lo, o_hi) can read,
 // widened by `margin` on both sides (none: the exact span, for statistics) and clipped
 // to the axis.
 static void axis_span(int64_t n_src, int64_t n_dst, int64_t o_lo, int64_t o_hi, int margin, int64_t& lo, int64_t& hi) {
+  if (o_lo == 0 && o_hi == n_dst) {
+    lo = 0;   // the first and the last output reach beyond the axis
+    hi = n_src;
+    return;
+  }
   if (n_src == n_dst) {
     lo = o_lo;
     hi = o_hi;
   } else {
     const double ratio = (double)n_src / (double)n_dst;
     const double radius = ratio > 1.0 ? ratio : 1.0;
-    lo = (int64_t)std::floor((o_lo + 0.5) * ratio - 0.5 - radius) - margin;
-    hi = (int64_t)std::ceil((o_hi - 0.5) * ratio - 0.5 + radius) + 1 + margin;
-    if (margin > 0) {
-      lo -= axis_slack((int32_t)n_src);
-      hi += axis_slack((int32_t)n_src);
-    }
+    const int around = margin > 0 ? margin + axis_slack((int32_t)n_src) : 0;
+    lo = floor_to((o_lo + 0.5) * ratio - 0.5 - radius) - around;
+    hi = ceil_to((o_hi - 0.5) * ratio - 0.5 + radius) + 1 + around;
   }
   lo = std::max<int64_t>(lo, 0);
   hi = std::min<int64_t>(hi, n_src);

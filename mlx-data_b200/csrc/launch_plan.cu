@@ -239,6 +239,10 @@ static void split_walk(DevSample& s, int channels, int px, int rows) {
 
 static void plan_strips(DevSample* samples, int n, StripPlan& plan) {
   constexpr int kWarps = kStripThreads / 32;
+  // (An unlike batch, whose samples have their largest needs in different places, can take
+  // more than the 45.6 KB a CTA that five an SM leave: 256 of 256-800 px to 224x224 take 51,
+  // of which four fit.  Planned for four places they take as long, 117.1 us and 117.0, with
+  // walks cut until five fit 138.8.)
   constexpr float kWarpsAtOnce = 148 * kStripCtas * kWarps;
   plan = StripPlan{};
   double total = 0.0;
@@ -390,18 +394,20 @@ static float wide_time(const DevSample& s, int channels) {
 //   to 4 and three by more, to 41x41: 38.7 us in one, 31.0 in two; 17 to 231x231 49.7 and 41.5.
 static bool one_launch(const DevSample* samples, int n, int channels) {
   float cells = 0.0f, most = 0.0f, strong = 0.0f;
-  int resizes = 0;
+  int resizes = 0, light = 0;
+  const int stride = std::max(1, n / 32);
   for (int i = 0; i < n; i++) {
     const DevSample& s = samples[i];
-    if (s.mode == kModeResize || s.mode == kModeResizeWide) {
+    const bool is_strong = s.mode == kModeResizeWide;
+    resizes += is_strong || s.mode == kModeResize;
+    if (is_strong || (s.mode == kModeResize && light++ % stride == 0)) {   // the light ones are counted from a few
       int warps;
       const float rows = std::max(1.0f, std::min((float)kWalkMaxRows, (float)(kWalkMaxSteps / 4) / std::max(s.axis_y[0], 1.0f)));
       const float chunks = (float)wide_chunks(s, channels, warps);
       const float own = chunks * std::ceil((float)s.post_h / rows);
-      cells += own;
+      cells += is_strong ? own : own * (float)stride;
       most = std::max(most, own);
-      strong += s.mode == kModeResizeWide ? chunks * std::ceil((float)s.post_h / std::min(rows, 16.0f)) : 0.0f;
-      resizes++;
+      strong += is_strong ? chunks * std::ceil((float)s.post_h / std::min(rows, 16.0f)) : 0.0f;
     }
   }
   const float grid = most * (float)resizes;
@@ -413,17 +419,19 @@ static bool one_launch(const DevSample* samples, int n, int channels) {
 // Which kernel runs a resize that both can, decided for the batch.  One with strong
 // shrinks: one_launch().  Any other goes where it takes less time, into strips when in
 // doubt: what small launches take beyond the sums is a few us less there.  Up to three
-// channels strips win by 1.0 to 2.5 where the image shrinks by less than three, so the
-// times are made up only when a quarter of a batch shrinks by more (512 images of 748x748x3
-// to 136x136: 564 us in strips, 386 in resize_walk.cu; 564 of 507x507x3 to 136x136, bytes,
-// 339 and 276).
+// channels strips win by 1.0 to 2.5 where the image shrinks by less than three, with four
+// where it is enlarged by 1.3 at least, so the times are made up only when a quarter of a
+// batch is beyond that, and for 32 to 63 of its samples (512 images of 748x748x3 to
+// 136x136: 564 us in strips, 386 in resize_walk.cu; 564 of 507x507x3 to 136x136, bytes, 339
+// and 276).
 static void choose_resize_kernel(DevSample* samples, int n, int channels) {
   int strips = 0, strong = 0, doubt = 0;
+  const float edge = channels == 4 ? 0.75f : 3.0f;
   for (int i = 0; i < n; i++) {
     const DevSample& s = samples[i];
     const int can = s.mode == kModeResize;
     strips += can;
-    doubt += can & ((channels == 4) | (s.axis_x[0] >= 3.0f) | (s.axis_y[0] >= 3.0f));
+    doubt += can & ((s.axis_x[0] >= edge) | (s.axis_y[0] >= 3.0f));
     strong += s.mode == kModeResizeWide;
   }
   if (strips == 0 || (strong == 0 && 4 * doubt <= strips)) {
@@ -437,7 +445,8 @@ static void choose_resize_kernel(DevSample* samples, int n, int channels) {
     constexpr float kInDoubt = 3e6f;
     float in_strips = 0.0f, in_wide = 0.0f, strip = 0.0f, wide = 0.0f;
     const DevSample* last = nullptr;
-    for (int i = 0; i < n; i++) {
+    const int stride = std::max(1, n / 32);
+    for (int i = 0; i < n; i += stride) {
       DevSample& s = samples[i];
       if (s.mode != kModeResize) {
         continue;
@@ -452,7 +461,7 @@ static void choose_resize_kernel(DevSample* samples, int n, int channels) {
       in_strips += strip;
       in_wide += wide;
     }
-    if (in_strips < in_wide + kInDoubt) {
+    if (in_strips < in_wide + kInDoubt / (float)stride) {
       return;
     }
   }
