@@ -382,6 +382,13 @@ static float wide_time(const DevSample& s, int channels) {
   return (float)(chunks * ((s.post_h + 3) / 4)) * (760.0f * std::max(s.axis_y[0], 1.5f) + 1100.0f * (float)warps);
 }
 
+// Cells of a resize with walks of at most `most` rows.
+static float wide_cells(const DevSample& s, int channels, float most) {
+  int warps;
+  const float rows = std::max(1.0f, std::min(most, (float)(kWalkMaxSteps / 4) / std::max(s.axis_y[0], 1.0f)));
+  return (float)wide_chunks(s, channels, warps) * std::ceil((float)s.post_h / rows);
+}
+
 // A batch that resize_walk.cu has to run a part of: whether it should run all of it.  Two
 // kernels run one after the other and each leaves the GPU part empty at its end: two
 // launches took 1.13 times as long as one over 143 batches of shrinks by 1 to 12 (2 images
@@ -401,13 +408,10 @@ static bool one_launch(const DevSample* samples, int n, int channels) {
     const bool is_strong = s.mode == kModeResizeWide;
     resizes += is_strong || s.mode == kModeResize;
     if (is_strong || (s.mode == kModeResize && light++ % stride == 0)) {   // the light ones are counted from a few
-      int warps;
-      const float rows = std::max(1.0f, std::min((float)kWalkMaxRows, (float)(kWalkMaxSteps / 4) / std::max(s.axis_y[0], 1.0f)));
-      const float chunks = (float)wide_chunks(s, channels, warps);
-      const float own = chunks * std::ceil((float)s.post_h / rows);
+      const float own = wide_cells(s, channels, kWalkMaxRows);
       cells += is_strong ? own : own * (float)stride;
       most = std::max(most, own);
-      strong += is_strong ? chunks * std::ceil((float)s.post_h / std::min(rows, 16.0f)) : 0.0f;
+      strong += is_strong ? wide_cells(s, channels, 16.0f) : 0.0f;
     }
   }
   const float grid = most * (float)resizes;
@@ -418,12 +422,14 @@ static bool one_launch(const DevSample* samples, int n, int channels) {
 
 // Which kernel runs a resize that both can, decided for the batch.  One with strong
 // shrinks: one_launch().  Any other goes where it takes less time, into strips when in
-// doubt: what small launches take beyond the sums is a few us less there.  Up to three
-// channels strips win by 1.0 to 2.5 where the image shrinks by less than three, with four
-// where it is enlarged by 1.3 at least, so the times are made up only when a quarter of a
-// batch is beyond that, and for 32 to 63 of its samples (512 images of 748x748x3 to
-// 136x136: 564 us in strips, 386 in resize_walk.cu; 564 of 507x507x3 to 136x136, bytes, 339
-// and 276).
+// doubt: what a small launch takes beyond the sums is a few us less there, and with cells
+// for less than 1.3 rounds of CTAs resize_walk.cu is the slower one whatever the sums say
+// (53 batches: 1.1 to 1.27 times as long; 8 images shrunk by 3 to 6 to 288x288: 42.2 us and
+// 33.6).  Up to three channels strips win by 1.0 to 2.5 where the image shrinks by less than
+// three, with four where it is enlarged by 1.3 at least, so the times are made up only when
+// a quarter of a batch is beyond that, and for 32 to 63 of its samples (512 images of
+// 748x748x3 to 136x136: 564 us in strips, 386 in resize_walk.cu; 564 of 507x507x3 to
+// 136x136, bytes, 339 and 276).
 static void choose_resize_kernel(DevSample* samples, int n, int channels) {
   int strips = 0, strong = 0, doubt = 0;
   const float edge = channels == 4 ? 0.75f : 3.0f;
@@ -443,7 +449,7 @@ static void choose_resize_kernel(DevSample* samples, int n, int channels) {
     }
   } else {
     constexpr float kInDoubt = 3e6f;
-    float in_strips = 0.0f, in_wide = 0.0f, strip = 0.0f, wide = 0.0f;
+    float in_strips = 0.0f, in_wide = 0.0f, cells = 0.0f, strip = 0.0f, wide = 0.0f, own = 0.0f;
     const DevSample* last = nullptr;
     const int stride = std::max(1, n / 32);
     for (int i = 0; i < n; i += stride) {
@@ -456,12 +462,14 @@ static void choose_resize_kernel(DevSample* samples, int n, int channels) {
         split_strips(s);
         strip = strip_time(s, channels);
         wide = wide_time(s, channels);
+        own = wide_cells(s, channels, kWalkMaxRows);
         last = &s;
       }
       in_strips += strip;
       in_wide += wide;
+      cells += own;
     }
-    if (in_strips < in_wide + kInDoubt / (float)stride) {
+    if (in_strips < in_wide + kInDoubt / (float)stride || cells * (float)stride < 4 * kWideWantCtas) {
       return;
     }
   }

@@ -36,6 +36,13 @@ def test_two_launches_of_ragged_slots(pkg, ctx, oracle):
     _check(pkg, ctx, oracle, light[:3] + [(4800, 4800)] + light[3:], 1, ops, seed=0)
 
 
+# enough cells for the kernel of strong shrinks to be the faster one of two that can run them (two channels: the strips)
+@pytest.mark.parametrize("c,side", [(1, 470), (2, 520), (3, 500), (4, 340)])
+def test_large_batch_of_strong_shrinks(pkg, ctx, oracle, c, side):
+    ops = [("image_random_h_flip", dict(key="image", prob=0.5)), ("image_resize", dict(key="image", w=100, h=98))]
+    _check(pkg, ctx, oracle, [(side + i % 5, side - i % 7) for i in range(320)], c, ops, seed=c)
+
+
 # either side of the lines (three to one, 13 / 3 down the rows, four channels), batches of a few images and of many
 @pytest.mark.parametrize("c", [1, 2, 3, 4])
 @pytest.mark.parametrize("n", [2, 40])
