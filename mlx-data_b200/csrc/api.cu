@@ -325,14 +325,12 @@ int mlxd_fused_batch_on_stream(
   if (rc != MLXD_OK) {
     return rc;
   }
-  // A table of at most 32 KB is taken from ordinary memory: the driver copies it into
+  // A table of at most 64 KB is taken from ordinary memory: the driver copies it into
   // the command stream before the call returns, which costs a pass 2 us where a copy
   // from page-locked memory, started by a copy engine, costs 6 (32 to 240 samples
-  // ahead of a kernel of 20 us).  Writing the command stream is slow for the host, though:
-  // a batch of tiny images, which the host's work bounds, takes 18.4 us a pass with 256
-  // samples (17.7 by the copy engine), 23.0 with 384 (21.5), 27.5 with 512 (25.2).
+  // ahead of a kernel of 20 us).
   const void* table = dev.data();
-  if (table_bytes > 32 * 1024) {
+  if (table_bytes > 64 * 1024) {
     rc = arena_reserve(ctx, ring.h_desc[slot], table_bytes, true, nullptr);
     if (rc != MLXD_OK) {
       return rc;
