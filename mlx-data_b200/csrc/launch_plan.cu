@@ -421,23 +421,27 @@ static bool one_launch(const DevSample* samples, int n, int channels) {
 }
 
 // Which kernel runs a resize that both can, decided for the batch.  One with strong
-// shrinks: one_launch().  Any other goes where it takes less time, into strips when in
-// doubt: what a small launch takes beyond the sums is a few us less there, and with cells
-// for less than 1.3 rounds of CTAs resize_walk.cu is the slower one whatever the sums say
-// (53 batches: 1.1 to 1.27 times as long; 8 images shrunk by 3 to 6 to 288x288: 42.2 us and
-// 33.6).  Up to three channels strips win by 1.0 to 2.5 where the image shrinks by less than
-// three, with four where it is enlarged by 1.3 at least, so the times are made up only when
-// a quarter of a batch is beyond that, and for 32 to 63 of its samples (512 images of
-// 748x748x3 to 136x136: 564 us in strips, 386 in resize_walk.cu; 564 of 507x507x3 to
-// 136x136, bytes, 339 and 276).
+// shrinks: one_launch().  With four channels the columns of a shrink by two or three meet in
+// one or two of the banks' eight places: a batch with a quarter of those is resize_walk.cu's
+// (96 images to 224x224 133 us in strips at 2:1 and 110 there, 178 and 148 at 3:1).  Any
+// other goes where it takes less time, into strips when in doubt: what a small launch takes
+// beyond the sums is a few us less there, and with cells for less than one round of CTAs
+// resize_walk.cu is the slower one although the sums are equal (53 batches: 1.1 to 1.27
+// times as long; 8 images shrunk by 3 to 6 to 288x288: 42.2 us and 33.6).  Up to three
+// channels strips win by 1.0 to 2.5 where the image shrinks by less than three, with four
+// where it is enlarged by 1.3 at least, so the times are made up only when a quarter of a
+// batch is beyond that, and for 32 to 63 of its samples (512 images of 748x748x3 to
+// 136x136: 564 us in strips, 386 in resize_walk.cu; 564 of 507x507x3 to 136x136, bytes, 339
+// and 276).
 static void choose_resize_kernel(DevSample* samples, int n, int channels) {
-  int strips = 0, strong = 0, doubt = 0;
+  int strips = 0, strong = 0, doubt = 0, meet = 0;
   const float edge = channels == 4 ? 0.75f : 3.0f;
   for (int i = 0; i < n; i++) {
     const DevSample& s = samples[i];
     const int can = s.mode == kModeResize;
     strips += can;
     doubt += can & ((s.axis_x[0] >= edge) | (s.axis_y[0] >= 3.0f));
+    meet += can & (s.axis_x[0] > 1.75f) & (s.axis_x[0] < 3.5f);
     strong += s.mode == kModeResizeWide;
   }
   if (strips == 0 || (strong == 0 && 4 * doubt <= strips)) {
@@ -447,7 +451,7 @@ static void choose_resize_kernel(DevSample* samples, int n, int channels) {
     if (!one_launch(samples, n, channels)) {
       return;
     }
-  } else {
+  } else if (channels < 4 || 4 * meet <= strips) {
     constexpr float kInDoubt = 3e6f;
     float in_strips = 0.0f, in_wide = 0.0f, cells = 0.0f, strip = 0.0f, wide = 0.0f, own = 0.0f;
     const DevSample* last = nullptr;
@@ -469,7 +473,8 @@ static void choose_resize_kernel(DevSample* samples, int n, int channels) {
       in_wide += wide;
       cells += own;
     }
-    if (in_strips < in_wide + kInDoubt / (float)stride || cells * (float)stride < 4 * kWideWantCtas) {
+    const bool few = cells * (float)stride < 3 * kWideWantCtas;   // six CTAs an SM
+    if (few || in_strips < in_wide + kInDoubt / (float)stride) {
       return;
     }
   }
