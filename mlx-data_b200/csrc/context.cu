@@ -202,13 +202,18 @@ int plan_one_sample(const mlxd_sample_desc& d, int i, const mlxd_batch_desc* b, 
 }
 
 int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, DevSample* out, ResizePlan& plan) {
+  bool resizes = false;
   for (int i = 0; i < n; i++) {
     const int rc = plan_one_sample(samples[i], i, b, i > 0 ? &out[i - 1] : nullptr, out[i]);
     if (rc != MLXD_OK) {
       return rc;
     }
+    resizes |= is_resize(out[i]);
   }
-  plan_resize(out, n, b->channels, plan);
+  plan = ResizePlan{};
+  if (resizes) {
+    plan_resize(out, n, b->channels, plan);
+  }
   return MLXD_OK;
 }
 
