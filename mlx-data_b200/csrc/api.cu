@@ -160,7 +160,7 @@ void mlxd_ctx_destroy(mlxd_ctx* ctx) {
     destroy_lane(l);
   }
   for (auto& kv : ctx->luts) {
-    cudaFree(kv.second);
+    cudaFree(kv.second.values);
   }
   if (ctx->d_status) {
     cudaFree(ctx->d_status);

@@ -306,6 +306,44 @@ void compute_cast_table(const mlxd_batch_desc* b, int c_out, float* table) {
   }
 }
 
+// A division of a float x by a float d, correctly rounded, is fma(x, hi, x * lo) with
+// hi + lo = 1 / d to 48 bits, unless the quotient lies within 2^-48 of the middle between
+// two floats: so every value is compared with the table's, and a cast with one that differs
+// (or with infinities) keeps the table.  The channel reduction's casts do too: their values
+// are whole numbers, which index it as they are.
+void cast_steps(const mlxd_batch_desc* b, int c_out, const float* table, CastSteps& steps) {
+  std::memset(&steps, 0, sizeof(steps));
+  if (b->gray) {
+    return;
+  }
+  auto reciprocal = [](float d, float (&hi)[2], float (&lo)[2]) {
+    const double r = 1.0 / (double)d;
+    hi[0] = hi[1] = (float)r;
+    lo[0] = lo[1] = (float)(r - (double)hi[0]);
+  };
+  reciprocal(b->divisor, steps.r_hi, steps.r_lo);
+  for (int c = 0; c < c_out && b->normalise; c++) {
+    steps.neg_mean[c][0] = steps.neg_mean[c][1] = -b->mean[c];
+    reciprocal(b->std_[c], steps.s_hi[c], steps.s_lo[c]);
+  }
+  for (int c = 0; c < c_out; c++) {
+    for (int v = 0; v < 256; v++) {
+      const volatile float x = (float)v;
+      const volatile float low = x * steps.r_lo[0];
+      float y = std::fma((float)x, steps.r_hi[0], (float)low);
+      if (b->normalise) {
+        const volatile float t = y + steps.neg_mean[c][0];
+        const volatile float t_low = t * steps.s_lo[c][0];
+        y = std::fma((float)t, steps.s_hi[c][0], (float)t_low);
+      }
+      if (std::memcmp(&y, &table[(size_t)c * 256 + v], sizeof(y)) != 0) {
+        return;
+      }
+    }
+  }
+  steps.mode = b->normalise ? kCastNormalise : kCastScale;
+}
+
 LutUse::LutUse(mlxd_ctx* ctx) {
   bool full;
   {
@@ -319,7 +357,7 @@ LutUse::LutUse(mlxd_ctx* ctx) {
       DeviceGuard on_device(ctx->device);
       cudaDeviceSynchronize();
       for (auto& kv : ctx->luts) {
-        cudaFree(kv.second);
+        cudaFree(kv.second.values);
       }
       ctx->luts.clear();
     }
@@ -327,11 +365,12 @@ LutUse::LutUse(mlxd_ctx* ctx) {
   hold_ = std::shared_lock<std::shared_mutex>(ctx->lut_users);
 }
 
-int get_lut(mlxd_ctx* ctx, const mlxd_batch_desc* b, int c_out, const float** lut) {
+int get_lut(mlxd_ctx* ctx, const mlxd_batch_desc* b, int c_out, CastTable& out) {
   LutKey key;
   std::memset(&key, 0, sizeof(key));
   key.c_out = c_out;
   key.normalise = b->normalise ? 1 : 0;
+  key.gray = b->gray ? 1 : 0;
   std::memcpy(&key.divisor_bits, &b->divisor, 4);
   if (key.normalise) {
     std::memcpy(key.mean_bits, b->mean, 4 * c_out);
@@ -340,7 +379,7 @@ int get_lut(mlxd_ctx* ctx, const mlxd_batch_desc* b, int c_out, const float** lu
   std::lock_guard<std::mutex> g(ctx->lut_mu);
   auto it = ctx->luts.find(key);
   if (it != ctx->luts.end()) {
-    *lut = it->second;
+    out = it->second;
     return MLXD_OK;
   }
   std::vector<float> table((size_t)c_out * 256);
@@ -352,8 +391,9 @@ int get_lut(mlxd_ctx* ctx, const mlxd_batch_desc* b, int c_out, const float** lu
     cudaFree(d);
     return fail_cuda(e, "cudaMemcpy(cast table)");
   }
-  ctx->luts[key] = d;
-  *lut = d;
+  out.values = d;
+  cast_steps(b, c_out, table.data(), out.steps);
+  ctx->luts[key] = out;
   return MLXD_OK;
 }
 
@@ -394,7 +434,11 @@ int prepare_launch(mlxd_ctx* ctx, const mlxd_batch_desc* b, int n, LaunchParams&
   if (rc != MLXD_OK || !p.out_f32) {
     return rc;
   }
-  return get_lut(ctx, b, p.c_out, &p.lut);
+  CastTable cast;
+  const int got = get_lut(ctx, b, p.c_out, cast);
+  p.lut = cast.values;
+  p.cast = cast.steps;
+  return got;
 }
 
 // Threads that pack one batch's pageable sources (the caller included):

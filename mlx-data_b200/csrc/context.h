@@ -91,10 +91,17 @@ struct Lane {
 
 struct LutKey {
   int32_t c_out, normalise;
+  int32_t gray;   // (such a cast has no steps)
   uint32_t divisor_bits;
   uint32_t mean_bits[4];
   uint32_t std_bits[4];
   bool operator<(const LutKey& o) const;
+};
+
+// A cast on the device and as steps.
+struct CastTable {
+  float* values = nullptr;
+  CastSteps steps{};
 };
 
 } // namespace mlxd
@@ -105,7 +112,7 @@ struct mlxd_ctx {
   int n_user_lanes = 0;
   int32_t* d_status = nullptr;        // one self-check word per lane, 64 bytes apart
   std::mutex lut_mu;
-  std::map<mlxd::LutKey, float*> luts;   // at most mlxd::kMaxCastTables entries, see LutUse
+  std::map<mlxd::LutKey, mlxd::CastTable> luts;   // at most mlxd::kMaxCastTables entries, see LutUse
   std::shared_mutex lut_users;           // shared: a launch being prepared holds a table pointer; exclusive: emptying the cache
   std::atomic<uint64_t> batches{0}, samples{0}, launches{0}, h2d{0}, d2h{0}, reserved{0};
   std::atomic<uint64_t> kernel_ns{0}, timed_launches{0};
@@ -152,6 +159,9 @@ int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, 
 // The cast table of a batch descriptor: table[c * 256 + v], c < c_out.
 void compute_cast_table(const mlxd_batch_desc* b, int c_out, float* table);
 
+// The same cast as steps, where they give every value of the table (else kCastTable).
+void cast_steps(const mlxd_batch_desc* b, int c_out, const float* table, CastSteps& steps);
+
 // Launch-wide parameters from a batch descriptor, without the cast table, and with it.
 int describe_launch(const mlxd_batch_desc* b, int n, LaunchParams& p);
 int prepare_launch(mlxd_ctx* ctx, const mlxd_batch_desc* b, int n, LaunchParams& p);
@@ -162,7 +172,7 @@ int capture_batch(
     LaunchParams& p, const ResizePlan& plan, const DevSample* samples, const mlxd_batch_desc* batch, cudaStream_t stream);
 
 // Device cast table for a batch descriptor (cached per context).
-int get_lut(mlxd_ctx* ctx, const mlxd_batch_desc* b, int c_out, const float** lut);
+int get_lut(mlxd_ctx* ctx, const mlxd_batch_desc* b, int c_out, CastTable& table);
 
 // The cache of cast tables is bounded: a caller that changes mean/std on every
 // call would otherwise grow it for ever.  Every entry point that prepares a

@@ -107,6 +107,7 @@ struct ResizePlan {
   StripPlan strip;
   WalkPlan wide;
   int32_t first_wide, wides;   // all of them are among these samples
+  bool enlarges;      // most resizes enlarge along the row
 };
 
 __host__ __device__ inline bool is_resize(const DevSample& s) {
@@ -117,6 +118,16 @@ __host__ __device__ inline bool is_resize(const DevSample& s) {
 __host__ __device__ inline int walk_strips(const DevSample& s) {
   return (s.slot_w - s.post_w + kWalkPadPx - 1) / kWalkPadPx;
 }
+
+// The cast of a float32 batch as steps that give the table's values bit for bit (context.cu:
+// cast_steps): x = v * r, then for kCastNormalise (x + neg_mean) * s, each factor a sum of two
+// floats, every float twice as an operand of the packed instructions.
+enum CastMode : int32_t { kCastTable = 0, kCastScale = 1, kCastNormalise = 2 };
+struct CastSteps {
+  float r_hi[2], r_lo[2];
+  float neg_mean[4][2], s_hi[4][2], s_lo[4][2];
+  int32_t mode;   // kCastTable: no such steps, or the channel reduction's
+};
 
 struct LaunchParams {
   const DevSample* samples;
@@ -129,6 +140,7 @@ struct LaunchParams {
   int32_t gray_bias;
   int32_t out_f32;
   const float* lut;           // [c_out][256] cast table, device
+  CastSteps cast;
   int32_t pad_px;             // pad value as a pixel
   int32_t* status;            // device word, non-zero once a self-check failed
   int32_t band_tiles;         // band kernel: tiles per CTA along a row band (set at launch)
@@ -139,6 +151,11 @@ struct LaunchParams {
   int32_t fill_every;         // resize kernels, then: every so many CTAs, from the first on, one of them fills
   int32_t direct;             // some sample is kModeResizeDirect: resize_direct_kernel runs last
 };
+
+// Channels of cast tables that a resize kernel keeps in shared memory.
+__host__ __device__ inline int table_channels(const LaunchParams& p) {
+  return p.out_f32 && p.cast.mode == kCastTable ? p.c_out : 0;
+}
 
 // Launch the kernels the parameters call for: the resize kernel or, without a
 // resize and when p.pad_apart is set, pad_fill_kernel, the band kernel, resize_direct_kernel.

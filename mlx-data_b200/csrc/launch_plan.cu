@@ -59,9 +59,12 @@ void choose_kernels(LaunchParams& p, ResizePlan& plan, const DevSample* host_sam
   p.pad_apart = n > 0 && below * 8 >= rows ? 1 : 0;
   Cells strip, wide;
   plan.first_wide = plan.wides = 0;
+  int enlarged = 0, resized = 0;
   for (int i = 0; i < n; i++) {
     const DevSample& s = host_samples[i];
     const int h = p.pad_apart ? s.post_h : s.slot_h;
+    resized += is_resize(s);
+    enlarged += is_resize(s) && s.pre_w < s.geom_w;
     if (s.mode == kModeResize) {
       const int cell_rows = s.walk_rows * (kStripThreads / 32);
       strip.add((h + cell_rows - 1) / cell_rows, s.walk_chunks + walk_strips(s));
@@ -73,6 +76,7 @@ void choose_kernels(LaunchParams& p, ResizePlan& plan, const DevSample* host_sam
   }
   strip.put(plan.strip.cells_y, plan.strip.cells_x);
   wide.put(plan.wide.cells_y, plan.wide.cells_x);
+  plan.enlarges = 2 * enlarged > resized;
   p.walk = plan.wide;
 }
 

@@ -56,7 +56,7 @@ constexpr float kScaleY = 0x1p127f, kScaleX = 0x1p22f;
 struct StripSmem {
   unsigned mid;      // per warp: float4 [256]
   unsigned ring;     // per warp: source rows [slots]
-  unsigned lut;      // float [c_out][256]
+  unsigned lut;      // float [table_channels][256]
   unsigned weights;  // per warp: {wa, wa, wb, wb} per step
   unsigned places;   // per warp: {address of lane 0's word A, funnel shift} per step
   unsigned count;    // per warp: byte [kStripMaxRows]  steps of every output row
@@ -66,7 +66,7 @@ struct StripSmem {
   unsigned ring_bytes;
 };
 
-__host__ __device__ constexpr size_t strip_layout(int c_out, const StripPlan& w, unsigned base, StripSmem* out) {
+__host__ __device__ constexpr size_t strip_layout(int tables, const StripPlan& w, unsigned base, StripSmem* out) {
   StripSmem sm{};
   size_t off = 0;
   sm.mid = base;
@@ -75,7 +75,7 @@ __host__ __device__ constexpr size_t strip_layout(int c_out, const StripPlan& w,
   sm.ring_bytes = (unsigned)w.slots * kSlotBytes;
   off += kWarps * sm.ring_bytes;
   sm.lut = base + (unsigned)off;
-  off += (size_t)c_out * 1024;
+  off += (size_t)tables * 1024;
   sm.weights = base + (unsigned)off;
   off += (size_t)kWarps * w.steps * 16;
   sm.places = base + (unsigned)off;
@@ -370,10 +370,11 @@ __device__ __forceinline__ void walk_cell(
   const Axis ax = planned_axis(s.axis_x, pre_w, s.geom_w);
   // the cast table's values set out here and are stored behind the other tables
   constexpr int kLutQuads = U8 ? 0 : CO * 64;
+  const bool looks_up = p.cast.mode == kCastTable;
   float4 lut[2] = {};
 #pragma unroll
   for (int i = 0; i < 2; i++) {
-    if (tid + i * kStripThreads < kLutQuads) {
+    if (looks_up && tid + i * kStripThreads < kLutQuads) {
       lut[i] = __ldg(reinterpret_cast<const float4*>(p.lut) + tid + i * kStripThreads);
     }
   }
@@ -572,7 +573,7 @@ __device__ __forceinline__ void walk_cell(
   }
 #pragma unroll
   for (int i = 0; i < 2; i++) {
-    if (tid + i * kStripThreads < kLutQuads) {
+    if (looks_up && tid + i * kStripThreads < kLutQuads) {
       sp<float4>(sm.lut)[tid + i * kStripThreads] = lut[i];
     }
   }
@@ -641,7 +642,7 @@ __global__ void __launch_bounds__(kStripThreads, kStripCtas)
   const int fill_y1 = p.pad_apart ? vy1 : y1;         // rows below the post window are the fill CTAs' then
   if (!pad && y0 < vy1) {
     StripSmem sm;
-    strip_layout(p.c_out, plan, smem_addr(smem_raw), &sm);
+    strip_layout(table_channels(p), plan, smem_addr(smem_raw), &sm);
     walk_cell<C, GRAY, U8>(s, p, plan, sm, y0, vy1, x0, x1);
   }
   if (fill_y0 < fill_y1) {
@@ -713,7 +714,7 @@ cudaError_t launch_resize_strip(const LaunchParams& p, const StripPlan& plan_in,
   // Blocks name their cell by three coordinates, which saves two divisions, where they can.
   plan.linear = p.pad_apart || plan.cells_y == 0 || plan.cells_y > 65535 || p.n > 65535;
   const dim3 b = plan.linear ? dim3((unsigned)blocks) : dim3((unsigned)plan.cells_x, (unsigned)plan.cells_y, (unsigned)p.n);
-  const size_t smem = strip_layout(p.c_out, plan, 0u, nullptr);
+  const size_t smem = strip_layout(table_channels(p), plan, 0u, nullptr);
   if (p.out_f32) {
     if (p.gray) {
       return launch<3, true, false>(p, plan, b, smem, stream);

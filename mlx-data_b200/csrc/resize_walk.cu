@@ -57,14 +57,14 @@ constexpr unsigned kMidBytes = kStageRows / 2 * kPairBytes;
 struct WalkSmem {
   unsigned mid;     // float2 [kStageRows / 2][kWalkRow]
   unsigned ring;    // source words [kSlots][warp][68]
-  unsigned lut;     // float [c_out][256]
+  unsigned lut;     // float [table_channels][256]
   unsigned steps;   // 32 bytes per step, kAhead leading entries that only name rows
   unsigned count;   // int [kWalkMaxRows]  steps of every output row
   unsigned hx;      // {first tap's byte offset in a row pair, signed, tap count << 16} per column
   unsigned hw;      // float [tap][walk_px]
 };
 
-__host__ __device__ constexpr size_t walk_layout(int c_out, const WalkPlan& w, unsigned base, WalkSmem* out) {
+__host__ __device__ constexpr size_t walk_layout(int tables, const WalkPlan& w, unsigned base, WalkSmem* out) {
   WalkSmem sm{};
   size_t off = 0;
   sm.mid = base;
@@ -72,7 +72,7 @@ __host__ __device__ constexpr size_t walk_layout(int c_out, const WalkPlan& w, u
   sm.ring = base + (unsigned)off;
   off += kSlots * kSlotBytes;
   sm.lut = base + (unsigned)off;
-  off += (size_t)c_out * 1024;
+  off += (size_t)tables * 1024;
   sm.steps = base + (unsigned)off;
   off += (size_t)(w.steps + 2 * kAhead) * 32;
   sm.count = base + (unsigned)off;
@@ -410,7 +410,7 @@ __device__ __forceinline__ void walk_chunk(
       }
     }
   }
-  if (!U8) {
+  if (!U8 && p.cast.mode == kCastTable) {
     for (int i = tid; i < CO * 256; i += kWalkThreads) {
       sp<float>(sm.lut)[i] = __ldg(p.lut + i);
     }
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
   const int fill_y1 = p.pad_apart ? vy1 : y1;         // rows below the post window are the fill CTAs' then
   if (!strip && y0 < vy1) {
     WalkSmem sm;
-    walk_layout(p.c_out, p.walk, smem_addr(smem_raw), &sm);
+    walk_layout(table_channels(p), p.walk, smem_addr(smem_raw), &sm);
     walk_chunk<C, GRAY, U8>(s, p, sm, y0, vy1, x0, x1);
   }
   if (fill_y0 < fill_y1) {
@@ -607,7 +607,7 @@ cudaError_t launch_resize_walk(const LaunchParams& p_in, bool fills_padding, cud
   if (blocks > 0x7fffffffULL) {
     return cudaErrorInvalidConfiguration;
   }
-  const size_t smem = walk_layout(p.c_out, p.walk, 0u, nullptr);
+  const size_t smem = walk_layout(table_channels(p), p.walk, 0u, nullptr);
   const unsigned b = (unsigned)blocks;
   if (p.out_f32) {
     if (p.gray) {
