@@ -6,6 +6,14 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+
+@pytest.fixture(autouse=True)
+def four_channels(pkg):
+    pkg.core.set_rgba_resize_independent(True)
+    yield
+    pkg.core.set_rgba_resize_independent(False)
+
+
 CASTS = [dict(), dict(scale=1.0), dict(scale=3.7), dict(scale=-2.5e-39), dict(scale=1e38),
          dict(mean=[0.485, 0.456, 0.406, 0.5], std=[0.229, 0.224, 0.225, 0.25]),
          dict(scale=127.5, mean=[1.0, 0.0, -3.0, 7e7], std=[0.5, 3.0, 1e-30, 0.1]),
@@ -24,7 +32,6 @@ def test_float_batch_is_the_cast_of_the_byte_batch(pkg, c, size, cast):
     for k in ("mean", "std"):
         if k in kw:
             kw[k] = kw[k][:co]
-    pkg.core.set_rgba_resize_independent(True)
     ds = pkg.buffer_from_vector(samples).image_resize("image", size, size - 5)
     if gray:
         ds = ds.image_channel_reduction("image", "default")
