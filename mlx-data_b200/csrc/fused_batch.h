@@ -107,6 +107,7 @@ struct ResizePlan {
   StripPlan strip;
   WalkPlan wide;
   int32_t first_wide, wides;   // all of them are among these samples
+  int32_t first_band, bands;   // and the samples of the band kernel (and the direct one) among these
   bool enlarges;      // most resizes enlarge along the row
 };
 
@@ -145,7 +146,6 @@ struct LaunchParams {
   int32_t* status;            // device word, non-zero once a self-check failed
   int32_t band_tiles;         // band kernel: tiles per CTA along a row band (set at launch)
   int32_t bands_x;            // band kernel: CTAs per row band
-  int32_t bands;              // some sample is copied or rotated: the band kernel runs
   WalkPlan walk;              // resize_walk.cu: ResizePlan::wide
   int32_t pad_apart;          // the rows below each post window are filled apart from the cells around them
   int32_t fill_every;         // resize kernels, then: every so many CTAs, from the first on, one of them fills

@@ -532,7 +532,9 @@ cudaError_t launch_fused_batch(const LaunchParams& described, const ResizePlan& 
       return e;
     }
   }
-  if (p.bands) {
+  if (plan.bands > 0) {
+    p.samples += plan.first_band;
+    p.n = plan.bands;
     const cudaError_t e = launch_bands(p, stream);
     if (e != cudaSuccess) {
       return e;

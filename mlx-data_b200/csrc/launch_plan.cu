@@ -42,12 +42,15 @@ struct Cells {
 } // namespace
 
 void choose_kernels(LaunchParams& p, ResizePlan& plan, const DevSample* host_samples, int n) {
-  p.bands = 0;
   p.direct = 0;
+  plan.first_band = plan.bands = 0;
   unsigned long long rows = 0, below = 0;
   for (int i = 0; i < n; i++) {
     const DevSample& s = host_samples[i];
-    p.bands |= s.mode != kModeResize && s.mode != kModeResizeWide;   // a direct sample's padding is the band kernel's too
+    if (s.mode != kModeResize && s.mode != kModeResizeWide) {   // a direct sample's padding is the band kernel's too
+      plan.first_band = plan.bands == 0 ? i : plan.first_band;
+      plan.bands = i + 1 - plan.first_band;
+    }
     p.direct |= s.mode == kModeResizeDirect;
     rows += (unsigned long long)s.slot_h;
     below += (unsigned long long)(s.slot_h > s.post_h ? s.slot_h - s.post_h : 0);
@@ -489,7 +492,48 @@ static void choose_resize_kernel(DevSample* samples, int n, int channels) {
   }
 }
 
+// Copies among resizes (images that have the size already) as resizes by 1 along both axes,
+// with weights of 1 and the same bytes: a launch of the band kernel behind the strips takes
+// 10 us and more, a strip of a copy not much more than the copy.  96 images to a shorter
+// side of 320, one of which has it, 50.4 us of kernels, 41.6 so.  Copies that add up to more
+// than the launch keep it, as do those beside samples that need it anyway.
+static void join_copies(DevSample* samples, int n, int channels) {
+  constexpr float kMost = 10e6f;
+  int copies = 0, strips = 0;
+  for (int i = 0; i < n; i++) {
+    copies += samples[i].mode == kModeCopy;
+    strips += samples[i].mode == kModeResize;
+    if (samples[i].mode == kModeAffine || samples[i].mode == kModeResizeDirect) {
+      return;
+    }
+  }
+  if (copies == 0 || strips == 0) {
+    return;
+  }
+  float cost = 0.0f;
+  for (int pass = 0; pass < 2; pass++) {
+    for (int i = 0; i < n; i++) {
+      if (samples[i].mode != kModeCopy) {
+        continue;
+      }
+      DevSample s = samples[i];
+      set_axes(s);
+      s.mode = resize_mode(s, channels);
+      if (pass == 1) {
+        samples[i] = s;
+        continue;
+      }
+      split_strips(s);
+      cost += strip_time(s, channels);
+      if (s.mode != kModeResize || cost > kMost) {
+        return;
+      }
+    }
+  }
+}
+
 void plan_resize(DevSample* samples, int n, int channels, ResizePlan& plan) {
+  join_copies(samples, n, channels);
   choose_resize_kernel(samples, n, channels);
   plan_strips(samples, n, plan.strip);
   plan_wide(samples, n, channels, plan.wide);
