@@ -1,6 +1,7 @@
 // extern "C" entry points declared in include/mlxd_b200.h.
 #include <cstring>
 #include <new>
+#include <memory>
 #include <optional>
 
 #include "context.h"
@@ -268,7 +269,7 @@ int mlxd_fused_batch_on_stream(
   MLXD_ON_DEVICE(ctx->device);
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   // validate + plan
-  std::vector<DevSample> dev;
+  const std::unique_ptr<DevSample[]> dev(new DevSample[n]);   // (planning sets all of a record)
   mlxd_batch_desc b = *batch;
   Lane& ring = *ctx->lanes[ctx->n_user_lanes + 1];
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -288,11 +289,11 @@ int mlxd_fused_batch_on_stream(
   }
   p.status = ring.d_status;
   ResizePlan plan;
-  rc = plan_samples(samples, n, &b, dev, plan);
+  rc = plan_samples(samples, n, &b, dev.get(), plan);
   if (rc != MLXD_OK) {
     return rc;
   }
-  choose_kernels(p, plan, dev.data(), n);
+  choose_kernels(p, plan, dev.get(), n);
   const size_t esize = p.out_f32 ? 4 : 1;
   const size_t slot_bytes = (size_t)b.slot_h * b.slot_w * p.c_out * esize;
   uint64_t algo_src = 0;
@@ -305,7 +306,7 @@ int mlxd_fused_batch_on_stream(
   ctx->algo_src += algo_src;
   ctx->algo_dst += slot_bytes * n;
   if (captured) {
-    rc = capture_batch(p, plan, dev.data(), &b, stream);
+    rc = capture_batch(p, plan, dev.get(), &b, stream);
     if (rc == MLXD_OK) {
       ctx->batches += 1;
       ctx->samples += n;
@@ -331,13 +332,13 @@ int mlxd_fused_batch_on_stream(
   // ahead of a kernel of 20 us; 285 to 390 samples whose kernels take 150 to 220 us: 3 to 4 %
   // of a pass).  Where the host is the bound it costs up to 2 us more (512 tiny images 27.5
   // us a pass, 25.2 by the copy engine).
-  const void* table = dev.data();
+  const void* table = dev.get();
   if (table_bytes > 64 * 1024) {
     rc = arena_reserve(ctx, ring.h_desc[slot], table_bytes, true, nullptr);
     if (rc != MLXD_OK) {
       return rc;
     }
-    std::memcpy(ring.h_desc[slot].ptr, dev.data(), table_bytes);
+    std::memcpy(ring.h_desc[slot].ptr, dev.get(), table_bytes);
     table = ring.h_desc[slot].ptr;
   }
   MLXD_CUDA(cudaMemcpyAsync(ring.d_desc[slot].ptr, table, table_bytes, cudaMemcpyHostToDevice, stream));

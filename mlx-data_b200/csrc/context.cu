@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <thread>
 
 namespace mlxd {
@@ -218,10 +219,8 @@ int plan_into(const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, 
 }
 
 int plan_samples(
-    const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b,
-    std::vector<DevSample>& out, ResizePlan& plan) {
-  out.resize(n);
-  const int rc = plan_into(samples, n, b, out.data(), plan);
+    const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, DevSample* out, ResizePlan& plan) {
+  const int rc = plan_into(samples, n, b, out, plan);
   // Test hook (MLXD_TEST_SHORT_PLAN=1, read per launch): room for one step a walk.
   // Every resize CTA that has more finds that before it copies or filters anything,
   // sets the status word and returns, so the kernel's self-check and the way from it
@@ -471,14 +470,14 @@ int enqueue_on_lane(
   if (rc != MLXD_OK) {
     return rc;
   }
-  std::vector<DevSample> dev;
+  const std::unique_ptr<DevSample[]> dev(new DevSample[n]);   // (planning sets all of a record)
   p.status = lane.d_status;
   ResizePlan plan;
-  rc = plan_samples(samples, n, batch, dev, plan);
+  rc = plan_samples(samples, n, batch, dev.get(), plan);
   if (rc != MLXD_OK) {
     return rc;
   }
-  choose_kernels(p, plan, dev.data(), n);
+  choose_kernels(p, plan, dev.get(), n);
   const size_t esize = p.out_f32 ? 4 : 1;
   const size_t slot_bytes = (size_t)batch->slot_h * batch->slot_w * p.c_out * esize;
   const size_t out_bytes = slot_bytes * n;
@@ -601,7 +600,7 @@ int enqueue_on_lane(
     dev[i].dst = per_sample_dst ? (*per_sample_dst)[i] : static_cast<void*>(out_base + slot_bytes * i);
   }
 
-  std::memcpy(lane.h_desc[slot].ptr, dev.data(), sizeof(DevSample) * n);
+  std::memcpy(lane.h_desc[slot].ptr, dev.get(), sizeof(DevSample) * n);
   size_t upload = sizeof(DevSample) * n;
   uint32_t gather_rows = 0;
   if (gather) {

@@ -126,8 +126,7 @@ namespace mlxd {
 // Validate descriptors and build the device programs (src/dst pointers are
 // filled by the caller).  Returns MLXD_OK or an error with the message set.
 int plan_samples(
-    const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b,
-    std::vector<DevSample>& out, ResizePlan& plan);
+    const mlxd_sample_desc* samples, int n, const mlxd_batch_desc* b, DevSample* out, ResizePlan& plan);
 
 // One rectangle of a host source that gather.cu packs into device memory:
 // `rows` rows of `row_bytes` bytes, `src_pitch` apart at the source (a pointer

@@ -1,5 +1,6 @@
 #include "mlx/data/core/State.h"
 
+#include <atomic>
 #include <mutex>
 
 namespace mlx {
@@ -15,6 +16,18 @@ std::mutex& process_mutex() {
   static std::mutex m;
   return m;
 }
+
+// The process's version, for threads to see without the lock whether they have it.
+std::atomic<int64_t> current_version{0};
+
+const std::shared_ptr<State>& mine() {
+  static thread_local std::shared_ptr<State> state;
+  if (!state || state->version != current_version.load(std::memory_order_acquire)) {
+    std::lock_guard<std::mutex> g(process_mutex());
+    state = std::make_shared<State>(process_state());
+  }
+  return state;
+}
 } // namespace
 
 void set_state(int64_t seed) {
@@ -22,16 +35,15 @@ void set_state(int64_t seed) {
   State& s = process_state();
   s.randomGenerator = std::mt19937(seed);
   s.version++;
+  current_version.store(s.version, std::memory_order_release);
 }
 
 std::shared_ptr<State> get_state() {
-  static thread_local std::shared_ptr<State> mine;
-  std::lock_guard<std::mutex> g(process_mutex());
-  const State& s = process_state();
-  if (!mine || mine->version != s.version) {
-    mine = std::make_shared<State>(s);
-  }
-  return mine;
+  return mine();
+}
+
+State& thread_state() {
+  return *mine();
 }
 
 } // namespace core

@@ -19,6 +19,10 @@ struct State {
 // The calling thread's state.
 std::shared_ptr<State> get_state();
 
+// The same for ops that draw from it and do not keep it: no lock and no counting as long
+// as it is current.
+State& thread_state();
+
 // Reseed the process-wide generator; call from the main thread only.
 void set_state(int64_t seed);
 

@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <stdexcept>
 #include <string>
 
@@ -53,15 +54,16 @@ void Window::crop(int64_t cx, int64_t cy, int64_t cw, int64_t ch) {
 
 // ---------------------------------------------------------------- LazyImage
 LazyImage::LazyImage(const std::shared_ptr<const Array>& src) : src_(src) {
-  if (src->ndim() != 3) {
+  const std::vector<int64_t>& shape = src->shape();
+  if (shape.size() != 3) {
     throw std::runtime_error("verifyImage: image must be 3 dimension Array (HWC)");
   }
-  channels_ = src->shape(2);
+  channels_ = shape[2];
   if (channels_ == 0 || channels_ > 4) {
     throw std::runtime_error("verifyImage: channels must be 0 <= c <= 4");
   }
-  pre_.w = src->shape(1);
-  pre_.h = src->shape(0);
+  pre_.w = shape[1];
+  pre_.h = shape[0];
   geom_w_ = pre_.w;
   geom_h_ = pre_.h;
   post_ = Window{0, 0, pre_.w, pre_.h, false};
@@ -211,24 +213,40 @@ void LazyImage::gray_params(int32_t m[3], int32_t& bias) const {
 }
 
 void LazyImage::describe(mlxd_sample_desc& d) const {
-  std::memset(&d, 0, sizeof(d));
+  const std::vector<int64_t>& shape = src_->shape();
+  // (a negative number has the high bits too)
+  const int64_t bits = shape[0] | shape[1] | pre_.x | pre_.y | pre_.w | pre_.h | geom_w_ | geom_h_ | post_.x | post_.y |
+      post_.w | post_.h;
+  if (bits & ~int64_t(0x7fffffff)) {
+    to_i32(shape[0], "height");
+    to_i32(shape[1], "width");
+    for (const Window* w : {&pre_, &post_}) {
+      to_i32(w->x, "crop offset");
+      to_i32(w->y, "crop offset");
+      to_i32(w->w, "crop width");
+      to_i32(w->h, "crop height");
+    }
+    to_i32(geom_w_, "target width");
+    to_i32(geom_h_, "target height");
+  }
   d.src = static_cast<const uint8_t*>(src_->data());
-  d.src_h = to_i32(src_->shape(0), "height");
-  d.src_w = to_i32(src_->shape(1), "width");
-  d.pre_x = to_i32(pre_.x, "crop offset");
-  d.pre_y = to_i32(pre_.y, "crop offset");
-  d.pre_w = to_i32(pre_.w, "crop width");
-  d.pre_h = to_i32(pre_.h, "crop height");
+  d.src_h = static_cast<int32_t>(shape[0]);
+  d.src_w = static_cast<int32_t>(shape[1]);
+  d.pre_x = static_cast<int32_t>(pre_.x);
+  d.pre_y = static_cast<int32_t>(pre_.y);
+  d.pre_w = static_cast<int32_t>(pre_.w);
+  d.pre_h = static_cast<int32_t>(pre_.h);
   d.pre_flip = pre_.flip ? 1 : 0;
   d.geom = geom_;
-  d.geom_w = to_i32(geom_w_, "target width");
-  d.geom_h = to_i32(geom_h_, "target height");
+  d.geom_w = static_cast<int32_t>(geom_w_);
+  d.geom_h = static_cast<int32_t>(geom_h_);
   std::memcpy(d.mx, mx_, sizeof(mx_));
-  d.post_x = to_i32(post_.x, "crop offset");
-  d.post_y = to_i32(post_.y, "crop offset");
-  d.post_w = to_i32(post_.w, "crop width");
-  d.post_h = to_i32(post_.h, "crop height");
+  d.post_x = static_cast<int32_t>(post_.x);
+  d.post_y = static_cast<int32_t>(post_.y);
+  d.post_w = static_cast<int32_t>(post_.w);
+  d.post_h = static_cast<int32_t>(post_.h);
   d.post_flip = post_.flip ? 1 : 0;
+  d.reserved = 0;
 }
 
 std::shared_ptr<Array> LazyImage::materialise() const {
@@ -517,7 +535,8 @@ std::shared_ptr<Array> Runtime::batch(
   const LazyImage& first = *images.front();
   int64_t max_h = 0, max_w = 0;
   int on_device = 0;
-  std::vector<mlxd_sample_desc> descs(images.size());
+  // (describe() sets all of a descriptor)
+  const std::unique_ptr<mlxd_sample_desc[]> descs(new mlxd_sample_desc[images.size()]);
   for (int i = 0; i < n; i++) {
     const LazyImage& im = *images[i];
     if (im.source()->type() != UInt8) {
@@ -567,12 +586,12 @@ std::shared_ptr<Array> Runtime::batch(
   mlxd_ctx* c = ctx();
   if (on_callers_stream) {
     // everything stays on the GPU: queue on the caller's stream and return
-    check(mlxd_fused_batch_on_stream(c, where.stream, descs.data(), n, &b));
+    check(mlxd_fused_batch_on_stream(c, where.stream, descs.get(), n, &b));
     return out;
   }
   // one lane per call in flight, whatever thread makes the call
   const int ln = acquire_lane();
-  int rc = mlxd_fused_batch(c, ln, descs.data(), n, &b);
+  int rc = mlxd_fused_batch(c, ln, descs.get(), n, &b);
   if (rc == MLXD_OK) {
     rc = mlxd_batch_wait(c, ln, -1);
   }

@@ -138,7 +138,7 @@ bool ImageRandomCrop::fold(gpu::LazyImage& image) const {
   if (h_ > h || w_ > w) {
     throw std::runtime_error("ImageRandomCrop: target image size larger than input image");
   }
-  auto state = core::get_state();
+  core::State* const state = &core::thread_state();
   // x is drawn before y
   std::uniform_int_distribution<int64_t> draw_x{0, w - w_};
   std::uniform_int_distribution<int64_t> draw_y{0, h - h_};
@@ -188,7 +188,7 @@ ImageRandomAreaCrop::Rect ImageRandomAreaCrop::draw(int64_t w, int64_t h) const 
   if (w_lo > w_hi) {
     return keep;
   }
-  auto state = core::get_state();
+  core::State* const state = &core::thread_state();
   std::uniform_int_distribution<int64_t> draw_w{w_lo, w_hi};
   int64_t tw = 0, th = 0;
   for (int trial = 0; trial < num_trial_; trial++) {
@@ -240,7 +240,7 @@ bool ImageRandomAreaCrop::fold(gpu::LazyImage& image) const {
 
 // ------------------------------------------------------------ flip
 bool ImageRandomHFlip::fold(gpu::LazyImage& image) const {
-  auto state = core::get_state();
+  core::State* const state = &core::thread_state();
   std::uniform_real_distribution<float> unit{0, 1.0};
   if (unit(state->randomGenerator) <= prob_) {
     return image.hflip();

@@ -117,6 +117,7 @@ class ImageRotate : public ImageTransformOp {
   bool fold(gpu::LazyImage& image) const override;
   bool fold_in(gpu::LazyImage& image, const Sample& sample) const override;
   bool reads_sample() const override { return !angle_key_.empty(); }
+  const std::string* reads_key() const override { return &angle_key_; }
 
  private:
   bool fold_angle(gpu::LazyImage& image, double angle) const;

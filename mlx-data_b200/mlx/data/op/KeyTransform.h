@@ -35,8 +35,8 @@ class KeyTransformOp : public Op {
 class FusableOp : public KeyTransformOp {
  public:
   FusableOp(const std::string& ikey, const std::string& okey = "") : KeyTransformOp(ikey, okey) {}
-  // Record this op on `image`.  Returns false when it cannot join the program
-  // already recorded; the caller then materialises the image and folds again,
+  // Record this op on `image`.  Returns false, the image as it was, when it cannot join
+  // the program already recorded; the caller then materialises the image and folds again,
   // and if the op cannot join an empty program either, runs apply_key() on
   // the pixels.
   virtual bool fold(gpu::LazyImage& image) const = 0;
@@ -47,6 +47,8 @@ class FusableOp : public KeyTransformOp {
     return fold(image);
   }
   virtual bool reads_sample() const { return false; }
+  // The entry that fold_in() reads, where it is only one.
+  virtual const std::string* reads_key() const { return nullptr; }
   // True for ops that only enlarge the image's claim on its batch slot (end
   // padding): they may follow one another; any other op after them needs the
   // pixels first.  The batch node checks this before it lets an op draw random

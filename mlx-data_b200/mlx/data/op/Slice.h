@@ -78,7 +78,7 @@ class RandomSlice : public FusableOp {
     std::uniform_real_distribution<> draw(0.0, 1.0);
     std::vector<int64_t> offsets(src->ndim(), 0);
     std::vector<int64_t> shape = src->shape();
-    auto state = core::get_state();
+    core::State* const state = &core::thread_state();
     for (size_t i = 0; i < dims_.size(); i++) {
       const int d = src->checkdim(dims_[i]);
       const int64_t room = shape[d] - sizes_[i];
@@ -103,7 +103,7 @@ class RandomSlice : public FusableOp {
     std::uniform_real_distribution<> draw(0.0, 1.0);
     int64_t off[2] = {0, 0};
     int64_t len[2] = {image.height(), image.width()};
-    auto state = core::get_state();
+    core::State* const state = &core::thread_state();
     for (size_t i = 0; i < dims_.size(); i++) {
       const int d = dims_[i] < 0 ? dims_[i] + 3 : dims_[i];
       const int64_t room = len[d] - sizes_[i];
