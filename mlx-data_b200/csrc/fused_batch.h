@@ -8,8 +8,8 @@
 
 namespace mlxd {
 
-constexpr int kTileH = 16;    // copy and affine bands: output rows per CTA
-constexpr int kTileW = 64;    // and output pixels per tile
+constexpr int kTileH = 16;    // copies and rotations: output rows per CTA
+constexpr int kTileW = 64;    // and output pixels per tile of a copy
 constexpr int kThreads = 256;
 
 // Resize kernel (resize_strip.cu): a warp walks down a strip of output columns.
@@ -108,6 +108,7 @@ struct ResizePlan {
   WalkPlan wide;
   int32_t first_wide, wides;   // all of them are among these samples
   int32_t first_band, bands;   // and the samples of the band kernel (and the direct one) among these
+  int32_t first_affine, affines;   // and those of affine.cu among these
   bool enlarges;      // most resizes enlarge along the row
 };
 
@@ -158,9 +159,11 @@ __host__ __device__ inline int table_channels(const LaunchParams& p) {
 }
 
 // Launch the kernels the parameters call for: the resize kernel or, without a
-// resize and when p.pad_apart is set, pad_fill_kernel, the band kernel, resize_direct_kernel.
+// resize and when p.pad_apart is set, pad_fill_kernel, affine_kernel, the band kernel,
+// resize_direct_kernel.
 cudaError_t launch_fused_batch(const LaunchParams& p, const ResizePlan& plan, cudaStream_t stream);
 cudaError_t launch_resize_strip(const LaunchParams& p, const StripPlan& plan, cudaStream_t stream);
+cudaError_t launch_affine(const LaunchParams& p, cudaStream_t stream);
 cudaError_t launch_resize_walk(const LaunchParams& p, bool fills_padding, cudaStream_t stream);
 
 // axis_x, axis_y (the divisions of make_axis(), correctly rounded here as there) and

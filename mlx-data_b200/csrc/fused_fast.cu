@@ -1,37 +1,18 @@
-// The kernels around the resize kernels (resize_strip.cu, resize_walk.cu): copy (crop / flip /
-// batch only) and nearest-neighbour affine bands, padding of ragged batches,
-// and resizes whose taps fit no chunk of resize_walk.cu.
+// The kernels around the resize kernels (resize_strip.cu, resize_walk.cu) and the rotations
+// (affine.cu): bands of copies (crop / flip / batch only), padding of ragged batches, and
+// resizes whose taps fit no chunk of resize_walk.cu.
 //
-// Copy and affine: one CTA per band of up to eight kTileH x kTileW tiles of one
-// sample's slot; the source is read through the read-only path, four pixels per
-// thread, and stored 16 bytes at a time; pad-only bands are plain 16-byte
-// stores.  The rows below a sample in a ragged batch go out through a linear fill
-// kernel when the launch has no resize (else CTAs of a resize kernel write them).
-// A resize too strong for both resize kernels is filtered pixel by pixel from
-// global memory by a kernel of its own.
+// Copies: one CTA per band of up to eight kTileH x kTileW tiles of one sample's slot;
+// the source is read through the read-only path, four pixels per thread, and stored 16
+// bytes at a time; pad-only bands are plain 16-byte stores.  The rows below a sample in
+// a ragged batch go out through a linear fill kernel when the launch has no resize (else
+// CTAs of a resize kernel write them).  A resize too strong for both resize kernels is
+// filtered pixel by pixel from global memory by a kernel of its own.
 #include "fused_batch.h"
 #include "kernel_common.cuh"
 
 namespace mlxd {
 namespace {
-
-// Source pixel of post-window pixel (px, y) of an affine sample: coordinates in
-// the pre window, or false when it falls outside it (the output is 0 there).
-// The coordinate is built from float products and float sums, then two double
-// additions, then truncation toward zero - the evaluation order of the
-// reference expression - and no multiply-add is contracted.
-__device__ __forceinline__ bool affine_source(
-    const DevSample& s, int gx, int gy, float twh, float thh, float wh, float hh, int& sx, int& sy) {
-  const float dxf = __fsub_rn((float)(long long)gx, twh);
-  const float dyf = __fsub_rn((float)(long long)gy, thh);
-  const float fx = __fadd_rn(__fadd_rn(__fmul_rn(s.mx[0], dxf), __fmul_rn(s.mx[1], dyf)), s.mx[2]);
-  const float fy = __fadd_rn(__fadd_rn(__fmul_rn(s.mx[3], dxf), __fmul_rn(s.mx[4], dyf)), s.mx[5]);
-  const long long ax = (long long)__dadd_rn(__dadd_rn((double)fx, 0.5), (double)wh);
-  const long long ay = (long long)__dadd_rn(__dadd_rn((double)fy, 0.5), (double)hh);
-  sx = (int)ax;
-  sy = (int)ay;
-  return !(ax < 0 || ay < 0 || ax >= s.pre_w || ay >= s.pre_h);
-}
 
 // N floats that start HEAD floats before a 16-byte boundary: whole 16-byte units
 // where they lie, single floats around them.
@@ -51,23 +32,18 @@ __device__ __forceinline__ void store_run(float* dst, const float* v) {
   }
 }
 
-// Copy (crop / flip / batch only) and nearest-neighbour affine tiles: rows
-// [y0, vy1) x columns [xa, xb) of the slot, a thread takes four adjacent pixels
-// of a row.  The cast table is read from shared memory (lut_s); the four pixels
-// leave as 16-byte stores when the row segment allows it.  Without a geometric
-// op the four source pixels are adjacent too and come as aligned words.
+// Copies (crop / flip / batch only): rows [y0, vy1) x columns [xa, xb) of the slot, a
+// thread takes four adjacent pixels of a row, which come as aligned words.  The cast
+// table is read from shared memory (lut_s); the four pixels leave as 16-byte stores
+// when the row segment allows it.
 template <int C, bool GRAY, bool U8>
-__device__ void gather_rows(
+__device__ void copy_rows(
     const DevSample& s, const LaunchParams& p, unsigned lut_s, int y0, int vy1, int xa, int xb) {
   constexpr int CO = GRAY ? 1 : C;
   const int nvx = xb - xa;
   const int nvy = vy1 - y0;
   const int quads = (nvx + 3) >> 2;
   float* base = reinterpret_cast<float*>(s.dst);
-  const float twh = (float)((double)s.geom_w / 2.0);
-  const float thh = (float)((double)s.geom_h / 2.0);
-  const float wh = (float)((double)s.pre_w / 2.0);
-  const float hh = (float)((double)s.pre_h / 2.0);
   const size_t row_floats = (size_t)s.slot_w * CO;
   const bool vec_ok = (row_floats & 3) == 0 && ((xa * CO) & 3) == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0;
   // last 4-byte word of the source image: nothing behind it is read
@@ -79,66 +55,44 @@ __device__ void gather_rows(
     const int npx = min(4, xb - x_first);
     const int gy = s.post_y + y0 + ry;
     unsigned px[4][C];   // source bytes of the four pixels
-    if (s.mode == kModeAffine) {
+    // pre_flip is folded into post_flip for copies: the source pixels of columns
+    // x_first .. x_first + 3 are adjacent, ascending or (mirrored) descending
+    const int gx_a = s.post_x + (s.post_flip ? (s.post_w - 1 - x_first) : x_first);
+    const int sx_lo = s.pre_x + (s.post_flip ? gx_a - (npx - 1) : gx_a);
+    const uintptr_t g =
+        reinterpret_cast<uintptr_t>(s.src) + ((size_t)(s.pre_y + gy) * s.src_w + sx_lo) * C;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(g & ~(uintptr_t)3);
+    const unsigned sh = (unsigned)(g & 3) * 8u;
+    const int need = (int)(g & 3) + npx * C;   // bytes from the first word on
+    uint32_t x[C + 1];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int x = x_first + (j < npx ? j : 0);
-        const int gx = s.post_x + (s.post_flip ? (s.post_w - 1 - x) : x);
-        int sx, sy;
-        const bool inside = affine_source(s, gx, gy, twh, thh, wh, hh, sx, sy);
-        const int ix = s.pre_x + (s.pre_flip ? (s.pre_w - 1 - sx) : sx);
-        // the pixel's C bytes from the one or two aligned words that hold them
-        const uintptr_t g = reinterpret_cast<uintptr_t>(s.src) + ((size_t)(s.pre_y + sy) * s.src_w + ix) * C;
-        const uint32_t* w = reinterpret_cast<const uint32_t*>(g & ~(uintptr_t)3);
-        const unsigned sh = (unsigned)(g & 3) * 8u;
-        const uint32_t w0 = inside ? __ldg(w) : 0u;
-        const uint32_t w1 = (inside && (int)(g & 3) + C > 4) ? __ldg(w + 1) : 0u;
-        const uint32_t v = __funnelshift_r(w0, w1, sh);
+    for (int k = 0; k < C + 1; k++) {
+      const bool take = 4 * k < need && reinterpret_cast<uintptr_t>(w + k) <= last_word;
+      x[k] = take ? __ldg(w + k) : 0u;
+    }
+    uint32_t v[C];   // the 4 * C bytes from g on
 #pragma unroll
-        for (int ch = 0; ch < C; ch++) {
-          px[j][ch] = (v >> (8 * ch)) & 0xffu;
-        }
-      }
-    } else {
-      // pre_flip is folded into post_flip for copies: the source pixels of columns
-      // x_first .. x_first + 3 are adjacent, ascending or (mirrored) descending
-      const int gx_a = s.post_x + (s.post_flip ? (s.post_w - 1 - x_first) : x_first);
-      const int sx_lo = s.pre_x + (s.post_flip ? gx_a - (npx - 1) : gx_a);
-      const uintptr_t g =
-          reinterpret_cast<uintptr_t>(s.src) + ((size_t)(s.pre_y + gy) * s.src_w + sx_lo) * C;
-      const uint32_t* w = reinterpret_cast<const uint32_t*>(g & ~(uintptr_t)3);
-      const unsigned sh = (unsigned)(g & 3) * 8u;
-      const int need = (int)(g & 3) + npx * C;   // bytes from the first word on
-      uint32_t x[C + 1];
+    for (int k = 0; k < C; k++) {
+      v[k] = __funnelshift_r(x[k], x[k + 1], sh);
+    }
 #pragma unroll
-      for (int k = 0; k < C + 1; k++) {
-        const bool take = 4 * k < need && reinterpret_cast<uintptr_t>(w + k) <= last_word;
-        x[k] = take ? __ldg(w + k) : 0u;
-      }
-      uint32_t v[C];   // the 4 * C bytes from g on
+    for (int j = 0; j < 4; j++) {
 #pragma unroll
-      for (int k = 0; k < C; k++) {
-        v[k] = __funnelshift_r(x[k], x[k + 1], sh);
-      }
+      for (int ch = 0; ch < C; ch++) {
+        const int byte = j * C + ch;
+        // mirrored: output pixel j is source pixel npx - 1 - j; places a row's last
+        // quad leaves over index the cast table too, so they get some byte of the quad
+        const int back = ((npx - 1 - j) & 3) * C + ch;
+        unsigned val = (v[byte >> 2] >> (8 * (byte & 3))) & 0xffu;
+        if (s.post_flip) {
+          val = 0;
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-#pragma unroll
-        for (int ch = 0; ch < C; ch++) {
-          const int byte = j * C + ch;
-          // mirrored: output pixel j is source pixel npx - 1 - j; places a row's last
-          // quad leaves over index the cast table too, so they get some byte of the quad
-          const int back = ((npx - 1 - j) & 3) * C + ch;
-          unsigned val = (v[byte >> 2] >> (8 * (byte & 3))) & 0xffu;
-          if (s.post_flip) {
-            val = 0;
-#pragma unroll
-            for (int o = 0; o < 4; o++) {
-              const int from = o * C + ch;
-              val = back == from ? (v[from >> 2] >> (8 * (from & 3))) & 0xffu : val;
-            }
+          for (int o = 0; o < 4; o++) {
+            const int from = o * C + ch;
+            val = back == from ? (v[from >> 2] >> (8 * (from & 3))) & 0xffu : val;
           }
-          px[j][ch] = val;
         }
+        px[j][ch] = val;
       }
     }
     if (U8) {
@@ -237,8 +191,8 @@ __device__ void run_band(const LaunchParams& p, float* lut_s) {
   if (n >= p.n) {
     return;
   }
-  if (p.samples[n].mode == kModeResize || p.samples[n].mode == kModeResizeWide) {
-    return;   // the resize kernels'
+  if (p.samples[n].mode != kModeCopy && p.samples[n].mode != kModeResizeDirect) {
+    return;   // the other kernels'
   }
   const DevSample s = p.samples[n];
   const int y0 = ty * kTileH;
@@ -280,7 +234,7 @@ __device__ void run_band(const LaunchParams& p, float* lut_s) {
   }
   if (s.mode != kModeResizeDirect) {
     __syncthreads();
-    gather_rows<C, GRAY, U8>(s, p, smem_addr(lut_s), y0, vy1, x0, vx1);
+    copy_rows<C, GRAY, U8>(s, p, smem_addr(lut_s), y0, vy1, x0, vx1);
   }
   // (the post window of a kModeResizeDirect sample is resize_direct_kernel's)
   // pad the part of the band outside the post window
@@ -528,6 +482,15 @@ cudaError_t launch_fused_batch(const LaunchParams& described, const ResizePlan& 
       q.n = plan.wides;
     }
     const cudaError_t e = launch_resize_walk(q, !strips, stream);
+    if (e != cudaSuccess) {
+      return e;
+    }
+  }
+  if (plan.affines > 0) {
+    LaunchParams q = p;
+    q.samples += plan.first_affine;
+    q.n = plan.affines;
+    const cudaError_t e = launch_affine(q, stream);
     if (e != cudaSuccess) {
       return e;
     }

@@ -43,11 +43,14 @@ struct Cells {
 
 void choose_kernels(LaunchParams& p, ResizePlan& plan, const DevSample* host_samples, int n) {
   p.direct = 0;
-  plan.first_band = plan.bands = 0;
+  plan.first_band = plan.bands = plan.first_affine = plan.affines = 0;
   unsigned long long rows = 0, below = 0;
   for (int i = 0; i < n; i++) {
     const DevSample& s = host_samples[i];
-    if (s.mode != kModeResize && s.mode != kModeResizeWide) {   // a direct sample's padding is the band kernel's too
+    if (s.mode == kModeAffine) {
+      plan.first_affine = plan.affines == 0 ? i : plan.first_affine;
+      plan.affines = i + 1 - plan.first_affine;
+    } else if (s.mode != kModeResize && s.mode != kModeResizeWide) {   // a direct sample's padding is the band kernel's too
       plan.first_band = plan.bands == 0 ? i : plan.first_band;
       plan.bands = i + 1 - plan.first_band;
     }

@@ -7,13 +7,6 @@
 
 namespace mlxd {
 
-// d = a * b + c on both lanes.
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
 // (int)(acc + 0.5) of both lanes as the low mantissa bits of 2^23 + that
 // integer.  acc is never negative and at most 255 (1 + 1e-4) here - pixels
 // times weights that sum to 1 within the rounding of a few hundred terms - so
@@ -38,18 +31,6 @@ __device__ __forceinline__ void sts_v4(unsigned a, float x, float y, float z, fl
 template <int OFF>
 __device__ __forceinline__ void lds_v4u32(unsigned a, uint32_t& x, uint32_t& y, uint32_t& z, uint32_t& w) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4+%5];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(a), "n"(OFF));
-}
-
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
 }
 
 __device__ __forceinline__ f32x2 both(const float (&pair)[2]) {
