@@ -65,6 +65,8 @@ struct Arena {
 };
 
 constexpr int kDescSlots = 4;
+constexpr int32_t kStatusPending = INT32_MIN;   // no status of a kernel
+constexpr int kLookMicroseconds = 3000;         // a thread looks for the status so long before it blocks
 
 struct Lane {
   cudaStream_t stream = nullptr;
@@ -85,7 +87,7 @@ struct Lane {
   bool out_timed[kDescSlots] = {};
   int next_slot = 0;
   int32_t* d_status = nullptr;        // this lane's word of the context's status block
-  int32_t* h_status = nullptr;        // pinned copy of the device status word
+  int32_t* h_status = nullptr;        // pinned copy of the device status word, kStatusPending while it is under way
   std::mutex mu;                      // one caller at a time per lane
 };
 
