@@ -304,9 +304,10 @@ __device__ __forceinline__ void affine_rows(
 }
 
 // One CTA: rows [y0, y0 + kTileH) of one slot, `columns` columns.
-template <int C, bool GRAY, bool U8>
+template <int C, bool GRAY, bool U8, int K>
 __global__ void __launch_bounds__(kAffineThreads, kAffineCtas)
-    affine_kernel(const __grid_constant__ LaunchParams p, int columns, int bands_x) {
+    affine_kernel(
+        const __grid_constant__ LaunchParams p, int columns, int bands_x, const __grid_constant__ Records<K> records) {
   constexpr int CO = GRAY ? 1 : C;
   __shared__ __align__(1024) float lut_s[U8 ? 1 : CO * 256];
   __shared__ __align__(16) unsigned char patch[kAffineThreads / 32][640];
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(kAffineThreads, kAffineCtas)
   const int tb = (int)(t % bands_x);
   t /= bands_x;
   const int y0 = (int)(t % p.tiles_y) * kTileH;
-  const DevSample* const sample = p.samples + t / p.tiles_y;
+  const DevSample* const sample = records.of(p, t / p.tiles_y);
   const DevSample& s = *sample;
   if (s.mode != kModeAffine) {
     return;   // the other kernels'
@@ -366,10 +367,18 @@ __global__ void __launch_bounds__(kAffineThreads, kAffineCtas)
   }
 }
 
+template <int C, bool GRAY, bool U8, int K>
+void launch_one(
+    const LaunchParams& p, unsigned blocks, int columns, int bands_x, const Records<K>& records, cudaStream_t stream) {
+  affine_kernel<C, GRAY, U8, K><<<blocks, kAffineThreads, 0, stream>>>(p, columns, bands_x, records);
+}
+
 template <int C, bool GRAY, bool U8>
 cudaError_t launch(const LaunchParams& p, unsigned blocks, int columns, int bands_x, cudaStream_t stream) {
-  affine_kernel<C, GRAY, U8><<<blocks, kAffineThreads, 0, stream>>>(p, columns, bands_x);
-  return cudaGetLastError();
+  return with_records(p, [&](const auto& records) {
+    launch_one<C, GRAY, U8>(p, blocks, columns, bands_x, records, stream);
+    return cudaGetLastError();
+  });
 }
 
 template <bool U8>

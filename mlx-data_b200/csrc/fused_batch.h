@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cstring>
+
 namespace mlxd {
 
 constexpr int kTileH = 16;    // copies and rotations: output rows per CTA
@@ -132,8 +134,10 @@ struct CastSteps {
 };
 
 struct LaunchParams {
-  const DevSample* samples;
+  const DevSample* samples;   // in device memory, or null: `carried`
+  const DevSample* carried;   // in host memory, for the launch to take along (carried_samples)
   int32_t n;
+  int32_t first;              // the launch's samples are these from `first` on
   int32_t tiles_y, tiles_x;   // tile grid of the largest slot
   int32_t c_in;               // channels of every source
   int32_t c_out;              // 1 when gray, else c_in
@@ -153,9 +157,49 @@ struct LaunchParams {
   int32_t direct;             // some sample is kModeResizeDirect: resize_direct_kernel runs last
 };
 
+// Sample records as a kernel's parameter: up to K of them, or (0) none, where they are read
+// from LaunchParams::samples.  A kernel may have 32 764 bytes of parameters; each launch
+// moves all of them, so there are two sizes.  4 images of 480x640 to 224x224 take 10.8 us a pass
+// with 24, 13.2 with 128, 15.3 with a table copied ahead of the kernel; 32 of 200-500 px 17.5 with
+// 128 and 20.9 with a table.
+constexpr int kFewSamples = 24, kMoreSamples = 128;
+
+template <int K>
+struct Records {
+  DevSample at[K];
+  __device__ __forceinline__ const DevSample* of(const LaunchParams& p, unsigned t) const { return at + p.first + t; }
+};
+
+template <>
+struct Records<0> {
+  __device__ __forceinline__ const DevSample* of(const LaunchParams& p, unsigned t) const { return p.samples + p.first + t; }
+};
+
+// launch(records) with the records of a launch's samples.
+template <class F>
+inline cudaError_t with_records(const LaunchParams& p, F&& launch) {
+  if (p.samples) {
+    return launch(Records<0>{});
+  }
+  const int count = p.first + p.n;
+  if (count <= kFewSamples) {
+    Records<kFewSamples> r;
+    std::memcpy(r.at, p.carried, sizeof(DevSample) * count);
+    return launch(r);
+  }
+  Records<kMoreSamples> r;
+  std::memcpy(r.at, p.carried, sizeof(DevSample) * count);
+  return launch(r);
+}
+
 // Channels of cast tables that a resize kernel keeps in shared memory.
 __host__ __device__ inline int table_channels(const LaunchParams& p) {
   return p.out_f32 && p.cast.mode == kCastTable ? p.c_out : 0;
+}
+
+// Whether launches can carry their samples: those of the kernels for strong shrinks are read from a table.
+inline bool carried_samples(const LaunchParams& p, const ResizePlan& plan) {
+  return p.n <= kMoreSamples && plan.wide.px == 0 && !p.direct;
 }
 
 // Launch the kernels the parameters call for: the resize kernel or, without a

@@ -181,8 +181,8 @@ __device__ void copy_rows(
 }
 
 // One CTA: rows [y0, y0 + kTileH) of one slot, columns of p.band_tiles tiles.
-template <int C, bool GRAY, bool U8>
-__device__ void run_band(const LaunchParams& p, float* lut_s) {
+template <int C, bool GRAY, bool U8, int K>
+__device__ void run_band(const LaunchParams& p, const Records<K>& records, float* lut_s) {
   unsigned t = blockIdx.x;
   const int tb = t % p.bands_x;
   t /= p.bands_x;
@@ -191,10 +191,11 @@ __device__ void run_band(const LaunchParams& p, float* lut_s) {
   if (n >= p.n) {
     return;
   }
-  if (p.samples[n].mode != kModeCopy && p.samples[n].mode != kModeResizeDirect) {
+  const DevSample* const sample = records.of(p, (unsigned)n);
+  if (sample->mode != kModeCopy && sample->mode != kModeResizeDirect) {
     return;   // the other kernels'
   }
-  const DevSample s = p.samples[n];
+  const DevSample s = *sample;
   const int y0 = ty * kTileH;
   const int x0 = tb * p.band_tiles * kTileW;
   if (y0 >= s.slot_h || x0 >= s.slot_w) {
@@ -244,53 +245,63 @@ __device__ void run_band(const LaunchParams& p, float* lut_s) {
   pad_rect(y0, vy1, vx1, x1);
 }
 
-__global__ void __launch_bounds__(kThreads, 3) fused_fast_kernel(const LaunchParams p) {
+template <int K>
+__global__ void __launch_bounds__(kThreads, 3) fused_fast_kernel(
+    const __grid_constant__ LaunchParams p, const __grid_constant__ Records<K> records) {
   __shared__ __align__(16) float lut_s[4 * 256];
   if (p.c_in == 3) {
-    run_band<3, false, false>(p, lut_s);
+    run_band<3, false, false>(p, records, lut_s);
   } else if (p.c_in == 1) {
-    run_band<1, false, false>(p, lut_s);
+    run_band<1, false, false>(p, records, lut_s);
   } else {
-    run_band<4, false, false>(p, lut_s);
+    run_band<4, false, false>(p, records, lut_s);
   }
 }
 
 // Two-channel images, float32 batches.  Rare; kept out of the kernel above so
 // that its register allocation is decided by the common cases alone.
-__global__ void __launch_bounds__(kThreads, 3) fused_fast_c2_kernel(const LaunchParams p) {
+template <int K>
+__global__ void __launch_bounds__(kThreads, 3) fused_fast_c2_kernel(
+    const __grid_constant__ LaunchParams p, const __grid_constant__ Records<K> records) {
   __shared__ __align__(16) float lut_s[2 * 256];
-  run_band<2, false, false>(p, lut_s);
+  run_band<2, false, false>(p, records, lut_s);
 }
 
 // uint8 batches (no cast): stand-alone ops, images between two geometric ops,
 // pipelines that cast on the host.  Kernels of their own for the same reason
 // as the channel-reduction one.
-__global__ void __launch_bounds__(kThreads, 3) fused_fast_u8_kernel(const LaunchParams p) {
+template <int K>
+__global__ void __launch_bounds__(kThreads, 3) fused_fast_u8_kernel(
+    const __grid_constant__ LaunchParams p, const __grid_constant__ Records<K> records) {
   __shared__ __align__(16) float lut_s[4];
   if (p.c_in == 3) {
     if (p.gray) {
-      run_band<3, true, true>(p, lut_s);
+      run_band<3, true, true>(p, records, lut_s);
     } else {
-      run_band<3, false, true>(p, lut_s);
+      run_band<3, false, true>(p, records, lut_s);
     }
   } else if (p.c_in == 1) {
-    run_band<1, false, true>(p, lut_s);
+    run_band<1, false, true>(p, records, lut_s);
   } else if (p.c_in == 2) {
-    run_band<2, false, true>(p, lut_s);
+    run_band<2, false, true>(p, records, lut_s);
   } else {
-    run_band<4, false, true>(p, lut_s);
+    run_band<4, false, true>(p, records, lut_s);
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 6) pad_fill_kernel(const LaunchParams p) {
-  pad_below_any<kThreads>(p, blockIdx.x);
+template <int K>
+__global__ void __launch_bounds__(kThreads, 6) pad_fill_kernel(
+    const __grid_constant__ LaunchParams p, const __grid_constant__ Records<K> records) {
+  pad_below_any<kThreads>(p, records, blockIdx.x);
 }
 
 // Launches that end in the channel reduction: three channels in, one out.  A
 // kernel of its own, so that the usual one's register allocation is not touched.
-__global__ void __launch_bounds__(kThreads, 3) fused_fast_gray_kernel(const LaunchParams p) {
+template <int K>
+__global__ void __launch_bounds__(kThreads, 3) fused_fast_gray_kernel(
+    const __grid_constant__ LaunchParams p, const __grid_constant__ Records<K> records) {
   __shared__ __align__(16) float lut_s[256];
-  run_band<3, true, false>(p, lut_s);
+  run_band<3, true, false>(p, records, lut_s);
 }
 
 } // namespace
@@ -385,8 +396,8 @@ __device__ void direct_pixel(const DevSample& s, const LaunchParams& p, int ox, 
 
 constexpr int kDirectChunks = 64;   // CTAs per sample
 
-__global__ void __launch_bounds__(kThreads) resize_direct_kernel(const LaunchParams p) {
-  const DevSample& s = p.samples[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) resize_direct_kernel(const __grid_constant__ LaunchParams p) {
+  const DevSample& s = *Records<0>().of(p, blockIdx.y);
   if (s.mode != kModeResizeDirect) {
     return;
   }
@@ -405,6 +416,24 @@ __global__ void __launch_bounds__(kThreads) resize_direct_kernel(const LaunchPar
     } else {
       direct_pixel<4>(s, p, ox, oy);
     }
+  }
+}
+
+template <int K>
+static void launch_fill(const LaunchParams& p, const Records<K>& records, cudaStream_t stream) {
+  pad_fill_kernel<K><<<(unsigned)p.n * kPadChunks, kThreads, 0, stream>>>(p, records);
+}
+
+template <int K>
+static void launch_band_kernel(const LaunchParams& p, const Records<K>& records, unsigned blocks, cudaStream_t stream) {
+  if (!p.out_f32) {
+    fused_fast_u8_kernel<K><<<blocks, kThreads, 0, stream>>>(p, records);
+  } else if (p.c_in == 2) {
+    fused_fast_c2_kernel<K><<<blocks, kThreads, 0, stream>>>(p, records);
+  } else if (p.gray) {
+    fused_fast_gray_kernel<K><<<blocks, kThreads, 0, stream>>>(p, records);
+  } else {
+    fused_fast_kernel<K><<<blocks, kThreads, 0, stream>>>(p, records);
   }
 }
 
@@ -439,16 +468,10 @@ static cudaError_t launch_bands(LaunchParams p, cudaStream_t stream) {
   if (blocks > 0x7fffffffULL) {
     return cudaErrorInvalidConfiguration;
   }
-  if (!p.out_f32) {
-    fused_fast_u8_kernel<<<(unsigned)blocks, kThreads, 0, stream>>>(p);
-  } else if (p.c_in == 2) {
-    fused_fast_c2_kernel<<<(unsigned)blocks, kThreads, 0, stream>>>(p);
-  } else if (p.gray) {
-    fused_fast_gray_kernel<<<(unsigned)blocks, kThreads, 0, stream>>>(p);
-  } else {
-    fused_fast_kernel<<<(unsigned)blocks, kThreads, 0, stream>>>(p);
-  }
-  return cudaGetLastError();
+  return with_records(p, [&](const auto& records) {
+    launch_band_kernel(p, records, (unsigned)blocks, stream);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t launch_fused_batch(const LaunchParams& described, const ResizePlan& plan, cudaStream_t stream) {
@@ -463,8 +486,10 @@ cudaError_t launch_fused_batch(const LaunchParams& described, const ResizePlan& 
   }
   const bool strips = plan.strip.columns > 0, wides = plan.wide.px > 0;
   if (p.pad_apart && !strips && !wides) {   // a resize kernel fills the padding itself
-    pad_fill_kernel<<<(unsigned)p.n * kPadChunks, kThreads, 0, stream>>>(p);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = with_records(p, [&](const auto& records) {
+      launch_fill(p, records, stream);
+      return cudaGetLastError();
+    });
     if (e != cudaSuccess) {
       return e;
     }
@@ -478,7 +503,7 @@ cudaError_t launch_fused_batch(const LaunchParams& described, const ResizePlan& 
   if (wides) {
     LaunchParams q = p;
     if (strips) {
-      q.samples += plan.first_wide;
+      q.first += plan.first_wide;
       q.n = plan.wides;
     }
     const cudaError_t e = launch_resize_walk(q, !strips, stream);
@@ -488,7 +513,7 @@ cudaError_t launch_fused_batch(const LaunchParams& described, const ResizePlan& 
   }
   if (plan.affines > 0) {
     LaunchParams q = p;
-    q.samples += plan.first_affine;
+    q.first += plan.first_affine;
     q.n = plan.affines;
     const cudaError_t e = launch_affine(q, stream);
     if (e != cudaSuccess) {
@@ -496,7 +521,7 @@ cudaError_t launch_fused_batch(const LaunchParams& described, const ResizePlan& 
     }
   }
   if (plan.bands > 0) {
-    p.samples += plan.first_band;
+    p.first += plan.first_band;
     p.n = plan.bands;
     const cudaError_t e = launch_bands(p, stream);
     if (e != cudaSuccess) {

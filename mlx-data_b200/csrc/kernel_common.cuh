@@ -296,14 +296,14 @@ __device__ __forceinline__ void fill_rect_u8(
 // strips to the right of the post window are the band kernel's, or cells of the
 // resize kernel.  THREADS is a CTA's thread count: read from blockDim, it made the
 // fill kernel spill (64 images of 64x64 in slots of 4000x100: 99.3 us a pass, 96.5 so).
-template <int CO, int THREADS>
-__device__ __forceinline__ void pad_below(const LaunchParams& p, unsigned block) {
+template <int CO, int THREADS, int K>
+__device__ __forceinline__ void pad_below(const LaunchParams& p, const Records<K>& records, unsigned block) {
   const int n = (int)(block / kPadChunks);
   const int chunk = (int)(block % kPadChunks);
   if (n >= p.n) {
     return;
   }
-  const DevSample* s = p.samples + n;
+  const DevSample* s = records.of(p, (unsigned)n);
   const int slot_h = s->slot_h, slot_w = s->slot_w;
   const int post_h = s->post_h < slot_h ? s->post_h : slot_h;
   const int first_row = post_h;
@@ -343,14 +343,14 @@ __device__ __forceinline__ void pad_below(const LaunchParams& p, unsigned block)
 }
 
 // The same for a uint8 batch: a linear fill of bytes.
-template <int THREADS>
-__device__ __forceinline__ void pad_below_u8(const LaunchParams& p, unsigned block) {
+template <int THREADS, int K>
+__device__ __forceinline__ void pad_below_u8(const LaunchParams& p, const Records<K>& records, unsigned block) {
   const int n = (int)(block / kPadChunks);
   const int chunk = (int)(block % kPadChunks);
   if (n >= p.n) {
     return;
   }
-  const DevSample* s = p.samples + n;
+  const DevSample* s = records.of(p, (unsigned)n);
   const int slot_h = s->slot_h, slot_w = s->slot_w;
   const int post_h = s->post_h < slot_h ? s->post_h : slot_h;
   const int first_row = post_h;
@@ -380,18 +380,18 @@ __device__ __forceinline__ void pad_below_u8(const LaunchParams& p, unsigned blo
 }
 
 // Block `block` of n * kPadChunks.
-template <int THREADS>
-__device__ __forceinline__ void pad_below_any(const LaunchParams& p, unsigned block) {
+template <int THREADS, int K>
+__device__ __forceinline__ void pad_below_any(const LaunchParams& p, const Records<K>& records, unsigned block) {
   if (!p.out_f32) {
-    pad_below_u8<THREADS>(p, block);
+    pad_below_u8<THREADS>(p, records, block);
   } else if (p.c_out == 3) {
-    pad_below<3, THREADS>(p, block);
+    pad_below<3, THREADS>(p, records, block);
   } else if (p.c_out == 1) {
-    pad_below<1, THREADS>(p, block);
+    pad_below<1, THREADS>(p, records, block);
   } else if (p.c_out == 2) {
-    pad_below<2, THREADS>(p, block);
+    pad_below<2, THREADS>(p, records, block);
   } else {
-    pad_below<4, THREADS>(p, block);
+    pad_below<4, THREADS>(p, records, block);
   }
 }
 

@@ -585,9 +585,11 @@ __device__ __forceinline__ void walk_cell(
 
 // One cell: a strip (or one of padding) of a slot.
 // OWN: samples count their own cells off (StripPlan::cells_y of 0).
-template <int C, bool GRAY, bool U8, bool OWN>
+template <int C, bool GRAY, bool U8, bool OWN, int K>
 __global__ void __launch_bounds__(kStripThreads, kStripCtas)
-    resize_strip_kernel(const __grid_constant__ LaunchParams p, const __grid_constant__ StripPlan plan) {
+    resize_strip_kernel(
+        const __grid_constant__ LaunchParams p, const __grid_constant__ StripPlan plan,
+        const __grid_constant__ Records<K> records) {
   extern __shared__ __align__(64) unsigned char smem_raw[];
   constexpr int CO = GRAY ? 1 : C;
   unsigned t = blockIdx.x;
@@ -598,7 +600,7 @@ __global__ void __launch_bounds__(kStripThreads, kStripCtas)
     const bool mixed = t < plan.mixed_blocks;
     const unsigned fills = mixed ? (unsigned)((unsigned long long)t * plan.fill_ratio >> 32) : t - plan.walks;
     if (!mixed || (unsigned)((unsigned long long)(t + 1) * plan.fill_ratio >> 32) != fills) {
-      pad_below_any<kStripThreads>(p, fills);
+      pad_below_any<kStripThreads>(p, records, fills);
       return;
     }
     t -= fills;
@@ -614,7 +616,7 @@ __global__ void __launch_bounds__(kStripThreads, kStripCtas)
   } else {
     t = blockIdx.z;
   }
-  const DevSample& s = p.samples[t];
+  const DevSample& s = *records.of(p, t);
   if (s.mode != kModeResize) {
     return;   // the other kernels'
   }
@@ -663,28 +665,30 @@ __global__ void __launch_bounds__(kStripThreads, kStripCtas)
 constexpr size_t kStripMaxSmem =
     strip_layout(4, StripPlan{kStripMaxPx, kStripMaxTaps, kStripMaxSteps, kStripSlots, 0, 0, 0, 0, 0, 0}, 0u, nullptr);
 
-template <int C, bool GRAY, bool U8, bool OWN>
+template <int C, bool GRAY, bool U8, bool OWN, int K>
 cudaError_t launch_kernel(
-    const LaunchParams& p, const StripPlan& plan, dim3 blocks, size_t smem, cudaStream_t stream) {
+    const LaunchParams& p, const StripPlan& plan, dim3 blocks, size_t smem, const Records<K>& records, cudaStream_t stream) {
   // More than the 48 KB that every kernel may have is asked for.  The limit belongs to
   // the kernel on the current device and is shared by all host threads, so each of
   // them sets the same value: one that set its own launch's need could lower the
   // limit between another's setting and its launch.
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(
-        resize_strip_kernel<C, GRAY, U8, OWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStripMaxSmem);
+        resize_strip_kernel<C, GRAY, U8, OWN, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStripMaxSmem);
     if (e != cudaSuccess) {
       return e;
     }
   }
-  resize_strip_kernel<C, GRAY, U8, OWN><<<blocks, kStripThreads, smem, stream>>>(p, plan);
+  resize_strip_kernel<C, GRAY, U8, OWN, K><<<blocks, kStripThreads, smem, stream>>>(p, plan, records);
   return cudaGetLastError();
 }
 
 template <int C, bool GRAY, bool U8>
 cudaError_t launch(const LaunchParams& p, const StripPlan& plan, dim3 blocks, size_t smem, cudaStream_t stream) {
-  return plan.cells_y == 0 ? launch_kernel<C, GRAY, U8, true>(p, plan, blocks, smem, stream)
-                           : launch_kernel<C, GRAY, U8, false>(p, plan, blocks, smem, stream);
+  return with_records(p, [&](const auto& records) {
+    return plan.cells_y == 0 ? launch_kernel<C, GRAY, U8, true>(p, plan, blocks, smem, records, stream)
+                             : launch_kernel<C, GRAY, U8, false>(p, plan, blocks, smem, records, stream);
+  });
 }
 
 } // namespace

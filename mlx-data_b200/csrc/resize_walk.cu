@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
   if (p.pad_apart && p.fill_every > 0) {   // (0: the other resize kernel fills)
     const unsigned fills = (unsigned)p.n * kPadChunks, every = (unsigned)p.fill_every;
     if (t % every == 0 && t / every < fills) {
-      pad_below_any<kWalkThreads>(p, t / every);
+      pad_below_any<kWalkThreads>(p, Records<0>(), t / every);
       return;
     }
     t -= min(t / every + 1, fills);
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
   t /= p.walk.cells_x;
   int cx = (int)cell;
   int cy = OWN ? 0 : (int)(t % p.walk.cells_y);
-  const DevSample& s = p.samples[OWN ? t : t / p.walk.cells_y];
+  const DevSample& s = *Records<0>().of(p, OWN ? t : t / p.walk.cells_y);
   if (s.mode != kModeResizeWide) {
     return;   // the other kernels'
   }
