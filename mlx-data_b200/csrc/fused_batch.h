@@ -78,15 +78,15 @@ struct __align__(16) DevSample {
       float stage_cost;             // the planner's, of four output rows of a strip
     };
   };
-  int32_t walk_part;      // resize_strip.cu: output rows whose source rows are in shared memory together, 1, 2 or 4
+  // resize_strip.cu: output rows whose source rows are in shared memory together (1, 2 or 4), those
+  // source rows << 8, and steps of a warp's walk << 16, at most
+  int32_t walk_sizes;
 };
 
 // What the resize kernel of one launch is sized by: the largest needs of its samples.
 struct StripPlan {
-  int32_t columns;    // columns of the widest strip, a multiple of 32 (0: no sample runs the kernel)
-  int32_t taps;       // horizontal weights of a strip
+  int32_t bytes;      // shared memory of a strip, without cast tables (0: no sample runs the kernel)
   int32_t steps;      // steps of a warp's walk
-  int32_t slots;      // source rows of a part
   int32_t cells_y;    // grid of cells of every sample, the most rows and the most columns of any of them;
   int32_t cells_x;    // or 0 rows: cells_x CTAs per sample, which counts its own cells off
   // with LaunchParams::pad_apart, set at launch: CTAs that walk; the first blocks, which hold
@@ -221,10 +221,6 @@ Mode resize_mode(DevSample& s, int channels);
 // the launches.
 void plan_resize(DevSample* samples, int n, int channels, ResizePlan& plan);
 
-// Which kernels a launch needs and their grids; call after plan_resize with the
-// host copy of the sample table.
-void choose_kernels(LaunchParams& p, ResizePlan& plan, const DevSample* host_samples, int n);
-
 // Samples by which the distance of two taps of an axis of n source samples can exceed
 // its exact value, beyond the one that the bounds below always add: a tap's position
 // goes through at most four float32 roundings (and the ratio's), each of them half a
@@ -232,6 +228,55 @@ void choose_kernels(LaunchParams& p, ResizePlan& plan, const DevSample* host_sam
 __host__ __device__ constexpr int32_t axis_slack(int32_t n) {
   return n >> 21;
 }
+
+// Shared memory of a CTA of resize_strip.cu, laid out for its own sample: in an unlike batch
+// the samples have their largest needs in different places, and every CTA has room for the
+// largest sum.  256 of 256-800 px to 224x224: 51 KB with room for the largest of each, 44.7 so, of which
+// five fit an SM: 113.3 us a pass and 105.4.
+struct StripSmem {
+  unsigned mid;      // per warp: float4 [256]
+  unsigned lut;      // float [tables][256]
+  unsigned ring;     // per warp: source rows [slots]
+  unsigned weights;  // per warp: {wa, wa, wb, wb} per step
+  unsigned places;   // per warp: {address of lane 0's word A, funnel shift} per step
+  unsigned parts;    // per warp: {first, last source row} per part
+  unsigned hx;       // {tap offset | taps << 16, column} per column
+  unsigned hw;       // float [tap][columns]
+  unsigned count;    // per warp: byte [kStripMaxRows]  steps of every output row
+  unsigned ring_bytes, parts_bytes;
+  int steps, slots, part_rows;
+};
+
+constexpr unsigned kStripSlotBytes = 272;                // a row's 16 units of 16 bytes, and the word behind them
+constexpr unsigned kStripMidBytes = 256 * 16;            // four rows of 256 byte columns
+
+__host__ __device__ inline unsigned strip_layout(const DevSample& s, int tables, unsigned base, StripSmem* out) {
+  constexpr unsigned kWarps = kStripThreads / 32;
+  StripSmem sm;
+  sm.steps = s.walk_sizes >> 16;
+  sm.slots = (s.walk_sizes >> 8) & 255;
+  sm.part_rows = s.walk_sizes & 255;
+  sm.ring_bytes = (unsigned)sm.slots * kStripSlotBytes;
+  sm.parts_bytes = (unsigned)s.walk_rows * 8u >> (sm.part_rows >> 1);   // (walk_rows is a multiple of four)
+  const unsigned columns = (unsigned)(s.walk_px + 31) / 32 * 32;
+  sm.mid = base;
+  sm.lut = sm.mid + kWarps * kStripMidBytes;
+  sm.ring = sm.lut + (unsigned)tables * 1024u;
+  sm.weights = sm.ring + kWarps * sm.ring_bytes;
+  sm.places = sm.weights + kWarps * (unsigned)sm.steps * 16u;
+  sm.parts = sm.places + kWarps * (unsigned)sm.steps * 8u;
+  sm.hx = sm.parts + kWarps * sm.parts_bytes;
+  sm.hw = sm.hx + columns * 8u;
+  sm.count = sm.hw + columns * (unsigned)s.cap_x * 4u;
+  if (out) {
+    *out = sm;
+  }
+  return (sm.count + kWarps * kStripMaxRows + 15u - base) & ~15u;
+}
+
+// Which kernels a launch needs and their grids; call after plan_resize with the
+// host copy of the sample table.
+void choose_kernels(LaunchParams& p, ResizePlan& plan, const DevSample* host_samples, int n);
 
 // Conservative per-axis bounds used by the host planner.
 struct AxisPlan {

@@ -484,7 +484,7 @@ cudaError_t launch_fused_batch(const LaunchParams& described, const ResizePlan& 
     // has fewer: 128 images of 32x32 to 224x224 take 33.2 us with the table, 34.7 without.
     p.cast.mode = kCastTable;
   }
-  const bool strips = plan.strip.columns > 0, wides = plan.wide.px > 0;
+  const bool strips = plan.strip.bytes > 0, wides = plan.wide.px > 0;
   if (p.pad_apart && !strips && !wides) {   // a resize kernel fills the padding itself
     const cudaError_t e = with_records(p, [&](const auto& records) {
       launch_fill(p, records, stream);

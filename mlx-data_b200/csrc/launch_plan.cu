@@ -154,10 +154,11 @@ static int strip_most_px(const DevSample& s, int channels) {
 // Bound on the source rows that `rows` output rows read.
 static int strip_span(const DevSample& s, int rows) {
   const float ratio = s.axis_y[0];
-  return (int)std::min(1e6f, (float)(rows - 1) * ratio + 2.0f * std::max(1.0f, ratio)) + 2 + axis_slack(s.pre_h);
+  const float span = (float)(rows - 1) * ratio + 2.0f * (ratio > 1.0f ? ratio : 1.0f);
+  return (int)(span < 1e6f ? span : 1e6f) + 2 + axis_slack(s.pre_h);
 }
 
-// walk_steps() from the ratio in the sample's record.
+// Bound on the steps of a walk over `rows` output rows (launch_plan.cu: walk_steps).
 static int strip_steps(const DevSample& s, int rows) {
   const int slack = axis_slack(s.pre_h);
   if (s.pre_h <= s.geom_h) {
@@ -249,10 +250,8 @@ static void split_walk(DevSample& s, int channels, int px, int rows) {
 
 static void plan_strips(DevSample* samples, int n, StripPlan& plan) {
   constexpr int kWarps = kStripThreads / 32;
-  // (An unlike batch, whose samples have their largest needs in different places, can take
-  // more than the 45.6 KB a CTA that five an SM leave: 256 of 256-800 px to 224x224 take 51,
-  // of which four fit.  Planned for four places they take as long, 117.1 us and 117.0, with
-  // walks cut until five fit 138.8.)
+  // (Five CTAs an SM leave 45.7 KB each, which a batch of strong shrinks down the rows among many
+  // taps can still exceed; walks cut until five fit took 138.8 us where four took 117.)
   constexpr float kWarpsAtOnce = 148 * kStripCtas * kWarps;
   plan = StripPlan{};
   double total = 0.0;
@@ -268,16 +267,13 @@ static void plan_strips(DevSample* samples, int n, StripPlan& plan) {
         s.axis_y[0] == last->axis_y[0]) {
       s.walk_px = last->walk_px;
       s.walk_chunks = last->walk_chunks;
-      s.walk_part = last->walk_part;
+      s.walk_sizes = last->walk_sizes;
       s.stage_cost = last->stage_cost;
     } else {
       split_strips(s);
-      s.walk_part = strip_span(s, 4) <= kStripSlots ? 4 : strip_span(s, 2) <= kStripSlots ? 2 : 1;
-      plan.slots = std::max(plan.slots, strip_span(s, s.walk_part));
+      const int part = strip_span(s, 4) <= kStripSlots ? 4 : strip_span(s, 2) <= kStripSlots ? 2 : 1;
+      s.walk_sizes = part | strip_span(s, part) << 8;
     }
-    const int columns = (s.walk_px + 31) / 32 * 32;
-    plan.columns = std::max(plan.columns, columns);
-    plan.taps = std::max(plan.taps, columns * s.cap_x);
     total += (double)(s.walk_chunks * ((s.post_h + 3) / 4)) * s.stage_cost;
     last = &s;
     last_most = most;
@@ -298,6 +294,7 @@ static void plan_strips(DevSample* samples, int n, StripPlan& plan) {
     long long ctas = 0;
     bool longest = true;
     plan.steps = 0;
+    plan.bytes = 0;
     int stages = 0, post_h = 0, even = 0, down = 0;   // of the sample before
     for (int i = 0; i < n; i++) {
       DevSample& s = samples[i];
@@ -322,6 +319,8 @@ static void plan_strips(DevSample* samples, int n, StripPlan& plan) {
       }
       s.walk_rows = rows;
       plan.steps = std::max(plan.steps, steps);
+      s.walk_sizes = (s.walk_sizes & 0xffff) | steps << 16;
+      plan.bytes = std::max(plan.bytes, (int32_t)strip_layout(s, 0, 0u, nullptr));
       ctas += s.walk_chunks * (long long)(rows == even ? down : (post_h + rows * kWarps - 1) / (rows * kWarps));
     }
     // A small batch: whole CTAs make the one round a little more than one, which takes as

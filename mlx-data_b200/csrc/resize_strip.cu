@@ -49,50 +49,8 @@ namespace mlxd {
 namespace {
 
 constexpr int kWarps = kStripThreads / 32;
-constexpr unsigned kSlotBytes = 272;                // a row's 16 units of 16 bytes, and the word behind them
-constexpr unsigned kMidBytes = 256 * 16;            // four rows of 256 byte columns
+constexpr unsigned kSlotBytes = kStripSlotBytes, kMidBytes = kStripMidBytes;
 constexpr float kScaleY = 0x1p127f, kScaleX = 0x1p22f;
-
-struct StripSmem {
-  unsigned mid;      // per warp: float4 [256]
-  unsigned ring;     // per warp: source rows [slots]
-  unsigned lut;      // float [table_channels][256]
-  unsigned weights;  // per warp: {wa, wa, wb, wb} per step
-  unsigned places;   // per warp: {address of lane 0's word A, funnel shift} per step
-  unsigned count;    // per warp: byte [kStripMaxRows]  steps of every output row
-  unsigned parts;    // per warp: {first, last source row} [kStripMaxRows]
-  unsigned hx;       // {tap offset | taps << 16, column} per column
-  unsigned hw;       // float [tap][columns]
-  unsigned ring_bytes;
-};
-
-__host__ __device__ constexpr size_t strip_layout(int tables, const StripPlan& w, unsigned base, StripSmem* out) {
-  StripSmem sm{};
-  size_t off = 0;
-  sm.mid = base;
-  off += kWarps * kMidBytes;
-  sm.ring = base + (unsigned)off;
-  sm.ring_bytes = (unsigned)w.slots * kSlotBytes;
-  off += kWarps * sm.ring_bytes;
-  sm.lut = base + (unsigned)off;
-  off += (size_t)tables * 1024;
-  sm.weights = base + (unsigned)off;
-  off += (size_t)kWarps * w.steps * 16;
-  sm.places = base + (unsigned)off;
-  off += (size_t)kWarps * w.steps * 8;
-  sm.parts = base + (unsigned)off;
-  off += kWarps * kStripMaxRows * 8;
-  sm.count = base + (unsigned)off;
-  off += kWarps * kStripMaxRows;
-  sm.hx = base + (unsigned)off;
-  off += (size_t)w.columns * 8;
-  sm.hw = base + (unsigned)off;
-  off += (size_t)w.taps * 4;
-  if (out) {
-    *out = sm;
-  }
-  return (off + 15) & ~(size_t)15;
-}
 
 __device__ __forceinline__ void copy16(unsigned dst, uintptr_t src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -396,13 +354,13 @@ __device__ __forceinline__ void walk_cell(
   const int common = shifted ? 0 : (int)(g0 & 3);
   Strip c;
   c.passes = (nc + 31) >> 5;
-  if (wbytes > kStripRow || c.passes * 32 > plan.columns || c.passes * 32 * s.cap_x > plan.taps) {
+  if (wbytes > kStripRow) {
     if (tid == 0) {
       atomicOr(p.status, 8);
     }
     return;
   }
-  c.part_rows = s.walk_part;
+  c.part_rows = sm.part_rows;
   c.mid = sm.mid + (unsigned)warp * kMidBytes;
   c.hx = sm.hx;
   c.hw = sm.hw;
@@ -424,9 +382,9 @@ __device__ __forceinline__ void walk_cell(
   k.from = (int)unit - wbytes;
   k.dst = ring + (unsigned)(lane >> 4) * kSlotBytes + unit;
   k.lane4 = (unsigned)lane * 4u;
-  k.tp = sm.weights + (unsigned)(warp * plan.steps) * 16u;
-  k.ip = sm.places + (unsigned)(warp * plan.steps) * 8u;
-  k.part = sm.parts + (unsigned)warp * (kStripMaxRows * 8u);
+  k.tp = sm.weights + (unsigned)(warp * sm.steps) * 16u;
+  k.ip = sm.places + (unsigned)(warp * sm.steps) * 8u;
+  k.part = sm.parts + (unsigned)warp * sm.parts_bytes;
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     k.sel[j] = 0x4440u + (unsigned)(j ^ ((lane >> 1) & 3));
@@ -463,7 +421,7 @@ __device__ __forceinline__ void walk_cell(
       const int t = __shfl_up_sync(0xffffffffu, sum, d);
       sum += lane >= d ? t : 0;
     }
-    bad = __any_sync(0xffffffffu, lane < rows && (sum > plan.steps || part_last - part_first >= plan.slots || own > 255));
+    bad = __any_sync(0xffffffffu, lane < rows && (sum > min(sm.steps, plan.steps) || part_last - part_first >= sm.slots || own > 255));
     if (!bad) {
       fetch_rows(k, __shfl_sync(0xffffffffu, part_first, 0), __shfl_sync(0xffffffffu, part_last, 0));
       if (lane < rows) {
@@ -644,7 +602,7 @@ __global__ void __launch_bounds__(kStripThreads, kStripCtas)
   const int fill_y1 = p.pad_apart ? vy1 : y1;         // rows below the post window are the fill CTAs' then
   if (!pad && y0 < vy1) {
     StripSmem sm;
-    strip_layout(table_channels(p), plan, smem_addr(smem_raw), &sm);
+    strip_layout(s, table_channels(p), smem_addr(smem_raw), &sm);
     walk_cell<C, GRAY, U8>(s, p, plan, sm, y0, vy1, x0, x1);
   }
   if (fill_y0 < fill_y1) {
@@ -662,8 +620,8 @@ __global__ void __launch_bounds__(kStripThreads, kStripCtas)
 }
 
 // No plan needs more shared memory than this.
-constexpr size_t kStripMaxSmem =
-    strip_layout(4, StripPlan{kStripMaxPx, kStripMaxTaps, kStripMaxSteps, kStripSlots, 0, 0, 0, 0, 0, 0}, 0u, nullptr);
+constexpr size_t kStripMaxSmem = kWarps * (kMidBytes + kStripSlots * kSlotBytes + kStripMaxSteps * 24u + kStripMaxRows * 9u) +
+    4 * 1024 + kStripMaxPx * 8 + kStripMaxTaps * 4;
 
 template <int C, bool GRAY, bool U8, bool OWN, int K>
 cudaError_t launch_kernel(
@@ -718,7 +676,7 @@ cudaError_t launch_resize_strip(const LaunchParams& p, const StripPlan& plan_in,
   // Blocks name their cell by three coordinates, which saves two divisions, where they can.
   plan.linear = p.pad_apart || plan.cells_y == 0 || plan.cells_y > 65535 || p.n > 65535;
   const dim3 b = plan.linear ? dim3((unsigned)blocks) : dim3((unsigned)plan.cells_x, (unsigned)plan.cells_y, (unsigned)p.n);
-  const size_t smem = strip_layout(table_channels(p), plan, 0u, nullptr);
+  const size_t smem = (size_t)plan.bytes + (size_t)table_channels(p) * 1024;
   if (p.out_f32) {
     if (p.gray) {
       return launch<3, true, false>(p, plan, b, smem, stream);
