@@ -6,6 +6,7 @@
 #include <emmintrin.h>
 #include <sched.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -679,6 +680,7 @@ int enqueue_on_lane(
   const bool timed = ctx->timing.load() != 0;
   lane.in_timed[slot] = false;
   lane.out_timed[slot] = false;
+  bool sent_early = false;   // all sources are on their way already
   if (bounce) {
     // Pack the rectangles of the pageable sources into the lane's page-locked
     // block (the calling thread does the copying), then one copy for all of
@@ -693,23 +695,55 @@ int enqueue_on_lane(
     // batch take samples off a shared counter; packing is plain row copies.
     std::atomic<int> next{0};
     uint8_t* const block = static_cast<uint8_t*>(lane.h_src.ptr);
-    auto pack = [&]() {
+    // Where all sources are packed, the calling thread sends off what is ready between its
+    // own samples, in parts of two megabytes, so that the copy runs beside the packing.  One batch
+    // of 32 images of 256-640 px (12.3 MB): 905 us, 797 so; two of 48 1425 and 1180; four lanes at
+    // once, which fill each other's gaps, 2508 and 2450.
+    constexpr size_t kPart = size_t(2) << 20;
+    sent_early = !timed && stage_bytes >= 2 * kPart && std::find(direct_copy.begin(), direct_copy.end(), 1) == direct_copy.end();
+    const std::unique_ptr<std::atomic<bool>[]> packed(new std::atomic<bool>[n]());
+    int sent = 0;
+    size_t sent_bytes = 0;
+    cudaError_t sending = cudaSuccess;
+    auto send = [&](size_t least) {
+      int ready = sent;
+      while (ready < n && packed[ready].load(std::memory_order_acquire)) {
+        ready++;
+      }
+      const size_t end = ready == n ? stage_bytes : pieces[ready].offset;
+      if (sending == cudaSuccess && end >= sent_bytes + least) {
+        sending = cudaMemcpyAsync(
+            static_cast<uint8_t*>(lane.d_src.ptr) + sent_bytes, block + sent_bytes, end - sent_bytes, cudaMemcpyHostToDevice,
+            lane.stream);
+        sent = ready;
+        sent_bytes = end;
+      }
+    };
+    auto pack = [&](bool caller) {
       for (int i = next.fetch_add(1); i < n; i = next.fetch_add(1)) {
         if (direct_copy[i]) {
           continue;
         }
         pack_rows(block + pieces[i].offset, pieces[i].from, pieces[i].from_pitch, pieces[i].row_bytes, pieces[i].rows);
+        packed[i].store(true, std::memory_order_release);
+        if (caller && sent_early) {
+          send(kPart);
+        }
       }
     };
     const int helpers = stage_bytes >= (size_t(8) << 20) ? std::min(pack_threads() - 1, n - 1) : 0;
     std::vector<std::thread> crew;
     crew.reserve(helpers > 0 ? helpers : 0);
     for (int t = 0; t < helpers; t++) {
-      crew.emplace_back(pack);
+      crew.emplace_back(pack, false);
     }
-    pack();
+    pack(true);
     for (auto& th : crew) {
       th.join();
+    }
+    if (sent_early) {
+      send(1);
+      MLXD_CUDA(sending);
     }
     ctx->host_stage_ns += (uint64_t)std::chrono::duration_cast<std::chrono::nanoseconds>(
         std::chrono::steady_clock::now() - t0).count();
@@ -733,7 +767,9 @@ int enqueue_on_lane(
     for (int i = 0; i < n; i++) {
       all_bounced = all_bounced && !direct_copy[i];
     }
-    if (all_bounced) {
+    if (sent_early) {
+      // (nothing is left)
+    } else if (all_bounced) {
       MLXD_CUDA(cudaMemcpyAsync(lane.d_src.ptr, lane.h_src.ptr, stage_bytes, cudaMemcpyHostToDevice, lane.stream));
     } else {
       for (int i = 0; i < n; i++) {
