@@ -12,16 +12,16 @@
 // 2^-30, which reaches a whole number from below only where f itself is the whole distance:
 // -2^-26 < f < 0 beside a whole c.  A warp that meets such an f takes the doubles.
 //
-// What bounds it (128 images of 512x512x3, an angle each, 448x448 floats: 102.5 us, 113 in
-// bands of CTA-wide 16x64-pixel tiles, four neighbouring pixels a lane): the latency of the
-// loads at 24 warps an SM, the L1 pipe 60 % busy, DRAM 3.4 TB/s.  The tiles' loads met 5.4
+// What bounds it (128 images of 512x512x3, an angle each, 448x448 floats: 102.5 us, 92.5 with the
+// records as parameters, 113 in bands of CTA-wide 16x64-pixel tiles, four neighbouring pixels a
+// lane): the latency of the loads at 24 warps an SM, the L1 pipe 60 % busy, DRAM 3.4 TB/s.  The tiles' loads met 5.4
 // times in the banks (3 here), their stores brought sectors to L2 by halves (15.2 M sectors, 9.6 here),
-// and the coordinate took double additions and 64-bit conversions (25 % of that pipe, now
-// 16).  Bytes through shared memory make all stores whole lines whatever the row starts
+// and the coordinate took double additions and 64-bit conversions.  Bytes through shared memory make all stores whole lines whatever the row starts
 // at: 128 of 511x511x3 to 447x447 109.7 us, 128 before; four channels 107 and 160, one
 // channel 53.7 and 73.7, bytes 70 and 88.  Without the next words under way: 107 us; two rows of
 // 16 pixels a load 107 to 112; eight by four with 8-byte loads 143.
 #include <algorithm>
+#include <type_traits>
 
 #include "fused_batch.h"
 #include "kernel_common.cuh"
@@ -316,7 +316,9 @@ __global__ void __launch_bounds__(kAffineThreads, kAffineCtas)
   t /= bands_x;
   const int y0 = (int)(t % p.tiles_y) * kTileH;
   const DevSample* const sample = records.of(p, t / p.tiles_y);
-  const DevSample& s = *sample;
+  // (a record of the table is copied whole, in one wait: 200 images of 512x512 146 us, 153 field by
+  // field; one of the parameters is read as constants: 128 images 92.5 us, 97 copied)
+  typename std::conditional<K == 0, const DevSample, const DevSample&>::type s = *sample;
   if (s.mode != kModeAffine) {
     return;   // the other kernels'
   }

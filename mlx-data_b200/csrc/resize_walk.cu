@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
   t /= p.walk.cells_x;
   int cx = (int)cell;
   int cy = OWN ? 0 : (int)(t % p.walk.cells_y);
-  const DevSample& s = *Records<0>().of(p, OWN ? t : t / p.walk.cells_y);
+  const DevSample& s = p.samples[p.first + (OWN ? t : t / p.walk.cells_y)];
   if (s.mode != kModeResizeWide) {
     return;   // the other kernels'
   }
