@@ -14,12 +14,13 @@
 //
 // What bounds it (128 images of 512x512x3, an angle each, 448x448 floats: 102.5 us, 92.5 with the
 // records as parameters, 113 in bands of CTA-wide 16x64-pixel tiles, four neighbouring pixels a
-// lane): the latency of the loads at 24 warps an SM, the L1 pipe 60 % busy, DRAM 3.4 TB/s.  The tiles' loads met 5.4
-// times in the banks (3 here), their stores brought sectors to L2 by halves (15.2 M sectors, 9.6 here),
-// and the coordinate took double additions and 64-bit conversions.  Bytes through shared memory make all stores whole lines whatever the row starts
-// at: 128 of 511x511x3 to 447x447 109.7 us, 128 before; four channels 107 and 160, one
-// channel 53.7 and 73.7, bytes 70 and 88.  Without the next words under way: 107 us; two rows of
-// 16 pixels a load 107 to 112; eight by four with 8-byte loads 143.
+// lane): the latency of the loads at 24 warps an SM, the L1 pipe 60 % busy, DRAM 3.8 TB/s.
+// The tiles' loads met 5.6 times in the banks (3 here), their stores brought sectors to L2
+// by halves (15.2 M sectors, 9.6 here), and the coordinate took double additions and 64-bit
+// conversions.  Bytes through shared memory make all stores whole lines whatever the row
+// starts at: 128 of 511x511x3 to 447x447 109.7 us, 128 before; four channels 107 and 160,
+// one channel 53.7 and 73.7, bytes 70 and 88.  Without the next words under way: 107 us;
+// two rows of 16 pixels a load 107 to 112; eight by four with 8-byte loads 143.
 #include <algorithm>
 #include <type_traits>
 
