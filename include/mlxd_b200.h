@@ -141,8 +141,8 @@ MLXD_API const char* mlxd_last_error(void);
  * page-locked memory that did not come from here goes through the copy engines,
  * and sources in ordinary (pageable) memory are first packed - needed rectangle
  * only - into a page-locked block of the lane by the calling thread and up to
- * MLXD_PACK_THREADS - 1 helpers (default 4 threads in all), then copied once
- * per batch.  MLXD_HOST_GATHER=0 in the environment turns the kernel path off. */
+ * MLXD_PACK_THREADS - 1 helpers (default 4 threads in all) and copied, large
+ * batches in parts while the rest is being packed.  MLXD_HOST_GATHER=0 in the environment turns the kernel path off. */
 MLXD_API void* mlxd_pinned_alloc(size_t bytes);
 MLXD_API void mlxd_pinned_free(void* p);
 
@@ -219,7 +219,8 @@ MLXD_API int mlxd_batch_wait(mlxd_ctx* ctx, int lane, int timeout_ms);
 
 /* Same work for device-resident sources and destination, launched on the
  * caller's CUDA stream (a cudaStream_t passed as void*; NULL is the default
- * stream).  Nothing is copied except the descriptors.
+ * stream).  Nothing is copied except the descriptors (those of up to 128 samples
+ * travel with the launch).
  *
  * A stream under capture gets the call as nodes of the graph: the descriptors become
  * the graph's own, in an allocation node, so such a graph follows the rules of graphs
