@@ -12,7 +12,7 @@ namespace {
 
 thread_local std::string g_last;
 
-// int32 words between the self-check words of two lanes
+// int32 words between the status words of two lanes
 constexpr size_t kStatusStride = 16;
 
 void destroy_lane(Lane* l) {
@@ -56,12 +56,12 @@ int make_lane(Lane** out) {
     if (e == cudaSuccess) e = cudaEventCreate(&l->in_begin[s]);
     if (e == cudaSuccess) e = cudaEventCreate(&l->out_end[s]);
   }
-  if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&l->h_status), sizeof(int32_t), cudaHostAllocDefault);
+  if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&l->h_status), kStatusWords * sizeof(int32_t), cudaHostAllocDefault);
   if (e != cudaSuccess) {
     destroy_lane(l);
     return fail_cuda(e, "lane setup");
   }
-  *l->h_status = 0;
+  l->h_status[0] = l->h_status[1] = 0;
   *out = l;
   return MLXD_OK;
 }

@@ -809,11 +809,11 @@ int enqueue_on_lane(
       lane.out_timed[slot] = true;
     }
   }
-  *lane.h_status = kStatusPending;
+  lane.h_status[1] = 1;
   const cudaError_t brought =
-      cudaMemcpyAsync(lane.h_status, lane.d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, lane.stream);
+      cudaMemcpyAsync(lane.h_status, lane.d_status, kStatusWords * sizeof(int32_t), cudaMemcpyDeviceToHost, lane.stream);
   if (brought != cudaSuccess) {
-    *lane.h_status = 0;
+    lane.h_status[1] = 0;
     return fail_cuda(brought, "cudaMemcpyAsync(status)");
   }
   MLXD_CUDA(cudaEventRecord(lane.done, lane.stream));
@@ -862,10 +862,10 @@ int wait_lane(mlxd_ctx* ctx, Lane& lane, int timeout_ms) {
   if (timeout_ms < 0) {
     // No deadline.  Blocked in the driver a thread wakes 200 us and more after the GPU's
     // interrupt (a virtual machine's processor sleeps meanwhile), so it first looks a while at
-    // the word that the lane's last copy brings (kStatusPending until then), without asking
-    // the driver from every lane.  One batch of 8 full-HD frames 1027 us, 696 so.
-    const volatile int32_t* const word = lane.h_status;
-    for (int i = 0; *word == kStatusPending; i++) {
+    // the word that the lane's last copy clears, without asking the driver from every lane.
+    // One batch of 8 full-HD frames 1027 us, 696 so.
+    const volatile int32_t* const under_way = lane.h_status + 1;
+    for (int i = 0; *under_way != 0; i++) {
       _mm_pause();
       if (i % 64 == 63) {
         if (std::chrono::steady_clock::now() - start > std::chrono::microseconds(kLookMicroseconds)) {
@@ -874,9 +874,9 @@ int wait_lane(mlxd_ctx* ctx, Lane& lane, int timeout_ms) {
         sched_yield();
       }
     }
-    // (the event is next; with several batches in flight on the lane the word may be an earlier one's)
+    // (the event is next; with several batches in flight on the lane the word may be cleared by an earlier one)
     cudaError_t e = cudaErrorNotReady;
-    for (int i = 0; i < 64 && e == cudaErrorNotReady && *word != kStatusPending; i++) {
+    for (int i = 0; i < 64 && e == cudaErrorNotReady && *under_way == 0; i++) {
       e = cudaEventQuery(lane.done);
     }
     if (e != cudaSuccess) {

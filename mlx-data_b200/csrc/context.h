@@ -65,7 +65,7 @@ struct Arena {
 };
 
 constexpr int kDescSlots = 4;
-constexpr int32_t kStatusPending = INT32_MIN;   // no status of a kernel
+constexpr int kStatusWords = 2;                 // of a lane: its kernels' status, and one that is 0 on the device
 constexpr int kLookMicroseconds = 3000;         // a thread looks for the status so long before it blocks
 
 struct Lane {
@@ -86,8 +86,11 @@ struct Lane {
   bool in_timed[kDescSlots] = {};
   bool out_timed[kDescSlots] = {};
   int next_slot = 0;
-  int32_t* d_status = nullptr;        // this lane's word of the context's status block
-  int32_t* h_status = nullptr;        // pinned copy of the device status word, kStatusPending while it is under way
+  int32_t* d_status = nullptr;        // this lane's words of the context's status block
+  // Pinned copy of both.  The second is set when a batch queues it, so a thread that waits sees
+  // there, without asking the driver, that a copy has come.  Where another caller has queued
+  // since it does not say which, so the event decides; the first is a kernel's status at any time.
+  int32_t* h_status = nullptr;
   std::mutex mu;                      // one caller at a time per lane
 };
 

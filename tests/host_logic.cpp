@@ -1,0 +1,222 @@
+// The host side of the C ABI (context.cu, api.cu, launch_plan.cu, noalloc.cu) against a CUDA
+// runtime made up here: device memory is host memory, a stream is a list of work that runs when
+// it is waited for, kernels are functions below.  So what a call queues, and what another caller
+// does in between, is the same in every run, and calls can be made to fail.
+//
+// Usage: host_logic SCENARIO; exits with 0 if it holds, else prints what does not.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <deque>
+#include <functional>
+#include <map>
+#include <string>
+#include <vector>
+
+#include "context.h"
+
+using namespace mlxd;
+
+// ---------------------------------------------------------------- the runtime
+struct CUstream_st {
+  std::deque<std::function<void()>> work;
+  uint64_t queued = 0, done = 0;
+};
+struct CUevent_st {
+  CUstream_st* stream = nullptr;
+  uint64_t at = 0;
+};
+
+namespace {
+
+std::vector<std::string> calls;              // what was queued and waited for, in order
+std::function<cudaError_t(const std::string&)> before = [](const std::string&) { return cudaSuccess; };
+std::function<void()> looked = [] {};        // after an event was looked at
+std::function<void(const LaunchParams&)> kernel = [](const LaunchParams&) {};
+CUstream_st legacy;
+
+CUstream_st* of(cudaStream_t s) {
+  return s ? s : &legacy;
+}
+
+void queue(cudaStream_t s, std::function<void()> f) {
+  of(s)->work.push_back(std::move(f));
+  of(s)->queued++;
+}
+
+void run(cudaStream_t s) {
+  while (!of(s)->work.empty()) {
+    const auto f = of(s)->work.front();
+    of(s)->work.pop_front();
+    f();
+    of(s)->done++;
+  }
+}
+
+// Notes a call and lets the scenario act before it, or make it fail.
+cudaError_t note(const std::string& what) {
+  calls.push_back(what);
+  return before(what);
+}
+
+#define FAKE(what)                        \
+  const cudaError_t fails__ = note(what); \
+  if (fails__ != cudaSuccess) return fails__
+
+} // namespace
+
+extern "C" {
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+const char* cudaGetErrorString(cudaError_t) { return "made up"; }
+cudaError_t cudaDeviceGetPCIBusId(char* s, int, int) { *s = 0; return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) { *p = std::aligned_alloc(256, (n + 255) & ~size_t(255)); return cudaSuccess; }
+cudaError_t cudaFree(void* p) { std::free(p); return cudaSuccess; }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMalloc(p, n); }
+cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
+cudaError_t cudaHostGetDevicePointer(void** d, void* h, unsigned) { *d = h; return cudaSuccess; }
+cudaError_t cudaHostGetFlags(unsigned*, void*) { return cudaErrorInvalidValue; }   // all of it is pageable
+cudaError_t cudaGetSymbolAddress(void** p, const void* s) { *p = const_cast<void*>(s); return cudaSuccess; }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { std::memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemset(void* d, int v, size_t n) { std::memset(d, v, n); return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = new CUstream_st; return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t s) { delete s; return cudaSuccess; }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* c) { *c = cudaStreamCaptureStatusNone; return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { FAKE("wait stream"); run(s); return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = new CUevent_st; return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t* e) { return cudaEventCreateWithFlags(e, 0); }
+cudaError_t cudaEventDestroy(cudaEvent_t e) { delete e; return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+  FAKE("record");
+  queue(s, [] {});
+  e->stream = of(s);
+  e->at = of(s)->queued;
+  return cudaSuccess;
+}
+cudaError_t cudaEventQuery(cudaEvent_t e) {
+  FAKE("query");
+  const bool ready = !e->stream || e->stream->done >= e->at;
+  if (!ready) {
+    run(e->stream);   // the GPU goes on meanwhile
+  }
+  looked();
+  return ready ? cudaSuccess : cudaErrorNotReady;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+  FAKE("wait event");
+  if (e->stream && e->stream->done < e->at) {
+    run(e->stream);
+  }
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind kind, cudaStream_t stream) {
+  FAKE(kind == cudaMemcpyHostToDevice ? "copy in" : "copy out");
+  queue(stream, [=] { std::memcpy(d, s, n); });
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpy2DAsync(void*, size_t, const void*, size_t, size_t, size_t, cudaMemcpyKind, cudaStream_t) { std::abort(); }
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t stream) {
+  FAKE("set");
+  queue(stream, [=] { std::memset(d, v, n); });
+  return cudaSuccess;
+}
+}
+
+namespace mlxd {
+cudaError_t launch_fused_batch(const LaunchParams& p, const ResizePlan&, cudaStream_t stream) {
+  FAKE(p.samples ? "kernel" : "kernel with records");
+  LaunchParams q = p;
+  queue(stream, [q] { kernel(q); });
+  return cudaSuccess;
+}
+cudaError_t launch_gather_rows(const GatherPiece*, int, uint32_t, cudaStream_t) { std::abort(); }
+int capture_batch(LaunchParams&, const ResizePlan&, const DevSample*, const mlxd_batch_desc*, cudaStream_t) { std::abort(); }
+} // namespace mlxd
+
+// ---------------------------------------------------------------- scenarios
+namespace {
+
+int failures = 0;
+
+void check(bool holds, const char* what, int line) {
+  if (!holds) {
+    std::printf("line %d: %s (%s)\n", line, what, mlxd_last_error());
+    failures++;
+  }
+}
+#define CHECK(x) check((x), #x, __LINE__)
+
+mlxd_ctx* context() {
+  mlxd_ctx* ctx = nullptr;
+  CHECK(mlxd_ctx_create(0, 1, &ctx) == MLXD_OK);
+  return ctx;
+}
+
+mlxd_sample_desc whole(const uint8_t* src, int h, int w) {
+  mlxd_sample_desc d{};
+  d.src = src;
+  d.src_h = d.pre_h = d.geom_h = d.post_h = h;
+  d.src_w = d.pre_w = d.geom_w = d.post_w = w;
+  return d;
+}
+
+mlxd_batch_desc batch_of(void* dst, int h, int w, int c) {
+  mlxd_batch_desc b{};
+  b.dst = dst;
+  b.slot_h = h;
+  b.slot_w = w;
+  b.channels = c;
+  b.out_dtype = MLXD_U8;
+  b.divisor = 1.0f;
+  b.src_mem = b.dst_mem = MLXD_MEM_HOST;
+  return b;
+}
+
+// Another caller queues a batch on a lane at any look of a wait for it.
+void wait_beside_another_caller() {
+  uint8_t src[64 * 3] = {}, dst[2][64 * 3];
+  const mlxd_sample_desc d = whole(src, 8, 8);
+  const mlxd_batch_desc b[2] = {batch_of(dst[0], 8, 8, 3), batch_of(dst[1], 8, 8, 3)};
+  for (const int32_t status : {0, 8}) {
+    for (int step = 1; step <= 4; step++) {
+      mlxd_ctx* ctx = context();
+      kernel = [&](const LaunchParams& p) { *p.status |= status; };
+      CHECK(mlxd_fused_batch(ctx, 0, &d, 1, &b[0]) == MLXD_OK);
+      run(ctx->lanes[0]->stream);
+      kernel = [](const LaunchParams&) {};
+      int left = step;
+      looked = [&] {
+        if (--left == 0) {
+          CHECK(mlxd_fused_batch(ctx, 0, &d, 1, &b[1]) == MLXD_OK);
+        }
+      };
+      const int rc = mlxd_batch_wait(ctx, 0, -1);
+      CHECK(rc == (status ? MLXD_ERR_DEVICE : MLXD_OK));
+      CHECK(!status || std::strstr(mlxd_last_error(), "(status 8)"));
+      looked = [] {};
+      if (!status) {
+        CHECK(mlxd_batch_wait(ctx, 0, -1) == MLXD_OK);
+        CHECK(ctx->lanes[0]->stream->work.empty());
+      }
+      mlxd_ctx_destroy(ctx);
+    }
+  }
+}
+
+} // namespace
+
+int main(int argc, char** argv) {
+  const std::map<std::string, void (*)()> scenarios = {
+      {"wait_beside_another_caller", wait_beside_another_caller},
+  };
+  const auto it = argc == 2 ? scenarios.find(argv[1]) : scenarios.end();
+  if (it == scenarios.end()) {
+    return 2;
+  }
+  it->second();
+  return failures ? 1 : 0;
+}

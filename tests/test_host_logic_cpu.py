@@ -1,0 +1,30 @@
+"""The host side of the C ABI against a CUDA runtime made up in host_logic.cpp: orders of
+calls by two callers, calls that fail, plans, which no GPU is needed for and which a GPU would
+meet by chance."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "mlx-data_b200", "csrc")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+SOURCES = ["context.cu", "api.cu", "launch_plan.cu", "noalloc.cu"]
+
+
+@pytest.fixture(scope="module")
+def program(tmp_path_factory):
+    if not shutil.which("g++") or not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime.h")):
+        pytest.skip("needs g++ and CUDA's headers")
+    out = str(tmp_path_factory.mktemp("host_logic") / "host_logic")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I" + os.path.join(CUDA, "include"), "-I" + CSRC,
+                    "-x", "c++", os.path.join(HERE, "host_logic.cpp")] +
+                   [os.path.join(CSRC, s) for s in SOURCES] + ["-o", out], check=True)
+    return out
+
+
+@pytest.mark.parametrize("scenario", ["wait_beside_another_caller"])
+def test_scenario(program, scenario):
+    r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
