@@ -525,9 +525,12 @@ static void join_copies(DevSample* samples, int n, int channels) {
         samples[i] = s;
         continue;
       }
+      if (s.mode != kModeResize) {   // (a side so long that no strip holds a column: walk_px is 0)
+        return;
+      }
       split_strips(s);
       cost += strip_time(s, channels);
-      if (s.mode != kModeResize || cost > kMost) {
+      if (cost > kMost) {
         return;
       }
     }

@@ -207,11 +207,34 @@ void wait_beside_another_caller() {
   }
 }
 
+// Copies out of sources that no strip can take, beside a resize that runs in strips, stay copies.
+void copies_of_huge_sources_beside_a_resize() {
+  uint8_t src[4] = {}, dst[4];   // (planning reads no pixels)
+  struct Case { int w, channels; bool joins; };
+  for (const Case& k : {Case{1 << 30, 3, false}, Case{(1 << 29) + 5, 4, false}, Case{1 << 29, 1, false}, Case{1 << 28, 4, false},
+                        Case{1 << 27, 4, false}, Case{4000, 3, true}}) {
+    mlxd_sample_desc d[2] = {whole(src, 2, k.w), whole(src, 40, 30)};
+    d[0].post_x = k.w - 9;
+    d[0].post_w = 8;
+    d[1].geom = MLXD_GEOM_RESIZE;
+    d[1].geom_w = d[1].post_w = 8;
+    d[1].geom_h = d[1].post_h = 20;
+    const mlxd_batch_desc b = batch_of(dst, 20, 8, k.channels);
+    DevSample out[2];
+    ResizePlan plan;
+    CHECK(plan_into(d, 2, &b, out, plan) == MLXD_OK);
+    CHECK(out[0].mode == (k.joins ? kModeResize : kModeCopy));
+    CHECK(out[1].mode == kModeResize);
+    CHECK(out[0].post_x == k.w - 9 && out[0].post_w == 8 && out[0].post_h == 2);
+  }
+}
+
 } // namespace
 
 int main(int argc, char** argv) {
   const std::map<std::string, void (*)()> scenarios = {
       {"wait_beside_another_caller", wait_beside_another_caller},
+      {"copies_of_huge_sources_beside_a_resize", copies_of_huge_sources_beside_a_resize},
   };
   const auto it = argc == 2 ? scenarios.find(argv[1]) : scenarios.end();
   if (it == scenarios.end()) {
