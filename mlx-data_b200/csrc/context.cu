@@ -681,6 +681,17 @@ int enqueue_on_lane(
   lane.in_timed[slot] = false;
   lane.out_timed[slot] = false;
   bool sent_early = false;   // all sources are on their way already
+  // A call that fails while copies out of the lane's block are queued waits for them: the next
+  // one writes into it, and src_copied, which it waits for, does not tell of these.
+  struct Drain {
+    cudaStream_t stream;
+    bool armed;
+    ~Drain() {
+      if (armed) {
+        cudaStreamSynchronize(stream);
+      }
+    }
+  } block_in_use{lane.stream, false};
   if (bounce) {
     // Pack the rectangles of the pageable sources into the lane's page-locked
     // block (the calling thread does the copying), then one copy for all of
@@ -690,6 +701,7 @@ int enqueue_on_lane(
       return rc;
     }
     MLXD_CUDA(cudaEventSynchronize(lane.src_copied));
+    block_in_use.armed = true;
     const auto t0 = std::chrono::steady_clock::now();
     // The calling thread and up to pack_threads - 1 helpers started for this
     // batch take samples off a shared counter; packing is plain row copies.
@@ -789,6 +801,7 @@ int enqueue_on_lane(
     }
     if (bounce) {
       MLXD_CUDA(cudaEventRecord(lane.src_copied, lane.stream));
+      block_in_use.armed = false;
     }
     ctx->h2d += stage_bytes;
   }

@@ -229,12 +229,38 @@ void copies_of_huge_sources_beside_a_resize() {
   }
 }
 
+// A copy that fails after others of the same batch were queued: the call ends only when those,
+// which read the lane's block, have run.
+void failed_copy_of_a_part() {
+  const int h = 1100, w = 700, n = 3;   // a part each, packed by the caller alone
+  std::vector<uint8_t> src((size_t)h * w * 3, 7), dst(src.size() * n);
+  std::vector<mlxd_sample_desc> d(n, whole(src.data(), h, w));
+  const mlxd_batch_desc b = batch_of(dst.data(), h, w, 3);
+  for (int bad = 3; bad <= 4; bad++) {   // (the first is the descriptors')
+    mlxd_ctx* ctx = context();
+    int copies = 0;
+    calls.clear();
+    before = [&](const std::string& call) {
+      return call == "copy in" && ++copies == bad ? cudaErrorInvalidValue : cudaSuccess;
+    };
+    CHECK(mlxd_fused_batch(ctx, 0, d.data(), n, &b) == MLXD_ERR_CUDA);
+    before = [](const std::string&) { return cudaSuccess; };
+    CHECK(copies == bad);
+    CHECK(ctx->lanes[0]->stream->work.empty());
+    // and the lane goes on
+    CHECK(mlxd_fused_batch(ctx, 0, d.data(), n, &b) == MLXD_OK);
+    CHECK(mlxd_batch_wait(ctx, 0, -1) == MLXD_OK);
+    mlxd_ctx_destroy(ctx);
+  }
+}
+
 } // namespace
 
 int main(int argc, char** argv) {
   const std::map<std::string, void (*)()> scenarios = {
       {"wait_beside_another_caller", wait_beside_another_caller},
       {"copies_of_huge_sources_beside_a_resize", copies_of_huge_sources_beside_a_resize},
+      {"failed_copy_of_a_part", failed_copy_of_a_part},
   };
   const auto it = argc == 2 ? scenarios.find(argv[1]) : scenarios.end();
   if (it == scenarios.end()) {
