@@ -116,7 +116,8 @@ typedef struct mlxd_stats {
   uint64_t timed_launches;        /* launches included in kernel_ns; 0 unless timing is on */
   uint64_t algo_src_bytes;        /* summed source footprints: the uint8 source rectangle each sample's chain can read */
   uint64_t algo_dst_bytes;        /* summed batch tensor bytes written, padding included */
-  uint64_t h2d_ns;                /* timed launches: device time of the host-to-device stage (gather kernel or copies) */
+  uint64_t h2d_ns;                /* timed launches: device time of the host-to-device stage (gather kernel or copies,
+                                   * from the first of a batch's parts where those go out while the rest is packed) */
   uint64_t d2h_ns;                /* timed launches: device time of the batch's copy back to the host */
   uint64_t host_stage_ns;         /* host time spent copying sources from ordinary memory into page-locked blocks */
 } mlxd_stats;
@@ -220,7 +221,8 @@ MLXD_API int mlxd_batch_wait(mlxd_ctx* ctx, int lane, int timeout_ms);
 /* Same work for device-resident sources and destination, launched on the
  * caller's CUDA stream (a cudaStream_t passed as void*; NULL is the default
  * stream).  Nothing is copied except the descriptors (those of up to 128 samples
- * travel with the launch).
+ * travel with the launch, unless a resize among them runs in one of the kernels for strong
+ * shrinks).
  *
  * A stream under capture gets the call as nodes of the graph: the descriptors become
  * the graph's own, in an allocation node, so such a graph follows the rules of graphs

@@ -315,9 +315,13 @@ int mlxd_fused_batch_on_stream(
     return rc;
   }
   const bool timed = ctx->timing.load() != 0;
-  if (carried_samples(p, plan) && !timed) {
-    // The records go with the launch: no copy ahead of the kernel, nothing of the ring in use.
+  const bool carried = carried_samples(p, plan);
+  if (carried) {
+    // The records go with the launch: no copy ahead of the kernel, nothing of the ring in use
+    // but, when timed, the events of a slot.
     p.carried = dev.get();
+  }
+  if (carried && !timed) {
     MLXD_CUDA(launch_fused_batch(p, plan, stream));
     ctx->batches += 1;
     ctx->samples += n;
@@ -331,28 +335,30 @@ int mlxd_fused_batch_on_stream(
   // means neither the copy nor the kernel still needs the tables.
   MLXD_CUDA(cudaEventSynchronize(ring.desc_copied[slot]));
   harvest_timing(ctx, ring, slot, true);
-  const size_t table_bytes = sizeof(DevSample) * n;
-  rc = arena_reserve(ctx, ring.d_desc[slot], table_bytes, false, nullptr);
-  if (rc != MLXD_OK) {
-    return rc;
-  }
-  // A table of at most 64 KB is taken from ordinary memory: the driver copies it into
-  // the command stream before the call returns, which costs a pass 2 us where a copy
-  // from page-locked memory, started by a copy engine, costs 6 (32 to 240 samples
-  // ahead of a kernel of 20 us; 285 to 390 samples whose kernels take 150 to 220 us: 3 to 4 %
-  // of a pass).  Where the host is the bound it costs up to 2 us more (512 tiny images 27.5
-  // us a pass, 25.2 by the copy engine).
-  const void* table = dev.get();
-  if (table_bytes > 64 * 1024) {
-    rc = arena_reserve(ctx, ring.h_desc[slot], table_bytes, true, nullptr);
+  if (!carried) {
+    const size_t table_bytes = sizeof(DevSample) * n;
+    rc = arena_reserve(ctx, ring.d_desc[slot], table_bytes, false, nullptr);
     if (rc != MLXD_OK) {
       return rc;
     }
-    std::memcpy(ring.h_desc[slot].ptr, dev.get(), table_bytes);
-    table = ring.h_desc[slot].ptr;
+    // A table of at most 64 KB is taken from ordinary memory: the driver copies it into
+    // the command stream before the call returns, which costs a pass 2 us where a copy
+    // from page-locked memory, started by a copy engine, costs 6 (32 to 240 samples
+    // ahead of a kernel of 20 us; 285 to 390 samples whose kernels take 150 to 220 us: 3 to 4 %
+    // of a pass).  Where the host is the bound it costs up to 2 us more (512 tiny images 27.5
+    // us a pass, 25.2 by the copy engine).
+    const void* table = dev.get();
+    if (table_bytes > 64 * 1024) {
+      rc = arena_reserve(ctx, ring.h_desc[slot], table_bytes, true, nullptr);
+      if (rc != MLXD_OK) {
+        return rc;
+      }
+      std::memcpy(ring.h_desc[slot].ptr, dev.get(), table_bytes);
+      table = ring.h_desc[slot].ptr;
+    }
+    MLXD_CUDA(cudaMemcpyAsync(ring.d_desc[slot].ptr, table, table_bytes, cudaMemcpyHostToDevice, stream));
+    p.samples = static_cast<const DevSample*>(ring.d_desc[slot].ptr);
   }
-  MLXD_CUDA(cudaMemcpyAsync(ring.d_desc[slot].ptr, table, table_bytes, cudaMemcpyHostToDevice, stream));
-  p.samples = static_cast<const DevSample*>(ring.d_desc[slot].ptr);
   if (timed) {
     MLXD_CUDA(cudaEventRecord(ring.k_begin[slot], stream));
   }

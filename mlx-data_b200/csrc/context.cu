@@ -712,7 +712,7 @@ int enqueue_on_lane(
     // of 32 images of 256-640 px (12.3 MB): 905 us, 797 so; two of 48 1425 and 1180; four lanes at
     // once, which fill each other's gaps, 2508 and 2450.
     constexpr size_t kPart = size_t(2) << 20;
-    sent_early = !timed && stage_bytes >= 2 * kPart && std::find(direct_copy.begin(), direct_copy.end(), 1) == direct_copy.end();
+    sent_early = stage_bytes >= 2 * kPart && std::find(direct_copy.begin(), direct_copy.end(), 1) == direct_copy.end();
     const std::unique_ptr<std::atomic<bool>[]> packed(new std::atomic<bool>[n]());
     int sent = 0;
     size_t sent_bytes = 0;
@@ -724,7 +724,11 @@ int enqueue_on_lane(
       }
       const size_t end = ready == n ? stage_bytes : pieces[ready].offset;
       if (sending == cudaSuccess && end >= sent_bytes + least) {
-        sending = cudaMemcpyAsync(
+        if (timed && sent == 0) {
+          sending = cudaEventRecord(lane.in_begin[slot], lane.stream);
+          lane.in_timed[slot] = sending == cudaSuccess;
+        }
+        sending = sending != cudaSuccess ? sending : cudaMemcpyAsync(
             static_cast<uint8_t*>(lane.d_src.ptr) + sent_bytes, block + sent_bytes, end - sent_bytes, cudaMemcpyHostToDevice,
             lane.stream);
         sent = ready;
@@ -760,7 +764,7 @@ int enqueue_on_lane(
     ctx->host_stage_ns += (uint64_t)std::chrono::duration_cast<std::chrono::nanoseconds>(
         std::chrono::steady_clock::now() - t0).count();
   }
-  if (timed && host_src) {
+  if (timed && host_src && !sent_early) {
     MLXD_CUDA(cudaEventRecord(lane.in_begin[slot], lane.stream));
     lane.in_timed[slot] = true;
   }

@@ -254,6 +254,49 @@ void failed_copy_of_a_part() {
   }
 }
 
+// What a call queues besides events.
+std::vector<std::string> queued() {
+  std::vector<std::string> out;
+  for (const std::string& c : calls) {
+    if (c != "record" && c != "query" && c.rfind("wait", 0) != 0) {
+      out.push_back(c);
+    }
+  }
+  return out;
+}
+
+// Timed calls queue the same copies and kernels as others, and each is counted once.
+void timed_calls_take_the_same_way() {
+  const int h = 1100, w = 700, n = 3;
+  std::vector<uint8_t> src((size_t)h * w * 3, 7), dst(src.size() * 129);
+  const mlxd_batch_desc host = batch_of(dst.data(), h, w, 3);
+  mlxd_batch_desc device = batch_of(dst.data(), 8, 8, 3);
+  device.src_mem = device.dst_mem = MLXD_MEM_DEVICE;
+  std::vector<mlxd_sample_desc> frames(n, whole(src.data(), h, w)), tiny(129, whole(src.data(), 8, 8));
+  std::vector<std::string> way[2];
+  for (int timed = 0; timed < 2; timed++) {
+    mlxd_ctx* ctx = context();
+    CHECK(mlxd_ctx_set_timing(ctx, timed) == MLXD_OK);
+    calls.clear();
+    for (int i = 0; i < 6; i++) {   // (more than there are slots)
+      for (const int k : {1, 24, 128, 129}) {
+        CHECK(mlxd_fused_batch_on_stream(ctx, nullptr, tiny.data(), k, &device) == MLXD_OK);
+        run(nullptr);
+      }
+      CHECK(mlxd_fused_batch(ctx, 0, frames.data(), n, &host) == MLXD_OK);
+      CHECK(mlxd_batch_wait(ctx, 0, -1) == MLXD_OK);
+    }
+    way[timed] = queued();
+    mlxd_stats stats;
+    CHECK(mlxd_stats_get(ctx, &stats) == MLXD_OK);
+    CHECK(stats.timed_launches == (timed ? 30u : 0u));
+    CHECK(stats.kernel_ns == stats.timed_launches * 1000000u);   // (a made-up event is 1 ms from any other)
+    CHECK(stats.h2d_ns == (timed ? 6000000u : 0u));
+    mlxd_ctx_destroy(ctx);
+  }
+  CHECK(way[0] == way[1]);
+}
+
 } // namespace
 
 int main(int argc, char** argv) {
@@ -261,6 +304,7 @@ int main(int argc, char** argv) {
       {"wait_beside_another_caller", wait_beside_another_caller},
       {"copies_of_huge_sources_beside_a_resize", copies_of_huge_sources_beside_a_resize},
       {"failed_copy_of_a_part", failed_copy_of_a_part},
+      {"timed_calls_take_the_same_way", timed_calls_take_the_same_way},
   };
   const auto it = argc == 2 ? scenarios.find(argv[1]) : scenarios.end();
   if (it == scenarios.end()) {
