@@ -312,8 +312,9 @@ void compute_cast_table(const mlxd_batch_desc* b, int c_out, float* table) {
 // A division of a float x by a float d, correctly rounded, is fma(x, hi, x * lo) with
 // hi + lo = 1 / d to 48 bits, unless the quotient lies within 2^-48 of the middle between
 // two floats: so every value is compared with the table's, and a cast with one that differs
-// (or with infinities) keeps the table.  The channel reduction's casts do too: their values
-// are whole numbers, which index it as they are.
+// (or with infinities) keeps the table.  So does one with a NaN, of which arithmetic on the GPU
+// keeps neither sign nor payload, and the channel reduction's: its values are whole numbers,
+// which index the table as they are.
 void cast_steps(const mlxd_batch_desc* b, int c_out, const float* table, CastSteps& steps) {
   std::memset(&steps, 0, sizeof(steps));
   if (b->gray) {
@@ -339,7 +340,7 @@ void cast_steps(const mlxd_batch_desc* b, int c_out, const float* table, CastSte
         const volatile float t_low = t * steps.s_lo[c][0];
         y = std::fma((float)t, steps.s_hi[c][0], (float)t_low);
       }
-      if (std::memcmp(&y, &table[(size_t)c * 256 + v], sizeof(y)) != 0) {
+      if (y != y || std::memcmp(&y, &table[(size_t)c * 256 + v], sizeof(y)) != 0) {
         return;
       }
     }

@@ -4,6 +4,7 @@
 // does in between, is the same in every run, and calls can be made to fail.
 //
 // Usage: host_logic SCENARIO; exits with 0 if it holds, else prints what does not.
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -297,6 +298,30 @@ void timed_calls_take_the_same_way() {
   CHECK(way[0] == way[1]);
 }
 
+// Casts that give NaN are looked up: steps on the GPU would give other NaNs than the table's.
+void casts_with_nan_keep_the_table() {
+  const float nan = std::nanf("");
+  struct Case { float divisor, mean, std; int normalise, mode; };
+  for (const Case& k : {Case{255.0f, 0.0f, 1.0f, 0, kCastScale}, Case{255.0f, 0.4f, 0.2f, 1, kCastNormalise},
+                        Case{nan, 0.0f, 1.0f, 0, kCastTable}, Case{-nan, 0.4f, 0.2f, 1, kCastTable},
+                        Case{255.0f, 0.4f, nan, 1, kCastTable}, Case{255.0f, 0.4f, -nan, 1, kCastTable},
+                        Case{255.0f, nan, 0.2f, 1, kCastTable}, Case{255.0f, 0.0f, 0.0f, 1, kCastTable}}) {
+    mlxd_batch_desc b = batch_of(nullptr, 8, 8, 3);
+    b.out_dtype = MLXD_F32;
+    b.divisor = k.divisor;
+    b.normalise = k.normalise;
+    for (int c = 0; c < 3; c++) {
+      b.mean[c] = c == 1 ? k.mean : 0.5f;
+      b.std_[c] = c == 1 ? k.std : 0.25f;
+    }
+    float table[3 * 256];
+    CastSteps steps;
+    compute_cast_table(&b, 3, table);
+    cast_steps(&b, 3, table, steps);
+    CHECK(steps.mode == k.mode);
+  }
+}
+
 } // namespace
 
 int main(int argc, char** argv) {
@@ -305,6 +330,7 @@ int main(int argc, char** argv) {
       {"copies_of_huge_sources_beside_a_resize", copies_of_huge_sources_beside_a_resize},
       {"failed_copy_of_a_part", failed_copy_of_a_part},
       {"timed_calls_take_the_same_way", timed_calls_take_the_same_way},
+      {"casts_with_nan_keep_the_table", casts_with_nan_keep_the_table},
   };
   const auto it = argc == 2 ? scenarios.find(argv[1]) : scenarios.end();
   if (it == scenarios.end()) {
