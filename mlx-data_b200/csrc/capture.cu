@@ -53,7 +53,7 @@ int capture_batch(
   std::vector<float> cast(p.out_f32 ? (size_t)p.c_out * 256 : 0);
   if (p.out_f32) {
     compute_cast_table(batch, p.c_out, cast.data());
-    cast_steps(batch, p.c_out, cast.data(), p.cast);
+    kept_cast_steps(batch, p.c_out, cast.data(), p.cast);
   }
   const size_t cast_bytes = cast.size() * sizeof(float);
   void* block = nullptr;

@@ -166,6 +166,9 @@ void compute_cast_table(const mlxd_batch_desc* b, int c_out, float* table);
 // The same cast as steps, where they give every value of the table (else kCastTable).
 void cast_steps(const mlxd_batch_desc* b, int c_out, const float* table, CastSteps& steps);
 
+// The same with the last few casts' results kept, for calls that use no context's cache.
+void kept_cast_steps(const mlxd_batch_desc* b, int c_out, const float* table, CastSteps& steps);
+
 // Launch-wide parameters from a batch descriptor, without the cast table, and with it.
 int describe_launch(const mlxd_batch_desc* b, int n, LaunchParams& p);
 int prepare_launch(mlxd_ctx* ctx, const mlxd_batch_desc* b, int n, LaunchParams& p);

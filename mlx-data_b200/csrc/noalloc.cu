@@ -145,7 +145,7 @@ extern "C" int mlxd_fused_batch_noalloc(
   MLXD_CUDA(cudaMemcpyAsync(scratch, table, sizeof(DevSample) * n, cudaMemcpyHostToDevice, stream));
   if (p.out_f32) {
     compute_cast_table(batch, p.c_out, lut);
-    cast_steps(batch, p.c_out, lut, p.cast);
+    kept_cast_steps(batch, p.c_out, lut, p.cast);
     MLXD_CUDA(cudaMemcpyAsync(
         scratch + kTableBytes, lut, (size_t)p.c_out * 256 * sizeof(float), cudaMemcpyHostToDevice, stream));
   }

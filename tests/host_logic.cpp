@@ -4,6 +4,8 @@
 // does in between, is the same in every run, and calls can be made to fail.
 //
 // Usage: host_logic SCENARIO; exits with 0 if it holds, else prints what does not.
+#include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -322,6 +324,80 @@ void casts_with_nan_keep_the_table() {
   }
 }
 
+mlxd_batch_desc cast_batch(int c, int normalise, float divisor, float mean, float std) {
+  mlxd_batch_desc b = batch_of(nullptr, 8, 8, c);
+  b.src_mem = b.dst_mem = MLXD_MEM_DEVICE;
+  b.out_dtype = MLXD_F32;
+  b.divisor = divisor;
+  b.normalise = normalise;
+  for (int i = 0; i < 4; i++) {
+    b.mean[i] = mean + 0.01f * (float)i;
+    b.std_[i] = std + 0.01f * (float)i;
+  }
+  return b;
+}
+
+// Least microseconds of a call.
+template <class F>
+double least_us(F&& f) {
+  double best = 1e9;
+  for (int i = 0; i < 2000; i++) {
+    const auto t = std::chrono::steady_clock::now();
+    f();
+    best = std::min(best, std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t).count());
+  }
+  return best;
+}
+
+// Calls without a context's cache: each has the steps of its own cast, in whatever order casts come,
+// and a cast that comes again is not compared value by value again.
+void casts_without_a_cache() {
+  std::vector<mlxd_batch_desc> casts;
+  for (int c = 1; c <= 4; c++) {
+    casts.push_back(cast_batch(c, 0, 255.0f, 0.0f, 0.0f));
+    casts.push_back(cast_batch(c, 0, 1e-39f, 0.0f, 0.0f));
+    casts.push_back(cast_batch(c, 1, 255.0f, 0.4f, 0.2f));
+    casts.push_back(cast_batch(c, 1, 255.0f, 0.4f, 0.3f));
+  }
+  casts.push_back(cast_batch(3, 1, 255.0f, 0.4f, 0.2f));
+  casts.back().gray = 1;
+  uint8_t src[8 * 8 * 4] = {};
+  std::vector<uint8_t> dst(8 * 8 * 16);
+  LaunchParams launched;
+  kernel = [&](const LaunchParams& p) { launched = p; };
+  const mlxd_sample_desc d = whole(src, 8, 8);
+  auto call = [&](const mlxd_batch_desc& cast) {
+    mlxd_batch_desc b = cast;
+    b.dst = dst.data();
+    CHECK(mlxd_fused_batch_noalloc(0, nullptr, &d, 1, &b) == MLXD_OK);
+    run(nullptr);
+    calls.clear();
+  };
+  unsigned order = 1;
+  for (int i = 0; i < 400; i++) {
+    order = order * 1664525u + 1013904223u;
+    const mlxd_batch_desc& b = casts[i < 100 ? i % casts.size() : (order >> 8) % (i < 250 ? 4 : casts.size())];
+    call(b);
+    const int c_out = b.gray ? 1 : b.channels;
+    float table[4 * 256];
+    CastSteps steps;
+    compute_cast_table(&b, c_out, table);
+    cast_steps(&b, c_out, table, steps);
+    CHECK(std::memcmp(&steps, &launched.cast, sizeof(steps)) == 0);
+    CHECK(std::memcmp(table, launched.lut, sizeof(float) * 256 * c_out) == 0);
+  }
+  mlxd_batch_desc bytes = cast_batch(3, 0, 1.0f, 0.0f, 0.0f);
+  bytes.out_dtype = MLXD_U8;
+  const mlxd_batch_desc floats = cast_batch(3, 1, 255.0f, 0.4f, 0.2f);
+  float table[4 * 256];
+  CastSteps steps;
+  const double with_cast = least_us([&] { call(floats); }), without = least_us([&] { call(bytes); });
+  const double table_us = least_us([&] { compute_cast_table(&floats, 3, table); });
+  const double steps_us = least_us([&] { cast_steps(&floats, 3, table, steps); });
+  std::printf("float call %.2f us, byte call %.2f, table %.2f, steps %.2f\n", with_cast, without, table_us, steps_us);
+  CHECK(with_cast - without - table_us < 0.5 * steps_us);
+}
+
 } // namespace
 
 int main(int argc, char** argv) {
@@ -331,6 +407,7 @@ int main(int argc, char** argv) {
       {"failed_copy_of_a_part", failed_copy_of_a_part},
       {"timed_calls_take_the_same_way", timed_calls_take_the_same_way},
       {"casts_with_nan_keep_the_table", casts_with_nan_keep_the_table},
+      {"casts_without_a_cache", casts_without_a_cache},
   };
   const auto it = argc == 2 ? scenarios.find(argv[1]) : scenarios.end();
   if (it == scenarios.end()) {

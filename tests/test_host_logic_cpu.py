@@ -26,7 +26,7 @@ def program(tmp_path_factory):
 
 @pytest.mark.parametrize("scenario", ["wait_beside_another_caller", "copies_of_huge_sources_beside_a_resize",
                                       "failed_copy_of_a_part", "timed_calls_take_the_same_way",
-                                      "casts_with_nan_keep_the_table"])
+                                      "casts_with_nan_keep_the_table", "casts_without_a_cache"])
 def test_scenario(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, (r.returncode, r.stdout + r.stderr)
