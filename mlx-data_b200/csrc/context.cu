@@ -3,7 +3,9 @@
 
 #include <map>
 
+#ifdef __SSE2__
 #include <emmintrin.h>
+#endif
 #include <sched.h>
 
 #include <algorithm>
@@ -488,7 +490,8 @@ static int pack_threads() {
 // to the next multiple of 16), by stores past the caches: the copy engine reads lines that a
 // core holds modified at a third of the bus's rate.  Where one row ends and the next begins
 // inside 64 bytes they are put together first, so that whole lines leave.  32 images of 256-640
-// px, 12.3 MB: packing 290 us by memcpy, 200 so, the copy after it 650 and 230.
+// px, 12.3 MB: packing 290 us by memcpy, 200 so, the copy after it 650 and 230.  On a host
+// without SSE2 the stores are plain ones.
 static void pack_rows(uint8_t* to, const uint8_t* from, size_t pitch, size_t row_bytes, size_t rows) {
   if (row_bytes == pitch) {   // one piece
     row_bytes *= rows;
@@ -497,6 +500,7 @@ static void pack_rows(uint8_t* to, const uint8_t* from, size_t pitch, size_t row
   alignas(64) uint8_t buffer[64];
   size_t held = 0;
   auto stream = [](uint8_t* d, const uint8_t* s, size_t n) {   // n: a multiple of 64
+#ifdef __SSE2__
     for (size_t i = 0; i < n; i += 64) {
       const __m128i a = _mm_loadu_si128(reinterpret_cast<const __m128i*>(s + i));
       const __m128i b = _mm_loadu_si128(reinterpret_cast<const __m128i*>(s + i + 16));
@@ -507,6 +511,9 @@ static void pack_rows(uint8_t* to, const uint8_t* from, size_t pitch, size_t row
       _mm_stream_si128(reinterpret_cast<__m128i*>(d + i + 32), c);
       _mm_stream_si128(reinterpret_cast<__m128i*>(d + i + 48), e);
     }
+#else
+    std::memcpy(d, s, n);
+#endif
   };
   for (size_t r = 0; r < rows; r++) {
     const uint8_t* s = from + r * pitch;
@@ -535,7 +542,9 @@ static void pack_rows(uint8_t* to, const uint8_t* from, size_t pitch, size_t row
   if (held > 0) {
     std::memcpy(to, buffer, held);
   }
+#ifdef __SSE2__
   _mm_sfence();
+#endif
 }
 
 int enqueue_on_lane(
@@ -912,7 +921,9 @@ int wait_lane(mlxd_ctx* ctx, Lane& lane, int timeout_ms) {
     // One batch of 8 full-HD frames 1027 us, 696 so.
     const volatile int32_t* const under_way = lane.h_status + 1;
     for (int i = 0; *under_way != 0; i++) {
+#ifdef __SSE2__
       _mm_pause();
+#endif
       if (i % 64 == 63) {
         if (std::chrono::steady_clock::now() - start > std::chrono::microseconds(kLookMicroseconds)) {
           break;

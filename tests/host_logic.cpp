@@ -398,6 +398,61 @@ void casts_without_a_cache() {
   CHECK(with_cast - without - table_us < 0.5 * steps_us);
 }
 
+// Pageable sources through the lane's block: windows whose rows are shorter and longer than 64
+// bytes and start anywhere, in batches below and above what is sent in parts.
+void packed_sources() {
+  const int sizes[][4] = {{9, 5, 9, 5}, {40, 33, 31, 21}, {40, 33, 40, 33}, {300, 400, 299, 133}, {1300, 1111, 1207, 1111}, {900, 1001, 900, 777}};
+  for (int c = 1; c <= 4; c++) {
+    std::vector<std::vector<uint8_t>> src, got;
+    std::vector<mlxd_sample_desc> d;
+    for (const auto& k : sizes) {
+      src.emplace_back((size_t)k[0] * k[1] * c);
+      for (size_t i = 0; i < src.back().size(); i++) {
+        src.back()[i] = (uint8_t)(i * 2654435761u >> 13);
+      }
+    }
+    for (size_t i = 0; i < src.size(); i++) {
+      const auto& k = sizes[i];
+      d.push_back(whole(src[i].data(), k[0], k[1]));
+      d.back().post_y = k[0] - k[2];
+      d.back().post_x = k[1] - k[3];
+      d.back().post_h = k[2];
+      d.back().post_w = k[3];
+    }
+    std::vector<uint8_t> dst((size_t)1300 * 1111 * c * d.size());
+    const mlxd_batch_desc b = batch_of(dst.data(), 1300, 1111, c);
+    got.resize(d.size());
+    kernel = [&](const LaunchParams& p) {   // the window of every sample, from where the launch has its source
+      for (int i = 0; i < p.n; i++) {
+        const DevSample& s = p.samples[i];
+        for (int y = 0; y < s.post_h; y++) {
+          const uint8_t* row = s.src + ((size_t)(s.pre_y + s.post_y + y) * s.src_w + s.pre_x + s.post_x) * c;
+          got[i].insert(got[i].end(), row, row + (size_t)s.post_w * c);
+        }
+      }
+    };
+    mlxd_ctx* ctx = context();
+    for (size_t n : {size_t(1), size_t(4), d.size()}) {
+      for (auto& g : got) {
+        g.clear();
+      }
+      CHECK(mlxd_fused_batch(ctx, 0, d.data(), (int)n, &b) == MLXD_OK);
+      CHECK(mlxd_batch_wait(ctx, 0, -1) == MLXD_OK);
+      for (size_t i = 0; i < n; i++) {
+        const auto& k = sizes[i];
+        std::vector<uint8_t> want;
+        for (int y = k[0] - k[2]; y < k[0]; y++) {
+          const uint8_t* row = src[i].data() + ((size_t)y * k[1] + k[1] - k[3]) * c;
+          want.insert(want.end(), row, row + (size_t)k[3] * c);
+        }
+        CHECK(want == got[i]);
+      }
+    }
+    mlxd_ctx_destroy(ctx);
+  }
+  kernel = [](const LaunchParams&) {};
+}
+
 } // namespace
 
 int main(int argc, char** argv) {
@@ -408,6 +463,7 @@ int main(int argc, char** argv) {
       {"timed_calls_take_the_same_way", timed_calls_take_the_same_way},
       {"casts_with_nan_keep_the_table", casts_with_nan_keep_the_table},
       {"casts_without_a_cache", casts_without_a_cache},
+      {"packed_sources", packed_sources},
   };
   const auto it = argc == 2 ? scenarios.find(argv[1]) : scenarios.end();
   if (it == scenarios.end()) {
