@@ -161,7 +161,9 @@ struct LaunchParams {
 // from LaunchParams::samples.  A kernel may have 32 764 bytes of parameters; each launch
 // moves all of them, so there are two sizes.  4 images of 480x640 to 224x224 take 10.8 us a pass
 // with 24, 13.2 with 128, 15.3 with a table copied ahead of the kernel; 32 of 200-500 px 17.5 with
-// 128 and 20.9 with a table.
+// 128 and 20.9 with a table.  240, the most that fit, in place of 128 take 0.5 to 1 us off
+// batches of 129 to 240 (160 of 64x64 28.5 us a pass, 27.5; 240 of 200-500 px 77.2, 76.4) and put up to
+// 2 on those of 25 to 128 (64 of 64x64 18.4 us, 20.1; 128 of 256x256 rotated 45.2, 46.8).
 constexpr int kFewSamples = 24, kMoreSamples = 128;
 
 template <int K>

@@ -158,7 +158,7 @@ static int strip_span(const DevSample& s, int rows) {
   return (int)(span < 1e6f ? span : 1e6f) + 2 + axis_slack(s.pre_h);
 }
 
-// Bound on the steps of a walk over `rows` output rows (launch_plan.cu: walk_steps).
+// walk_steps() from the ratio in the sample's record.
 static int strip_steps(const DevSample& s, int rows) {
   const int slack = axis_slack(s.pre_h);
   if (s.pre_h <= s.geom_h) {
