@@ -45,13 +45,15 @@ __device__ __forceinline__ f32x2 both(const float (&pair)[2]) {
 // shared memory: 32 values meet three to four times in its banks, so a look-up takes the
 // shared-memory pipe, of which a shrink has least to spare, as long as three other accesses.
 // 512 images of 1080x1920x3 to 512x512: 1105 us, 1146 with the table; 256 random crops to
-// 224x224 113 and 115; one image 9.6 and 10.0.
-template <int C, bool GRAY, bool U8>
+// 224x224 113 and 115; one image 9.6 and 10.0.  CAST: the way is known at compile time (a
+// CastMode), or -1.
+template <int C, bool GRAY, bool U8, int CAST = -1>
 __device__ __forceinline__ void store_column(
     const LaunchParams& p, unsigned lut, const f32x2 (&acc)[2 * C], int rows, void* dst, size_t at, size_t row_stride,
     bool vec_ok) {
   constexpr int CO = GRAY ? 1 : C;
-  if (!U8 && !GRAY && p.cast.mode != kCastTable) {
+  const int mode = CAST < 0 ? p.cast.mode : CAST;
+  if (!U8 && !GRAY && mode != kCastTable) {
     const f32x2 half = pack2(0.5f, 0.5f), two23 = pack2(8388608.0f, 8388608.0f), minus_two23 = pack2(-8388608.0f, -8388608.0f);
     f32x2 v[2 * C];
 #pragma unroll
@@ -61,7 +63,7 @@ __device__ __forceinline__ void store_column(
       t = add2(t, minus_two23);
       v[i] = fma2(t, both(p.cast.r_hi), mul2(t, both(p.cast.r_lo)));
     }
-    if (p.cast.mode == kCastNormalise) {
+    if (mode == kCastNormalise) {
 #pragma unroll
       for (int i = 0; i < 2 * C; i++) {
         const f32x2 t = add2(v[i], both(p.cast.neg_mean[i / 2]));

@@ -37,6 +37,16 @@
 // move of a register between steps (1.62 - 1.89 ms).  One set of float rows and
 // two barriers a stage leave room for six CTAs per SM; the clamped tap loop of
 // chunks at an image's edge costs two instructions a tap.
+//
+// Unlike samples whose rows do and do not start on a word, with CTAs that fill padding among
+// them, keep several paths of the kernel in the instruction cache at a time.  So where the cast is
+// computed the horizontal half is there once for both kinds of rows, and an instance knows its way
+// of casting.  346 images of 880-1730 px, shorter side 323, padded and normalised: with the casts by
+// steps beside the look-ups in both halves 1357 us (0.67 stalls an issue for want of
+// instructions), look-ups alone 1320 (0.23), so 1300; 64 of 1400 px to 300x300 216, 223 and 216.
+// The way of casting alone known, the half still twice: 1471 and 236.  With the channel reduction
+// 226 us and 202.  Byte batches and look-ups, whose code is shorter, keep the half twice (300 of
+// 880-1730 px to 323x323, bytes, 908 us, 921 with one; 128 of 900 px to 64x64, looked up, 147.7 and 149.7).
 #include <algorithm>
 
 #include "fused_batch.h"
@@ -258,10 +268,13 @@ struct Chunk {
   bool edge_x, pre_flip;
 };
 
-// The stages of one chunk, tables in place.
-template <int C, bool GRAY, bool U8, bool SHIFT>
-__device__ __forceinline__ void walk_stages(const DevSample& s, const LaunchParams& p, const Chunk& c) {
+// The stages of one chunk, tables in place.  Its rows start on a word, or not, or (kAnyRows)
+// `shifted` says.
+enum RowStart { kWordRows, kShiftedRows, kAnyRows };
+template <int C, bool GRAY, bool U8, int CAST, RowStart ROWS>
+__device__ __forceinline__ void walk_stages(const DevSample& s, const LaunchParams& p, const Chunk& c, bool shifted) {
   constexpr int CO = GRAY ? 1 : C;
+  const bool shift = ROWS == kAnyRows ? shifted : ROWS == kShiftedRows;
   const int tid = threadIdx.x;
   const int first_word = (tid >> 5) * 64;
   const bool warp_works = first_word < c.nwords;
@@ -278,7 +291,11 @@ __device__ __forceinline__ void walk_stages(const DevSample& s, const LaunchPara
 #pragma unroll 1
     for (int j = 0; j < kAhead; j++) {
       const unsigned e = c.sm.steps + 32u * j;
-      fetch<SHIFT>(k, lds_u32<16>(e), (int)lds_u32<20>(e), (unsigned)j * kSlotBytes);
+      if (shift) {
+        fetch<true>(k, lds_u32<16>(e), (int)lds_u32<20>(e), (unsigned)j * kSlotBytes);
+      } else {
+        fetch<false>(k, lds_u32<16>(e), (int)lds_u32<20>(e), (unsigned)j * kSlotBytes);
+      }
     }
   }
   const size_t row_stride = (size_t)s.slot_w * CO;
@@ -291,7 +308,12 @@ __device__ __forceinline__ void walk_stages(const DevSample& s, const LaunchPara
   for (int r0 = 0; r0 < c.nr; r0 += kStageRows) {
     const int rows = min(kStageRows, c.nr - r0);
     if (warp_works) {
-      walk_pairs<SHIFT>(k, mid + (unsigned)k.word * 32u, c.sm.count + 4u * (unsigned)r0, rows);
+      const unsigned st = mid + (unsigned)k.word * 32u, count = c.sm.count + 4u * (unsigned)r0;
+      if (shift) {
+        walk_pairs<true>(k, st, count, rows);
+      } else {
+        walk_pairs<false>(k, st, count, rows);
+      }
     }
     __syncthreads();
     for (int x = tid; x < c.nc; x += kWalkThreads) {
@@ -320,7 +342,7 @@ __device__ __forceinline__ void walk_stages(const DevSample& s, const LaunchPara
         }
       }
       const int ox = post_flip ? c.x1 - 1 - x : c.x0 + x;
-      store_column<C, GRAY, U8>(
+      store_column<C, GRAY, U8, CAST>(
           p, c.sm.lut, acc, rows, dst, (size_t)(c.y0 + r0) * row_stride + (size_t)ox * CO, row_stride, vec_ok);
     }
     __syncthreads();
@@ -328,7 +350,7 @@ __device__ __forceinline__ void walk_stages(const DevSample& s, const LaunchPara
 }
 
 // Rows [y0, y1) x columns [x0, x1) of the slot, all inside the post window.
-template <int C, bool GRAY, bool U8>
+template <int C, bool GRAY, bool U8, int CAST>
 __device__ __forceinline__ void walk_chunk(
     const DevSample& s, const LaunchParams& p, const WalkSmem& sm, int y0, int y1, int x0, int x1) {
   constexpr int CO = GRAY ? 1 : C;
@@ -410,7 +432,7 @@ __device__ __forceinline__ void walk_chunk(
       }
     }
   }
-  if (!U8 && p.cast.mode == kCastTable) {
+  if (!U8 && CAST == kCastTable) {
     for (int i = tid; i < CO * 256; i += kWalkThreads) {
       sp<float>(sm.lut)[i] = __ldg(p.lut + i);
     }
@@ -487,16 +509,18 @@ __device__ __forceinline__ void walk_chunk(
 
   const Chunk c = {sm, g0 - common, pitch, common, nwords, nr, nc, y0, x0, x1, (int)sm.mid + common * 8,
                    (int)sm.mid + (common + (chi - clo) * C) * 8, edge_x, pre_flip};
-  if (shifted) {
-    walk_stages<C, GRAY, U8, true>(s, p, c);
+  if (!U8 && (GRAY || CAST != kCastTable)) {
+    walk_stages<C, GRAY, U8, CAST, kAnyRows>(s, p, c, shifted);
+  } else if (shifted) {
+    walk_stages<C, GRAY, U8, CAST, kShiftedRows>(s, p, c, true);
   } else {
-    walk_stages<C, GRAY, U8, false>(s, p, c);
+    walk_stages<C, GRAY, U8, CAST, kWordRows>(s, p, c, false);
   }
 }
 
 // One cell: walk_rows rows x one chunk (or one strip of padding) of a slot.
-// OWN: samples count their own cells off (WalkPlan::cells_y of 0).
-template <int C, bool GRAY, bool U8, bool OWN>
+// OWN: samples count their own cells off (WalkPlan::cells_y of 0).  CAST: how its floats are cast.
+template <int C, bool GRAY, bool U8, int CAST, bool OWN>
 __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __grid_constant__ LaunchParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int CO = GRAY ? 1 : C;
@@ -541,8 +565,8 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
   const int fill_y1 = p.pad_apart ? vy1 : y1;         // rows below the post window are the fill CTAs' then
   if (!strip && y0 < vy1) {
     WalkSmem sm;
-    walk_layout(table_channels(p), p.walk, smem_addr(smem_raw), &sm);
-    walk_chunk<C, GRAY, U8>(s, p, sm, y0, vy1, x0, x1);
+    walk_layout(!U8 && CAST == kCastTable ? CO : 0, p.walk, smem_addr(smem_raw), &sm);
+    walk_chunk<C, GRAY, U8, CAST>(s, p, sm, y0, vy1, x0, x1);
   }
   if (fill_y0 < fill_y1) {
     if (U8) {
@@ -561,7 +585,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) resize_walk_kernel(const __gr
 // No plan needs more shared memory than this.
 constexpr size_t kWalkMaxSmem = walk_layout(4, WalkPlan{kWalkMaxPx, kWalkMaxTaps, kWalkMaxSteps, 0, 0}, 0u, nullptr);
 
-template <int C, bool GRAY, bool U8, bool OWN>
+template <int C, bool GRAY, bool U8, int CAST, bool OWN>
 cudaError_t launch_kernel(const LaunchParams& p, unsigned blocks, size_t smem, cudaStream_t stream) {
   // Only strong shrinks need more than the 48 KB that every kernel may have.  The
   // limit belongs to the kernel on the current device and is shared by all host
@@ -569,19 +593,32 @@ cudaError_t launch_kernel(const LaunchParams& p, unsigned blocks, size_t smem, c
   // need could lower the limit between another's setting and its launch.
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(
-        resize_walk_kernel<C, GRAY, U8, OWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkMaxSmem);
+        resize_walk_kernel<C, GRAY, U8, CAST, OWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkMaxSmem);
     if (e != cudaSuccess) {
       return e;
     }
   }
-  resize_walk_kernel<C, GRAY, U8, OWN><<<blocks, kWalkThreads, smem, stream>>>(p);
+  resize_walk_kernel<C, GRAY, U8, CAST, OWN><<<blocks, kWalkThreads, smem, stream>>>(p);
   return cudaGetLastError();
+}
+
+template <int C, bool GRAY, bool U8, int CAST>
+cudaError_t launch_cast(const LaunchParams& p, unsigned blocks, size_t smem, cudaStream_t stream) {
+  return p.walk.cells_y == 0 ? launch_kernel<C, GRAY, U8, CAST, true>(p, blocks, smem, stream)
+                          : launch_kernel<C, GRAY, U8, CAST, false>(p, blocks, smem, stream);
 }
 
 template <int C, bool GRAY, bool U8>
 cudaError_t launch(const LaunchParams& p, unsigned blocks, size_t smem, cudaStream_t stream) {
-  return p.walk.cells_y == 0 ? launch_kernel<C, GRAY, U8, true>(p, blocks, smem, stream)
-                          : launch_kernel<C, GRAY, U8, false>(p, blocks, smem, stream);
+  if constexpr (!GRAY && !U8) {
+    if (p.cast.mode == kCastScale) {
+      return launch_cast<C, GRAY, U8, kCastScale>(p, blocks, smem, stream);
+    }
+    if (p.cast.mode == kCastNormalise) {
+      return launch_cast<C, GRAY, U8, kCastNormalise>(p, blocks, smem, stream);
+    }
+  }
+  return launch_cast<C, GRAY, U8, kCastTable>(p, blocks, smem, stream);
 }
 
 } // namespace
