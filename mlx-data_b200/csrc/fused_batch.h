@@ -170,14 +170,19 @@ template <int K>
 struct Records {
   DevSample at[K];
   __device__ __forceinline__ const DevSample* of(const LaunchParams& p, unsigned t) const { return at + p.first + t; }
+  __device__ __forceinline__ const DevSample* whole(const LaunchParams& p, unsigned t) const { return of(p, t); }
 };
 
 template <>
 struct Records<0> {
-  // (The record is asked for as a whole: a kernel reads it field by field as it decides what it
-  // needs, and waited for each of its four sectors.  512 full-HD frames 1100 -> 1097 us.)
-  __device__ __forceinline__ const DevSample* of(const LaunchParams& p, unsigned t) const {
-    const DevSample* const s = p.samples + p.first + t;
+  __device__ __forceinline__ const DevSample* of(const LaunchParams& p, unsigned t) const { return p.samples + p.first + t; }
+  // The record asked for as a whole, for a CTA that reads it field by field as it decides what it
+  // needs, and waited for each of its four sectors: 512 full-HD frames 1100 -> 1097 us.  CTAs of
+  // little work wait longer for what is asked: with it, those that fill padding and the bands took
+  // 1.02 to 1.34 times as long (200 one-channel images of 200-400 px padded to the largest, bytes,
+  // 87 us, 64 without; 500 of 200-500 px, shorter side 128, 178 and 163).
+  __device__ __forceinline__ const DevSample* whole(const LaunchParams& p, unsigned t) const {
+    const DevSample* const s = of(p, t);
 #ifdef __CUDA_ARCH__
     asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(s) + 32 * (threadIdx.x & 3)));
 #endif
