@@ -45,7 +45,7 @@ __device__ __forceinline__ f32x2 both(const float (&pair)[2]) {
 // shared memory: 32 values meet three to four times in its banks, so a look-up takes the
 // shared-memory pipe, of which a shrink has least to spare, as long as three other accesses.
 // 512 images of 1080x1920x3 to 512x512: 1105 us, 1146 with the table; 256 random crops to
-// 224x224 113 and 115; one image 9.6 and 10.0.  CAST: the way is known at compile time (a
+// 224x224 113 and 115; one image 9.6 and 10.0; in resize_walk.cu 64 of 1400 px to 300x300 216 and 223.  CAST: the way is known at compile time (a
 // CastMode), or -1.
 template <int C, bool GRAY, bool U8, int CAST = -1>
 __device__ __forceinline__ void store_column(

@@ -25,12 +25,13 @@
 // out times 2^-22 and the horizontal weights are kept times 2^22 - powers of two
 // throughout, so every rounding falls as without them.
 //
-// What bounds it (1080x1920x3 to 512x512, 512 images: 1.10 ms, 1.15 where casts are looked
-// up; 1.37 in resize_walk.cu, which runs a whole CTA down 832 bytes): with look-ups the
-// shared-memory pipe, 76 % busy (89 there), and its latency at 20 warps an SM;
-// instructions issue in 58 % of the cycles.  Per 32 columns x 4 rows, look-ups included,
-// a warp executes 780 instructions (830), about 310 of them on the steps, 260 on taps and
-// stores, 110 on copies and the skeleton of a stage.  Why this
+// What bounds it (1080x1920x3 to 512x512, 512 images: 1.12 ms, 1.16 where casts are looked
+// up; 1.37 in resize_walk.cu, which runs a whole CTA down 832 bytes): the latency of its own
+// results and of shared memory at 19 warps an SM (1.8 and 1.2 of 7.4 cycles an instruction);
+// instructions issue in 61 % of the cycles, the shared-memory pipe is 66 % busy (58 and 76 with
+// look-ups, 89 there).  Per 32 columns x 4 rows a warp executes 810 instructions (780 with look-ups,
+// 830 there), of them about 310 on the steps, 110 on copies and the skeleton of a stage, the rest on taps,
+// casts and stores.  Why this
 // split: two 4-byte cp.async a row cost the pipe nine wavefronts, one 16-byte cp.async
 // for two rows about two a row; a unit of four rows halves the loads of the taps, and
 // dealing columns to lanes by bank takes most of their conflicts; a CTA-wide walk meets
