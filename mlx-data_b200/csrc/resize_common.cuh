@@ -37,6 +37,9 @@ __device__ __forceinline__ f32x2 both(const float (&pair)[2]) {
   return pack2(pair[0], pair[1]);
 }
 
+#pragma nv_diagnostic push
+#pragma nv_diag_suppress 128   // (where the way of casting is known, the look-ups below are never reached)
+
 // One output column of four rows: filter sums acc[2 * c + h] (rows 2h and 2h + 1
 // of channel c) quantised, reduced to grey, cast and stored.  `at` is the first
 // row's place in the batch tensor in elements; the first `rows` rows are stored.
@@ -136,5 +139,7 @@ __device__ __forceinline__ void store_column(
     }
   }
 }
+
+#pragma nv_diagnostic pop
 
 } // namespace mlxd
